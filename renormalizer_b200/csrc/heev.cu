@@ -1161,9 +1161,6 @@ __global__ void __launch_bounds__(IV_THREADS) inviter_kernel(const __grid_consta
 // H_k0 ... H_k0+kb-1 = I - V T V^H, LAPACK's forward columnwise larft), the
 // blocks applied from the last to the first, each as three FP64 GEMMs.
 constexpr int NB = 64;
-constexpr int KCH = 256;  // row chunk of the split-K products V_b^H K
-
-inline int nch_max(int n) { return (int)ceil_div(std::max(n - 1, 1), KCH); }
 
 // rows 0..n-2 of A become the reflectors (0 before column k+1, 1 at k+1) and
 // row n-1 becomes 0, so that every reflector row can be read over all n columns
@@ -1175,17 +1172,15 @@ __global__ void clean_v_kernel(double2* __restrict__ A, int n) {
   else if (c == k + 1) A[idx] = make_double2(1.0, 0.0);
 }
 
-// minus the NB x NB upper-triangular T of block b from S = V^H V and tau,
-// written rep times side by side (row i of block b at
-// Tg + (b NB + i) NB rep): the split-K partials of V^H K then sum inside the
-// T product.  Thread i owns row i (written and read only by itself).
+// minus the NB x NB upper-triangular T of block b from S = V^H V and tau.
+// Thread i owns row i (written and read only by itself).
 __global__ void __launch_bounds__(NB) larft_kernel(const double2* __restrict__ Sg, const double2* __restrict__ tau,
-                                                   double2* __restrict__ Tg, int n, int rep) {
+                                                   double2* __restrict__ Tg, int n) {
   __shared__ double2 x[NB];
   const int b = blockIdx.x, i = threadIdx.x;
   const int k0 = b * NB, kb = min(NB, n - 1 - k0);
   const double2* S = Sg + (size_t)b * NB * NB;
-  double2* T = Tg + ((size_t)b * NB + i) * NB * rep;
+  double2* T = Tg + ((size_t)b * NB + i) * NB;
   for (int c = 0; c < NB; ++c) T[c] = make_double2(0.0, 0.0);
   for (int j = 0; j < kb; ++j) {
     const double2 tj = tau[k0 + j];
@@ -1200,10 +1195,7 @@ __global__ void __launch_bounds__(NB) larft_kernel(const double2* __restrict__ S
     }
     __syncthreads();
   }
-  for (int c = 0; c < NB; ++c) {
-    const double2 v = make_double2(-T[c].x, -T[c].y);
-    for (int r = 0; r < rep; ++r) T[(size_t)r * NB + c] = v;
-  }
+  for (int c = 0; c < NB; ++c) T[c] = make_double2(-T[c].x, -T[c].y);
 }
 
 }  // namespace heev
@@ -1237,9 +1229,9 @@ HeevLayout heev_layout(int n, int kt) {
   L.s = off;
   off += align256(nblk * NB * NB * sizeof(double2));
   L.t = off;
-  off += align256(nblk * NB * NB * nch_max(n) * sizeof(double2));
+  off += align256(nblk * NB * NB * sizeof(double2));
   L.w1 = off;
-  off += align256((size_t)nch_max(n) * NB * kt * sizeof(double2));
+  off += align256((size_t)NB * kt * sizeof(double2));
   L.w2 = off;
   off += align256((size_t)NB * kt * sizeof(double2));
   L.total = off;
@@ -1510,7 +1502,6 @@ extern "C" int reno_heev_backtransform(reno_ctx* ctx, int32_t n, int32_t kt, voi
   double2* Kc = static_cast<double2*>(K);
   cudaStream_t st = ctx->stream;
   const int nblk = (int)ceil_div(n - 1, NB);
-  const int rep = nch_max(n);
   const size_t nel = (size_t)n * n;
   count_launch();
   clean_v_kernel<<<(unsigned)ceil_div((int64_t)nel, 256), 256, 0, st>>>(V, n);
@@ -1535,7 +1526,6 @@ extern "C" int reno_heev_backtransform(reno_ctx* ctx, int32_t n, int32_t kt, voi
     p.sCm = NB;
     p.sCn = 1;
     p.sCb = (int64_t)NB * NB;
-    count_launch();
     rc = check_cuda(ctx, gemm_fp64(p, st), "reno_heev_backtransform: gram");
     if (rc != RENO_OK) return rc;
   }
@@ -1550,63 +1540,31 @@ extern "C" int reno_heev_backtransform(reno_ctx* ctx, int32_t n, int32_t kt, voi
     p.C = Sg + (size_t)nfull * NB * NB;
     p.sCm = NB;
     p.sCn = 1;
-    count_launch();
     rc = check_cuda(ctx, gemm_fp64(p, st), "reno_heev_backtransform: gram (last block)");
     if (rc != RENO_OK) return rc;
   }
   count_launch();
-  larft_kernel<<<nblk, NB, 0, st>>>(Sg, static_cast<const double2*>(tau), Tg, n, rep);
+  larft_kernel<<<nblk, NB, 0, st>>>(Sg, static_cast<const double2*>(tau), Tg, n);
   RENO_LAUNCH_CHECK(ctx, "reno_heev_backtransform: larft");
   for (int b = nblk - 1; b >= 0; --b) {
     const int k0 = b * NB, kb = std::min(NB, n - 1 - k0);
     const int rows = n - k0 - 1;
-    const int nfc = rows / KCH, rem = rows % KCH, nch = nfc + (rem > 0);
     const double2* Vb = V + (size_t)k0 * n + k0 + 1;
     double2* Kb = Kc + (size_t)(k0 + 1) * kt;
-    if (kb < NB) {
-      rc = check_cuda(ctx, cudaMemsetAsync(W1, 0, (size_t)nch * NB * kt * sizeof(double2), st),
-                      "reno_heev_backtransform: memset W1");
-      if (rc != RENO_OK) return rc;
-    }
-    // W1[s] = V_b^H K over row chunk s (split K: one batch entry per full chunk)
-    if (nfc > 0) {
-      GemmParams p1;
-      p1.M = kb;
-      p1.N = kt;
-      p1.K = KCH;
-      p1.batch = nfc;
-      p1.A = op(Vb, n, 1, 1);
-      p1.A.s_batch = KCH;
-      p1.B = op(Kb, 1, kt, 0);
-      p1.B.s_batch = (int64_t)KCH * kt;
-      p1.C = W1;
-      p1.sCm = kt;
-      p1.sCn = 1;
-      p1.sCb = (int64_t)NB * kt;
-      count_launch();
-      rc = check_cuda(ctx, gemm_fp64(p1, st), "reno_heev_backtransform: V^H K");
-      if (rc != RENO_OK) return rc;
-    }
-    if (rem > 0) {
-      GemmParams p1;
-      p1.M = kb;
-      p1.N = kt;
-      p1.K = rem;
-      p1.A = op(Vb + (size_t)nfc * KCH, n, 1, 1);
-      p1.B = op(Kb + (size_t)nfc * KCH * kt, 1, kt, 0);
-      p1.C = W1 + (size_t)nfc * NB * kt;
-      p1.sCm = kt;
-      p1.sCn = 1;
-      count_launch();
-      rc = check_cuda(ctx, gemm_fp64(p1, st), "reno_heev_backtransform: V^H K (last chunk)");
-      if (rc != RENO_OK) return rc;
-    }
-    // W2 = (-T_b) sum_s W1[s]: -T_b replicated along K
-    GemmParams p2;
+    GemmParams p1;  // W1 = V_b^H K
+    p1.M = kb;
+    p1.N = kt;
+    p1.K = rows;
+    p1.A = op(Vb, n, 1, 1);
+    p1.B = op(Kb, 1, kt, 0);
+    p1.C = W1;
+    p1.sCm = kt;
+    p1.sCn = 1;
+    GemmParams p2;  // W2 = (-T_b) W1
     p2.M = kb;
     p2.N = kt;
-    p2.K = NB * nch;
-    p2.A = op(Tg + (size_t)b * NB * NB * rep, (int64_t)NB * rep, 1, 0);
+    p2.K = kb;
+    p2.A = op(Tg + (size_t)b * NB * NB, NB, 1, 0);
     p2.B = op(W1, 1, kt, 0);
     p2.C = W2;
     p2.sCm = kt;
@@ -1622,8 +1580,8 @@ extern "C" int reno_heev_backtransform(reno_ctx* ctx, int32_t n, int32_t kt, voi
     p3.sCm = kt;
     p3.sCn = 1;
     p3.accumulate = 1;
-    count_launch(2);
-    rc = check_cuda(ctx, gemm_fp64(p2, st), "reno_heev_backtransform: T W");
+    rc = check_cuda(ctx, gemm_fp64(p1, st), "reno_heev_backtransform: V^H K");
+    if (rc == RENO_OK) rc = check_cuda(ctx, gemm_fp64(p2, st), "reno_heev_backtransform: T W");
     if (rc == RENO_OK) rc = check_cuda(ctx, gemm_fp64(p3, st), "reno_heev_backtransform: K += V W");
     if (rc != RENO_OK) return rc;
   }
@@ -1652,13 +1610,13 @@ extern "C" int reno_heev_backtransform_batched(reno_ctx* ctx, int32_t count, con
     return set_error(ctx, RENO_ERR_WORKSPACE, "reno_heev_backtransform_batched: workspace too small");
   cudaStream_t st = ctx->stream;
   struct One {
-    int n, kt, nblk, rep;
+    int n, kt, nblk;
     double2 *V, *K, *Sg, *Tg, *W1, *W2;
     const double2* tau;
   };
   std::vector<One> P;
   int rc = RENO_OK;
-  static_assert(2 * RENO_HEEV_MAX_BATCH < fp64gemm::MAX_GROUP, "one block step of a batch fits one group");
+  static_assert(2 * RENO_HEEV_MAX_BATCH <= fp64gemm::MAX_GROUP, "one block step of a batch fits one group");
   auto flush = [&](fp64gemm::GemmGroup& g, const char* what) -> int {
     if (g.count == 0) return RENO_OK;
     const int r = check_cuda(ctx, gemm_fp64_grouped(g, st), what);
@@ -1675,7 +1633,7 @@ extern "C" int reno_heev_backtransform_batched(reno_ctx* ctx, int32_t count, con
     if (p.n < 2) continue;
     char* base = static_cast<char*>(ws) + batched_offset(count, probs, i);
     const HeevLayout L = heev_layout(p.n, p.kt);
-    One o{p.n, p.kt, (int)ceil_div(p.n - 1, NB), nch_max(p.n), static_cast<double2*>(p.a),
+    One o{p.n, p.kt, (int)ceil_div(p.n - 1, NB), static_cast<double2*>(p.a),
           static_cast<double2*>(p.k), reinterpret_cast<double2*>(base + L.s), reinterpret_cast<double2*>(base + L.t),
           reinterpret_cast<double2*>(base + L.w1), reinterpret_cast<double2*>(base + L.w2),
           static_cast<const double2*>(p.tau)};
@@ -1726,7 +1684,7 @@ extern "C" int reno_heev_backtransform_batched(reno_ctx* ctx, int32_t count, con
   int bmax = 0;
   for (const One& o : P) {
     count_launch();
-    larft_kernel<<<o.nblk, NB, 0, st>>>(o.Sg, o.tau, o.Tg, o.n, o.rep);
+    larft_kernel<<<o.nblk, NB, 0, st>>>(o.Sg, o.tau, o.Tg, o.n);
     RENO_LAUNCH_CHECK(ctx, "reno_heev_backtransform_batched: larft");
     bmax = std::max(bmax, o.nblk);
   }
@@ -1736,47 +1694,23 @@ extern "C" int reno_heev_backtransform_batched(reno_ctx* ctx, int32_t count, con
       if (b >= o.nblk) continue;
       const int k0 = b * NB, kb = std::min(NB, o.n - 1 - k0);
       const int rows = o.n - k0 - 1;
-      const int nfc = rows / KCH, rem = rows % KCH, nch = nfc + (rem > 0);
       const double2* Vb = o.V + (size_t)k0 * o.n + k0 + 1;
       double2* Kb = o.K + (size_t)(k0 + 1) * o.kt;
-      if (kb < NB) {
-        rc = check_cuda(ctx, cudaMemsetAsync(o.W1, 0, (size_t)nch * NB * o.kt * sizeof(double2), st),
-                        "reno_heev_backtransform_batched: memset W1");
-        if (rc != RENO_OK) return rc;
-      }
-      if (nfc > 0) {  // W1[s] = V_b^H K over row chunk s
-        GemmParams q;
-        q.M = kb;
-        q.N = o.kt;
-        q.K = KCH;
-        q.batch = nfc;
-        q.A = op(Vb, o.n, 1, 1);
-        q.A.s_batch = KCH;
-        q.B = op(Kb, 1, o.kt, 0);
-        q.B.s_batch = (int64_t)KCH * o.kt;
-        q.C = o.W1;
-        q.sCm = o.kt;
-        q.sCn = 1;
-        q.sCb = (int64_t)NB * o.kt;
-        if ((rc = add(g1, q, "reno_heev_backtransform_batched: V^H K")) != RENO_OK) return rc;
-      }
-      if (rem > 0) {
-        GemmParams q;
-        q.M = kb;
-        q.N = o.kt;
-        q.K = rem;
-        q.A = op(Vb + (size_t)nfc * KCH, o.n, 1, 1);
-        q.B = op(Kb + (size_t)nfc * KCH * o.kt, 1, o.kt, 0);
-        q.C = o.W1 + (size_t)nfc * NB * o.kt;
-        q.sCm = o.kt;
-        q.sCn = 1;
-        if ((rc = add(g1, q, "reno_heev_backtransform_batched: V^H K")) != RENO_OK) return rc;
-      }
-      GemmParams q2;  // W2 = (-T_b) sum_s W1[s]
+      GemmParams q1;  // W1 = V_b^H K
+      q1.M = kb;
+      q1.N = o.kt;
+      q1.K = rows;
+      q1.A = op(Vb, o.n, 1, 1);
+      q1.B = op(Kb, 1, o.kt, 0);
+      q1.C = o.W1;
+      q1.sCm = o.kt;
+      q1.sCn = 1;
+      if ((rc = add(g1, q1, "reno_heev_backtransform_batched: V^H K")) != RENO_OK) return rc;
+      GemmParams q2;  // W2 = (-T_b) W1
       q2.M = kb;
       q2.N = o.kt;
-      q2.K = NB * nch;
-      q2.A = op(o.Tg + (size_t)b * NB * NB * o.rep, (int64_t)NB * o.rep, 1, 0);
+      q2.K = kb;
+      q2.A = op(o.Tg + (size_t)b * NB * NB, NB, 1, 0);
       q2.B = op(o.W1, 1, o.kt, 0);
       q2.C = o.W2;
       q2.sCm = o.kt;
