@@ -6,16 +6,18 @@
 // (zlarfg / dlarfg), and Q = H_0 H_1 ... H_{kq-1} [I; 0].
 //
 // Blocked right-looking algorithm, panels of nb columns:
-//   qr_panel_kernel  one 8-CTA thread-block cluster per matrix factorises the
-//                    panel: the panel's rows are split over the cluster's
-//                    shared memories, the column norms and the w = v^H A
-//                    products are reduced through distributed shared memory
-//                    (every CTA sums the 8 partials in the same order, so the
-//                    Householder scalars agree bit for bit), two cluster
-//                    barriers per column.  It writes R's rows and the
-//                    reflectors back, the explicit unit-lower V of the panel
-//                    and the panel's triangular factor T (H_p0 ... H_p0+nb-1
-//                    = I - V T V^H, LAPACK's forward columnwise zlarft).
+//   panel kernels    one 8-CTA thread-block cluster per matrix factorises the
+//                    panel, its rows split over the CTAs.  Up to 4096 rows
+//                    (8192 real) the panel lives in registers
+//                    (qr_panel_reg_kernel, one cluster barrier per column);
+//                    taller matrices keep it in shared memory
+//                    (qr_panel_kernel, two barriers per column).  The
+//                    partial sums are added in the same order by every CTA,
+//                    so the Householder scalars agree bit for bit.  Both
+//                    write R's rows and the reflectors back, the explicit
+//                    unit-lower V of the panel and the panel's triangular
+//                    factor T (H_p0 ... H_p0+nb-1 = I - V T V^H, LAPACK's
+//                    forward columnwise zlarft).
 //   trailing update  A[p0:, p0+nb:] -= V (T^H (V^H A[p0:, p0+nb:])): three
 //                    grouped FP64 GEMMs over every matrix of the batch.
 //   Q                Q = [I; 0], then for the panels from last to first
@@ -70,12 +72,24 @@ struct Elem<true> {
   static __device__ __forceinline__ T mul(T a, T b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
   }
+  // c + a b and c - a b in four fused operations
+  static __device__ __forceinline__ T mac(T c, T a, T b) {
+    return make_double2(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
+  }
+  static __device__ __forceinline__ T msub(T c, T a, T b) {
+    return make_double2(fma(a.y, b.y, fma(-a.x, b.x, c.x)), fma(-a.y, b.x, fma(-a.x, b.y, c.y)));
+  }
   static __device__ __forceinline__ T conj(T a) { return make_double2(a.x, -a.y); }
   static __device__ __forceinline__ T neg(T a) { return make_double2(-a.x, -a.y); }
   static __device__ __forceinline__ double abs2(T a) { return a.x * a.x + a.y * a.y; }
   static __device__ __forceinline__ T shfl_xor(T v, int o) {
     return make_double2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
   }
+  static __device__ __forceinline__ T shfl(T v, int l) {
+    return make_double2(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
+  }
+  static __device__ __forceinline__ double real(T a) { return a.x; }
+  static __device__ __forceinline__ T from(double x) { return make_double2(x, 0.0); }
 };
 template <>
 struct Elem<false> {
@@ -85,10 +99,15 @@ struct Elem<false> {
   static __device__ __forceinline__ T add(T a, T b) { return a + b; }
   static __device__ __forceinline__ T sub(T a, T b) { return a - b; }
   static __device__ __forceinline__ T mul(T a, T b) { return a * b; }
+  static __device__ __forceinline__ T mac(T c, T a, T b) { return fma(a, b, c); }
+  static __device__ __forceinline__ T msub(T c, T a, T b) { return fma(-a, b, c); }
   static __device__ __forceinline__ T conj(T a) { return a; }
   static __device__ __forceinline__ T neg(T a) { return -a; }
   static __device__ __forceinline__ double abs2(T a) { return a * a; }
   static __device__ __forceinline__ T shfl_xor(T v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+  static __device__ __forceinline__ T shfl(T v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+  static __device__ __forceinline__ double real(T a) { return a; }
+  static __device__ __forceinline__ T from(double x) { return x; }
 };
 
 template <bool C>
@@ -312,6 +331,228 @@ __global__ void __cluster_dims__(QCL, 1, 1) __launch_bounds__(QT, 1)
   cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
+// ---------------------------------------------------------------- register panels
+// The same panel with its entries in registers: warp w owns the columns
+// c = w + 8 s (s < NC), lane l the rows l + 32 i (i < R) of the CTA's chunk.
+// What bounds it is the chain per column, so that chain is one reduction and
+// one cluster barrier: with x the pivot column below the diagonal, every warp
+// has S_c = sum_r conj(x_r) A[r, c] of its columns ready, taken in the pass
+// that applied the previous reflector; S of the pivot itself is ||x||^2, so
+// beta, tau and the scale of v follow, and w_c = A[p, c] + conj(scale) S_c is
+// the row the update needs.  Columns left of the pivot hold reflectors, whose
+// S_c give the column of V^H V that T needs.  The partial S and the pivot row
+// are pushed into every CTA's shared memory before the barrier, so that all
+// reads after it are local.  A 2048 x 128 pair of complex matrices takes
+// 121 us per 32-column panel, 517 us in the shared-memory kernel (two
+// reductions, two cluster barriers and 200 KB of shared-memory traffic per
+// column).
+template <bool C>
+struct RegShared {
+  using T = typename Elem<C>::T;
+  T part[2][QCL][NBMAX];     // the CTAs' partial S, by column parity
+  T row[2][NBMAX];           // the pivot row
+  T tau[NBMAX];
+  T gram[NBMAX * NBMAX];     // V^H V above the diagonal
+  T tsm[NBMAX * NBMAX];      // T of the panel
+  T tmp[NBMAX * NBMAX / 2];
+};
+
+// v[s] of a register array by selects (an index would put the array in local memory)
+template <int NC, typename T>
+__device__ __forceinline__ T pick(const T (&v)[NC], int s) {
+  if constexpr (NC == 2) {
+    return (s & 1) ? v[1] : v[0];
+  } else {
+    const T lo = (s & 1) ? v[1] : v[0], hi = (s & 1) ? v[3] : v[2];
+    return (s & 2) ? hi : lo;
+  }
+}
+
+template <bool C, int NC, int R>
+constexpr size_t reg_panel_smem() {
+  return sizeof(RegShared<C>) + (2 * 32 * R + 32 * R * (8 * NC + 1)) * sizeof(typename Elem<C>::T);
+}
+
+template <bool C, int NC, int R>
+__global__ void __cluster_dims__(QCL, 1, 1) __launch_bounds__(QT, 1)
+    qr_panel_reg_kernel(const __grid_constant__ Table tab, int p0, int nb) {
+  using E = Elem<C>;
+  using T = typename E::T;
+  constexpr int W = 8 * NC;  // columns held; nb == W
+  constexpr int SP = W + 1;  // row pitch of the staging buffer
+  cg::cluster_group cluster = cg::this_cluster();
+  const Prob& P = tab.p[blockIdx.y];
+  if (p0 >= P.kq) return;  // every CTA of this cluster returns here together
+  const int rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nbp = min(nb, P.kq - p0);
+  const int mr = P.m - p0;
+  const int chunk = (mr + QCL - 1) / QCL;  // <= 32 R
+  const int r0 = min(mr, rank * chunk), r1 = min(mr, r0 + chunk);
+  const int nr = r1 - r0;
+  T* A = reinterpret_cast<T*>(P.a);
+  const int lda = P.k;
+
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RegShared<C>& sh = *reinterpret_cast<RegShared<C>*>(smem_raw);
+  T* xs = reinterpret_cast<T*>(smem_raw + sizeof(RegShared<C>));  // 2 x 32 R: the pivot column
+  T* stage = xs + 2 * 32 * R;                                     // 32 R x SP
+
+  for (int idx = tid; idx < nr * W; idx += QT) {
+    const int rl = idx / W, c = idx % W;
+    stage[rl * SP + c] = c < nbp ? A[(size_t)(p0 + r0 + rl) * lda + p0 + c] : E::zero();
+  }
+  __syncthreads();
+  T a[R][NC];
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int s = 0; s < NC; ++s) {
+      const int rl = lane + 32 * i;
+      a[i][s] = rl < nr ? stage[rl * SP + warp + 8 * s] : E::zero();
+    }
+
+  cluster.sync();  // no CTA pushes into another before that one runs
+  for (int j = 0; j < nbp; ++j) {
+    const int par = j & 1;
+    T* x = xs + par * 32 * R;
+    // ---- column j (its owner warp) into xs, then the partial S of every column
+    // against it over rows r > j, and row j, pushed to every CTA
+    if (warp == (j & 7)) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const T t = pick<NC>(a[i], j >> 3);
+        x[lane + 32 * i] = (r0 + lane + 32 * i > j) ? t : E::zero();
+      }
+    }
+    __syncthreads();
+    T acc[NC];
+#pragma unroll
+    for (int s = 0; s < NC; ++s) acc[s] = E::zero();
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      // rows up to j hold R and earlier reflectors' heads, not to be summed even where not finite
+      const bool below = r0 + lane + 32 * i > j;
+      const T xc = E::conj(x[lane + 32 * i]);
+#pragma unroll
+      for (int s = 0; s < NC; ++s)
+        if (below) acc[s] = E::mac(acc[s], xc, a[i][s]);
+    }
+#pragma unroll
+    for (int s = 0; s < NC; ++s) acc[s] = warp_sum<C>(acc[s]);
+    {
+      // row j < 32 of the panel is in register row 0 of lane j - r0 of its CTA
+      const int rl = j - r0;
+      const bool mine = rl >= 0 && rl < nr;
+      RegShared<C>* o = cluster.map_shared_rank(&sh, lane & 7);
+      T rv[NC];
+#pragma unroll
+      for (int s = 0; s < NC; ++s) rv[s] = E::shfl(a[0][s], rl & 31);
+      const int sl = lane >> 3;  // lane -> (CTA, column): 8 x NC pushes
+      const T pa = pick<NC>(acc, sl), pr = pick<NC>(rv, sl);
+      if (sl < NC) {
+        o->part[par][rank][warp + 8 * sl] = pa;
+        if (mine) o->row[par][warp + 8 * sl] = pr;
+      }
+    }
+    cluster.sync();
+    // ---- every warp: lane c holds S_c and the pivot row's entry of column c
+    T S = E::zero(), row = E::zero();
+    if (lane < W) {
+#pragma unroll
+      for (int q = 0; q < QCL; ++q) S = E::add(S, sh.part[par][q][lane]);
+      row = sh.row[par][lane];
+    }
+    const T alpha = E::shfl(row, j);
+    const double xn2 = E::real(E::shfl(S, j));
+    double beta;
+    T tau, scale;
+    householder<C>(alpha, xn2, beta, tau, scale);
+    if (warp == 0) {
+      if (lane == j) sh.tau[j] = tau;
+      if (lane < j) sh.gram[lane * NBMAX + j] = E::add(E::conj(row), E::mul(scale, E::conj(S)));
+    }
+    const T w = E::mul(E::conj(tau), E::add(row, E::mul(E::conj(scale), S)));  // conj(tau) w_c
+    T u[NC];
+#pragma unroll
+    for (int s = 0; s < NC; ++s) u[s] = E::shfl(w, warp + 8 * s);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int r = r0 + lane + 32 * i;
+      const T v = r == j ? E::one() : E::mul(x[lane + 32 * i], scale);
+#pragma unroll
+      for (int s = 0; s < NC; ++s) {
+        const int c = warp + 8 * s;
+        const T upd = E::msub(a[i][s], v, u[s]);
+        const T own = r == j ? E::from(beta) : v;
+        const T nv = c == j ? own : upd;
+        if (r >= j && c >= j) a[i][s] = nv;
+      }
+    }
+  }
+
+  // ---- write back R rows / reflectors and the explicit V of this panel
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int s = 0; s < NC; ++s)
+      if (lane + 32 * i < nr) stage[(lane + 32 * i) * SP + warp + 8 * s] = a[i][s];
+  __syncthreads();
+  T* V = reinterpret_cast<T*>(P.v);
+  for (int idx = tid; idx < nr * nbp; idx += QT) {
+    const int rl = idx / nbp, c = idx % nbp;
+    const int r = r0 + rl;
+    const T x = stage[rl * SP + c];
+    A[(size_t)(p0 + r) * lda + p0 + c] = x;
+    V[(size_t)(p0 + r) * P.kq + p0 + c] = (r == c) ? E::one() : (r > c ? x : E::zero());
+  }
+  if (rank == 0) {
+    // T = (diag(1 / tau) + striu(V^H V))^-1 by doubling: with the two
+    // diagonal blocks of order h known, T12 = -T11 (V^H V)12 T22
+    for (int e = tid; e < NBMAX * NBMAX; e += QT) {
+      const int i = e / NBMAX, c = e % NBMAX;
+      sh.tsm[e] = (i == c && i < nbp) ? sh.tau[i] : E::zero();
+    }
+    __syncthreads();
+    for (int h = 1; h < nbp; h *= 2) {
+      // entry (i, c) of the off-diagonal block of pair q: rows q 2h + i, columns q 2h + h + c
+      const int pairs = NBMAX / (2 * h), n = pairs * h * h;
+      for (int e = tid; e < n; e += QT) {
+        const int q = e / (h * h), i = (e / h) % h, c = e % h;
+        const int ri = 2 * h * q + i, ci = 2 * h * q + h;
+        T acc = E::zero();
+        if (ci + c < nbp)
+          for (int l = 0; l <= c; ++l)
+            acc = E::add(acc, E::mul(sh.gram[ri * NBMAX + ci + l], sh.tsm[(ci + l) * NBMAX + ci + c]));
+        sh.tmp[e] = acc;
+      }
+      __syncthreads();
+      for (int e = tid; e < n; e += QT) {
+        const int q = e / (h * h), i = (e / h) % h, c = e % h;
+        const int r2 = 2 * h * q;
+        T acc = E::zero();
+        if (r2 + h + c < nbp)
+          for (int l = i; l < h; ++l)
+            acc = E::add(acc, E::mul(sh.tsm[(r2 + i) * NBMAX + r2 + l], sh.tmp[q * h * h + l * h + c]));
+        if (r2 + h + c < nbp) sh.tsm[(r2 + i) * NBMAX + r2 + h + c] = E::neg(acc);
+      }
+      __syncthreads();
+    }
+    const int pi = p0 / nb;
+    T* Tm = reinterpret_cast<T*>(P.t) + (size_t)pi * nb * nb;
+    T* NT = reinterpret_cast<T*>(P.nt) + (size_t)pi * nb * nb;
+    T* NTH = reinterpret_cast<T*>(P.nth) + (size_t)pi * nb * nb;
+    for (int e = tid; e < nb * nb; e += QT) {
+      const int i = e / nb, j = e % nb;
+      const T t = sh.tsm[i * NBMAX + j];
+      Tm[e] = t;
+      NT[e] = E::neg(t);
+      NTH[e] = E::neg(E::conj(sh.tsm[j * NBMAX + i]));
+    }
+  }
+}
+
 // Q = [I; 0] (m x kq) for every matrix of the table
 template <bool C>
 __global__ void qr_init_q_kernel(const __grid_constant__ Table tab) {
@@ -348,18 +589,29 @@ namespace {
 
 size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// panel width: the largest power of two <= 32 whose panel rows fit a CTA
-int panel_width(int mmax) {
+// Panel of the tallest matrix of a call: width nb, and the register kernel's
+// rows per lane (0: the shared-memory kernel).  A lane holds 32 complex or 64
+// real entries, so wider panels trade for taller ones: 32 columns up to 2048
+// (4096 real) rows, 16 up to 4096 (8192 real); beyond, the shared-memory
+// kernel at the largest power of two <= 32 whose rows fit a CTA.
+struct Panel {
+  int nb, rpl;
+};
+Panel panel_of(int mmax, bool cplx) {
   const int rows = (mmax + qr::QCL - 1) / qr::QCL;
+  const int cap = cplx ? 8 : 16;
+  for (int rpl = 2; rpl <= cap; rpl *= 2)
+    if (rows <= 32 * rpl) return Panel{32, rpl};
+  if (rows <= 32 * 2 * cap) return Panel{16, 2 * cap};
   int nb = qr::NBMAX;
   while (nb > 1 && (size_t)rows * nb > (size_t)qr::PANEL_ELEMS) nb >>= 1;
-  return (size_t)rows * nb <= (size_t)qr::PANEL_ELEMS ? nb : 0;
+  return Panel{(size_t)rows * nb <= (size_t)qr::PANEL_ELEMS ? nb : 0, 0};
 }
 
 struct Layout {
   size_t off[RENO_QR_MAX_BLOCKS][7];
   size_t total = 0;
-  int nb = 0;
+  int nb = 0, rpl = 0;
 };
 
 int plan(int32_t count, const reno_qr_block* b, Layout& L, std::string& why) {
@@ -376,7 +628,9 @@ int plan(int32_t count, const reno_qr_block* b, Layout& L, std::string& why) {
     }
     mmax = std::max(mmax, (int)b[i].m);
   }
-  L.nb = panel_width(mmax);
+  const Panel pan = panel_of(mmax, b[0].dtype == RENO_C128);
+  L.nb = pan.nb;
+  L.rpl = pan.rpl;
   if (L.nb == 0) {
     why = "reno_qr_blocks: " + std::to_string(mmax) + " rows exceed the panel capacity";
     return RENO_ERR_UNSUPPORTED;
@@ -396,6 +650,17 @@ int plan(int32_t count, const reno_qr_block* b, Layout& L, std::string& why) {
   }
   L.total = o;
   return RENO_OK;
+}
+
+template <bool C, int NC, int R>
+cudaError_t launch_reg_panel(const qr::Table& tab, int p0, int nb, cudaStream_t st) {
+  constexpr size_t smem = qr::reg_panel_smem<C, NC, R>();
+  static std::atomic<unsigned long long> set{0};
+  const cudaError_t e = smem_optin_once(qr::qr_panel_reg_kernel<C, NC, R>, (int)smem, set);
+  if (e != cudaSuccess) return e;
+  count_launch();
+  qr::qr_panel_reg_kernel<C, NC, R><<<dim3(qr::QCL, tab.count), qr::QT, smem, st>>>(tab, p0, nb);
+  return cudaGetLastError();
 }
 
 GemmOperand op(const void* p, int64_t s_outer, int64_t s_k, bool cplx, bool conj = false) {
@@ -463,17 +728,38 @@ extern "C" int reno_qr_blocks(reno_ctx* ctx, int32_t count, const reno_qr_block*
       ((size_t)rows * nb + 2 * qr::NBMAX + qr::NBMAX + 2 * qr::NBMAX * qr::NBMAX + 2 * qr::NBMAX) * es;
   // the opt-in is made once per device, so it covers the largest panel any call can use
   const int smem_max = (int)(((size_t)qr::PANEL_ELEMS + 5 * qr::NBMAX + 2 * qr::NBMAX * qr::NBMAX) * 16);
-  static std::atomic<unsigned long long> set_c{0}, set_r{0};
-  cudaError_t e = cplx ? smem_optin_once(qr::qr_panel_kernel<true>, smem_max, set_c)
-                       : smem_optin_once(qr::qr_panel_kernel<false>, smem_max, set_r);
-  if (e != cudaSuccess) return check_cuda(ctx, e, "reno_qr_blocks: shared-memory opt-in");
+  auto launch_panel = [&](int p0) -> cudaError_t {
+    if (L.rpl == 0) {
+      static std::atomic<unsigned long long> set_c{0}, set_r{0};
+      const cudaError_t e = cplx ? smem_optin_once(qr::qr_panel_kernel<true>, smem_max, set_c)
+                                 : smem_optin_once(qr::qr_panel_kernel<false>, smem_max, set_r);
+      if (e != cudaSuccess) return e;
+      count_launch();
+      if (cplx) qr::qr_panel_kernel<true><<<dim3(qr::QCL, count), qr::QT, smem, st>>>(tab, p0, nb);
+      else qr::qr_panel_kernel<false><<<dim3(qr::QCL, count), qr::QT, smem, st>>>(tab, p0, nb);
+      return cudaGetLastError();
+    }
+    if (cplx) {
+      switch (L.rpl) {
+        case 2: return launch_reg_panel<true, 4, 2>(tab, p0, nb, st);
+        case 4: return launch_reg_panel<true, 4, 4>(tab, p0, nb, st);
+        case 8: return launch_reg_panel<true, 4, 8>(tab, p0, nb, st);
+        default: return launch_reg_panel<true, 2, 16>(tab, p0, nb, st);
+      }
+    }
+    switch (L.rpl) {
+      case 2: return launch_reg_panel<false, 4, 2>(tab, p0, nb, st);
+      case 4: return launch_reg_panel<false, 4, 4>(tab, p0, nb, st);
+      case 8: return launch_reg_panel<false, 4, 8>(tab, p0, nb, st);
+      case 16: return launch_reg_panel<false, 4, 16>(tab, p0, nb, st);
+      default: return launch_reg_panel<false, 2, 32>(tab, p0, nb, st);
+    }
+  };
 
   // ---- factorisation, panel by panel
   for (int p0 = 0; p0 < kqmax; p0 += nb) {
-    count_launch();
-    if (cplx) qr::qr_panel_kernel<true><<<dim3(qr::QCL, count), qr::QT, smem, st>>>(tab, p0, nb);
-    else qr::qr_panel_kernel<false><<<dim3(qr::QCL, count), qr::QT, smem, st>>>(tab, p0, nb);
-    RENO_LAUNCH_CHECK(ctx, "reno_qr_blocks: panel");
+    rc = check_cuda(ctx, launch_panel(p0), "reno_qr_blocks: panel");
+    if (rc != RENO_OK) return rc;
     fp64gemm::GemmGroup g1, g2, g3;
     for (int i = 0; i < count; ++i) {
       const qr::Prob& P = tab.p[i];
