@@ -25,8 +25,10 @@ The caller falls back to cuSOLVER for a block whose check fails.
 """
 from __future__ import annotations
 
+import math
 import os
 
+import numpy as np
 import torch
 
 from ._native import HEEV_MAX_BATCH, Engine, HeevProblem
@@ -128,3 +130,121 @@ def _heev_chunk(eng, Gs, kts):
                                    res]))
     eng.heev_batched(probs, status, ws, "back")
     return [(torch.flip(m[6], dims=[0]), K, chk) for m, K, chk in zip(mats, Ks, checks)]
+
+
+class LowRankOptions:
+    """Leading eigenpairs of a Gram matrix G = M^H M from its numerical range.
+
+    The Gram matrix of a coefficient whose singular values decay over the
+    kept ones has few eigenvalues above its own rounding errors (8 decades of
+    sigma are 16 of lambda), while forming it and reducing all of its n
+    columns to a tridiagonal matrix costs the same however few they are.  For
+    n >= ``min_ratio`` r the range is found first (Halko, Martinsson, Tropp,
+    SIAM Rev. 53, 2011): Q = orth(M^H (M Omega)) with r >= kt + ``oversample``
+    seeded Gaussian columns, B = M Q, T = B^H B.  T goes through the
+    device eigensolver, and with its eigenvectors S the wanted ones are
+    K = Q S and the projected block M K = B S, so G itself is never formed.
+
+    The result is kept only where Q carries all of G to its rounding level:
+    the invariance ||M^H B - Q T||_F <= ``tol`` ||T||_F, and the trace that is
+    missing, ||M||_F^2 - ||B||_F^2 <= ``tol`` ||M||_F^2, which bounds every
+    eigenvalue left out because G is positive semidefinite.  That is the size
+    of the dense reduction's own backward error.  A block that misses either
+    goes through the dense path.
+
+    r comes from a sketch of ``probe`` columns, whose R factor's diagonal
+    falls like the eigenvalues: the slope of its logarithm extrapolated to
+    rounding level (with 15 % more, for the sketch's scatter), at least
+    kt + oversample and at most n / min_ratio.  Where that upper limit is
+    below 0.7 of the extrapolation the block is not tried.
+
+    Truncation of a complex 4096 x 4096 coefficient with two 2048^2 blocks
+    to 256: 54 -> 16 ms with sigma falling 3.5 decades over the kept ones,
+    27 ms with 1.5 decades; a flat spectrum pays 0.5 ms for the probe."""
+
+    def __init__(self, min_ratio=2.5, oversample=96, probe=32, tol=2e-14):
+        self.min_ratio, self.oversample, self.probe, self.tol = min_ratio, oversample, probe, tol
+        self.calls = 0
+        self.missed = 0
+
+
+lowrank_opts = LowRankOptions()
+
+
+def _range_columns(n: int, kt: int, diag=None) -> int:
+    """Columns of the range sketch for kt eigenpairs of order n, given the
+    diagonal of its probe's R factor; 0 = dense path."""
+    least = (kt + lowrank_opts.oversample + 31) // 32 * 32
+    most = int(n / lowrank_opts.min_ratio) // 32 * 32
+    if least > most or diag is None:
+        return least if least <= most else 0
+    eps = np.finfo(np.float64).eps
+    if not (diag[0] > 0 and np.all(np.isfinite(diag))):
+        return 0
+    j = np.arange(4, len(diag))
+    slope = -np.polyfit(j, np.log(np.maximum(diag[4:] / diag[0], eps * eps)), 1)[0]
+    need = -math.log(eps) / slope if slope > 0 else math.inf
+    if most < 0.7 * need:
+        return 0
+    return min(most, max(least, (int(1.15 * need) + 31) // 32 * 32))
+
+
+def lowrank_top_batched(eng: Engine, Ms, kts):
+    """The kts[i] largest eigenpairs of each Gram matrix G = M^H M through its
+    numerical range (LowRankOptions).  Ms: (matrix, adjoint) pairs, M the
+    matrix or, with adjoint, its conjugate transpose.  Returns per entry
+    (w, K, check, M K) -- w, K and check like heev_top_batched, with 1 in the
+    check's second entry where the range misses part of G -- or None where
+    the dense path is to be taken."""
+    out = [None] * len(Ms)
+    size = lambda i: Ms[i][0].shape[0 if Ms[i][1] else 1]
+    idx = [i for i, kt in enumerate(kts) if _range_columns(size(i), kt)]
+    if not idx:
+        return out
+
+    def fwd(i, v):  # M v
+        X, adj = Ms[i]
+        return eng.matmul(X.transpose(0, 1), v, conj_a=True) if adj else eng.matmul(X, v)
+
+    def back(i, v):  # M^H v
+        X, adj = Ms[i]
+        return eng.matmul(X, v) if adj else eng.matmul(X.transpose(0, 1), v, conj_a=True)
+
+    dev = Ms[0][0].device
+
+    def sketch(i, cols, seed):  # seeded by its shape alone: a block's result does not depend on the batch it is in
+        gen = torch.Generator(device=dev).manual_seed(seed)
+        return back(i, fwd(i, torch.randn((size(i), cols), dtype=torch.float64, device=dev, generator=gen)))
+
+    Rs = _qr_by_type(eng, [sketch(i, lowrank_opts.probe, 0x5EED) for i in idx])[1]
+    diag = torch.stack([torch.diagonal(R).abs() for R in Rs]).cpu().numpy()
+    rs = {i: _range_columns(size(i), kts[i], d) for i, d in zip(idx, diag)}
+    idx = [i for i in idx if rs[i]]
+    if not idx:
+        return out
+    lowrank_opts.calls += len(idx)
+    Qs = _qr_by_type(eng, [sketch(i, rs[i], 0x5EED + 1) for i in idx])[0]
+    Bs = [fwd(i, Q) for i, Q in zip(idx, Qs)]
+    Ts = [eng.matmul(B.transpose(0, 1), B, conj_a=True) for B in Bs]
+    eig = heev_top_batched(eng, Ts, [kts[i] for i in idx])
+    norm = torch.linalg.vector_norm
+    for i, Q, B, T, (w, S, chk) in zip(idx, Qs, Bs, Ts, eig):
+        res = norm(back(i, B) - eng.matmul(Q, T)) / norm(T)
+        full = norm(Ms[i][0]) ** 2
+        miss = (full - norm(B) ** 2) / full
+        fail = ~((res <= lowrank_opts.tol) & (miss <= lowrank_opts.tol))
+        S = S if Q.is_complex() else S.real.contiguous()
+        out[i] = (w, eng.matmul(Q, S), torch.stack([chk[0], fail.to(torch.float64), chk[2]]), eng.matmul(B, S))
+    return out
+
+
+def _qr_by_type(eng: Engine, mats):
+    """Engine.qr_blocks for matrices of both types"""
+    Qs, Rs = [None] * len(mats), [None] * len(mats)
+    for cplx in (False, True):
+        idx = [i for i, m in enumerate(mats) if m.is_complex() == cplx]
+        if idx:
+            q, r = eng.qr_blocks([mats[i] for i in idx])
+            for i, a, b in zip(idx, q, r):
+                Qs[i], Rs[i] = a, b
+    return Qs, Rs

@@ -491,22 +491,28 @@ def _gram_eigh(eng: Engine, G: torch.Tensor, kt: int, use_heev: bool):
     return torch.flip(w, dims=[0]), torch.flip(V, dims=[1]), None
 
 
-def _gram_of(eng: Engine, X: torch.Tensor, keep_left: bool):
-    """(G, left) with G the Gram matrix of X's smaller side, X X^H (left) or
-    X^H X; a square block takes the kept side."""
+def _gram_is_left(X: torch.Tensor, keep_left: bool) -> bool:
+    """whether the Gram matrix of X's smaller side is X X^H; a square block takes the kept side"""
     m, n = X.shape
-    if m < n or (m == n and keep_left):
-        return eng.matmul(X, X.transpose(0, 1), conj_b=True), True
-    return eng.matmul(X.transpose(0, 1), X, conj_a=True), False
+    return m < n or (m == n and keep_left)
 
 
-def _finish_kept_side(eng: Engine, X: torch.Tensor, keep_left: bool, kt: int, w, E, chk, qr_out=None):
+def _gram_of(eng: Engine, X: torch.Tensor, keep_left: bool):
+    """The Gram matrix of X's smaller side, X X^H or X^H X"""
+    if _gram_is_left(X, keep_left):
+        return eng.matmul(X, X.transpose(0, 1), conj_b=True)
+    return eng.matmul(X.transpose(0, 1), X, conj_a=True)
+
+
+def _finish_kept_side(eng: Engine, X: torch.Tensor, keep_left: bool, kt: int, w, E, chk, qr_out=None, ME=None):
     """Kept-side basis K, projection P and sigma S of block X from the
     leading kt eigenvectors E of its smaller-side Gram matrix (w descending):
-    see _full_kept_side.  When the kept side is the larger one, the projected
-    vectors are orthonormalised by Householder QR; ``qr_out`` carries that QR
-    (computed for all blocks at once) and is None on the first pass, which
-    returns the matrix to factorise instead."""
+    see _full_kept_side.  ME: the other side's vectors E^H X or X E, as
+    columns (X^H E where the Gram matrix is X X^H), when they are known.
+    When the kept side is the larger one, those vectors are orthonormalised
+    by Householder QR; ``qr_out`` carries that QR (computed for all blocks at
+    once) and is None on the first pass, which returns the matrix to
+    factorise instead."""
     m, n = X.shape
     dim = min(m, n)
 
@@ -519,71 +525,87 @@ def _finish_kept_side(eng: Engine, X: torch.Tensor, keep_left: bool, kt: int, w,
 
     if keep_left and m <= n:
         K = E[:, :kt]
-        P = eng.matmul(K.transpose(0, 1).contiguous(), X, conj_a=True)       # (kt, n) = sigma Vh
+        if ME is None:
+            P = eng.matmul(K.transpose(0, 1).contiguous(), X, conj_a=True)   # (kt, n) = sigma Vh
+        else:
+            P = ME.mH.resolve_conj().contiguous()
         S = torch.linalg.vector_norm(P, dim=1)
         return dict(K=K, P=P, S=torch.cat([S, tail(w, S)]), dim=dim, chk=chk)
     if not keep_left and n <= m:
         K = E[:, :kt]
-        P = eng.matmul(X, K.contiguous())                                     # (m, kt) = U sigma
+        P = eng.matmul(X, K.contiguous()) if ME is None else ME               # (m, kt) = U sigma
         S = torch.linalg.vector_norm(P, dim=0)
         return dict(K=K, P=P, S=torch.cat([S, tail(w, S)]), dim=dim, chk=chk)
     if keep_left:
-        Us = eng.matmul(X, E[:, :kt].contiguous())                            # (m, kt) = U sigma
+        Us = eng.matmul(X, E[:, :kt].contiguous()) if ME is None else ME      # (m, kt) = U sigma
         if qr_out is None:
             return dict(need_qr=Us)
         S = torch.linalg.vector_norm(Us, dim=0)
         K = qr_out
         P = eng.matmul(K.transpose(0, 1).contiguous(), X, conj_a=True)
         return dict(K=K, P=P, S=torch.cat([S, tail(w, S)]), dim=dim, chk=chk)
-    Vs = eng.matmul(X.transpose(0, 1), E[:, :kt].contiguous(), conj_a=True)   # (n, kt): sigma v
+    if ME is None:
+        ME = eng.matmul(X.transpose(0, 1), E[:, :kt].contiguous(), conj_a=True)  # (n, kt): sigma v
     if qr_out is None:
-        return dict(need_qr=Vs)
-    S = torch.linalg.vector_norm(Vs, dim=0)
+        return dict(need_qr=ME)
+    S = torch.linalg.vector_norm(ME, dim=0)
     K = qr_out
     P = eng.matmul(X, K)
     return dict(K=K, P=P, S=torch.cat([S, tail(w, S)]), dim=dim, chk=chk)
 
 
 def _device_eig_ok(G: torch.Tensor) -> bool:
-    """whether the device eigensolver takes Gram block G (size 1 .. 4096)"""
-    n = G.shape[0]
+    """whether the device eigensolver takes the Gram matrix of G's smaller side (size 1 .. 4096)"""
+    n = min(G.shape)
     return heev.heev_opts.enabled and G.is_cuda and heev.heev_opts.min_n <= n <= 4096
 
 
-def _kept_sides(eng: Engine, Xs, keep_left: bool, ktops, use_heev: bool = True) -> list:
-    """_full_kept_side for all QN blocks of one truncation: one Gram matrix
-    per block, the device eigensolver on all of them at once
-    (heev_top_batched; blocks above its size limit, or with the device
-    eigensolver switched off, take cuSOLVER), and one batched Householder QR
-    where a projected basis needs orthonormalising."""
+def _kept_sides(eng: Engine, Xs, keep_left: bool, ktops, use_heev: bool = True, lowrank: bool = True) -> list:
+    """_full_kept_side for all QN blocks of one truncation: large blocks with
+    few eigenvalues above rounding through their numerical range
+    (heev.lowrank_top_batched), the others by their Gram matrix and the device
+    eigensolver on all of them at once (heev_top_batched; blocks above its
+    size limit, or with the device eigensolver switched off, take cuSOLVER),
+    and one batched Householder QR where a projected basis needs
+    orthonormalising."""
     items = []
     for X, ktop in zip(Xs, ktops):
-        m, n = X.shape
-        dim = min(m, n)
-        kt = dim if ktop is None else min(int(ktop), dim)
-        G, _ = _gram_of(eng, X, keep_left)
-        items.append(dict(X=X, G=G, kt=kt, dim=dim))
-    dev_idx = [i for i, it in enumerate(items) if use_heev and _device_eig_ok(it["G"])]
-    if dev_idx:
-        res = heev.heev_top_batched(eng, [items[i]["G"] for i in dev_idx], [items[i]["kt"] for i in dev_idx])
-        for i, (w, K, chk) in zip(dev_idx, res):
-            items[i].update(w=w, E=K if items[i]["G"].is_complex() else K.real.contiguous(), chk=chk)
+        dim = min(X.shape)
+        items.append(dict(X=X, kt=dim if ktop is None else min(int(ktop), dim), dim=dim, ME=None))
+    dev = [it for it in items if use_heev and _device_eig_ok(it["X"])]
+    if dev and lowrank:
+        res = heev.lowrank_top_batched(eng, [(it["X"], _gram_is_left(it["X"], keep_left)) for it in dev],
+                                       [it["kt"] for it in dev])
+        for it, r in zip(dev, res):
+            if r is not None:
+                it.update(w=r[0], E=r[1], chk=r[2], ME=r[3])
+        dev = [it for it, r in zip(dev, res) if r is None]
+    for it in items:
+        if "E" not in it:
+            it["G"] = _gram_of(eng, it["X"], keep_left)
+    if dev:
+        res = heev.heev_top_batched(eng, [it["G"] for it in dev], [it["kt"] for it in dev])
+        for it, (w, K, chk) in zip(dev, res):
+            it.update(w=w, E=K if it["G"].is_complex() else K.real.contiguous(), chk=chk)
     for it in items:
         if "E" not in it:
             w, V = torch.linalg.eigh(it["G"])
             it.update(w=torch.flip(w, dims=[0]), E=torch.flip(V, dims=[1]), chk=None)
-    outs = [_finish_kept_side(eng, it["X"], keep_left, it["kt"], it["w"], it["E"], it["chk"]) for it in items]
+    finish = lambda it, Q=None: _finish_kept_side(eng, it["X"], keep_left, it["kt"], it["w"], it["E"], it["chk"], Q,
+                                                  it["ME"])
+    outs = [finish(it) for it in items]
     need = [i for i, o in enumerate(outs) if "need_qr" in o]
     if need:
         Qs, _ = eng.qr_blocks([outs[i]["need_qr"] for i in need])
         for i, Q in zip(need, Qs):
-            it = items[i]
-            outs[i] = _finish_kept_side(eng, it["X"], keep_left, it["kt"], it["w"], it["E"], it["chk"], Q)
+            outs[i] = finish(items[i], Q)
+    for it, o in zip(items, outs):
+        o["lowrank"] = it["ME"] is not None
     return outs
 
 
 def _full_kept_side(eng: Engine, X: torch.Tensor, keep_left: bool, ktop: Optional[int] = None,
-                    use_heev: bool = True) -> dict:
+                    use_heev: bool = True, lowrank: bool = True) -> dict:
     """Kept-side basis K, projection P and sigma S of one block from the
     Hermitian eigendecomposition of the Gram matrix of its smaller side (all
     min(m, n) triplets).
@@ -599,7 +621,7 @@ def _full_kept_side(eng: Engine, X: torch.Tensor, keep_left: bool, ktop: Optiona
     entry sorts after every head entry of its block, and since a block
     contributes at most the cap (< ktop) entries, none is selected; they only
     fill the list the truncation rule reads."""
-    return _kept_sides(eng, [X], keep_left, [ktop], use_heev)[0]
+    return _kept_sides(eng, [X], keep_left, [ktop], use_heev, lowrank)[0]
 
 
 def svd_truncate(coef: torch.Tensor, qnbigl, qnbigr, qntot, keep_left: bool, m_trunc_fn, percent=0,
@@ -713,7 +735,7 @@ def _trunc_eig(states):
                 flop_log.append(_block_flops(m_, n_, b["ktop"] or min(m_, n_), b["X"].is_complex()))
         fulls = _kept_sides(states[0]["eng"], [b["X"] for b in group], keep_left, [b["ktop"] for b in group])
         for b, full in zip(group, fulls):
-            b.update(K=full["K"], P=full["P"], S=full["S"])
+            b.update(K=full["K"], P=full["P"], S=full["S"], lowrank=full["lowrank"])
             if full["chk"] is not None:
                 b["chk"] = full["chk"]
             else:
@@ -838,7 +860,14 @@ def _trunc_select(st, host):
         off += b["dim"]
     off_chk = off + 2 * len(sub)
     for i, b in enumerate(dev_eig):
-        if not heev.accepted(host[off_chk + 3 * i: off_chk + 3 * i + 3]):
+        ok = heev.accepted(host[off_chk + 3 * i: off_chk + 3 * i + 3])
+        if not ok and b["lowrank"]:
+            # part of the block's Gram matrix lies outside the sketched range: the dense device path
+            heev.lowrank_opts.missed += 1
+            b.update(_full_kept_side(eng, b["X"], keep_left, b["ktop"], lowrank=False))
+            host_b = torch.cat([b["S"], b["chk"]]).cpu().numpy()
+            b["Sh"], ok = host_b[:b["dim"]], heev.accepted(host_b[b["dim"]:])
+        if not ok:
             # the device eigensolver missed its checks on this block: cuSOLVER
             heev.heev_opts.fallbacks += 1
             b.update(_full_kept_side(eng, b["X"], keep_left, b["ktop"], use_heev=False))
