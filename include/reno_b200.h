@@ -422,6 +422,14 @@ int reno_vec_precond(reno_ctx* ctx, int64_t n, int32_t dtype, const void* r,
  *                      k = j vectors)
  *   RENO_VOP_ALLCLOSE  scalars[0] = allclose(x, y, rtol, atol)
  *                      (reno_vec_allclose)
+ *   RENO_VOP_STEP      one Lanczos step, krylov.py:231-256: ALPHA, ORTH and
+ *                      V[j+1] = w / beta_j with x = V[j], y = V[j-1], out = w
+ *                      (scratch afterwards), scalars = ab, V[j+1] at x + ldv;
+ *                      one launch up to 65536 complex (131072 real)
+ *                      elements, those three otherwise
+ *   RENO_VOP_CHECK     out = sum_{i<j} s[2i..] x[i ldv ..]; scalars[0] =
+ *                      allclose(the sum over i < j - 2 with the coefficients
+ *                      that follow in s, out, rtol, atol), krylov.py:252
  * workspace: reno_vec_grouped_workspace_bytes(count) bytes.
  * ---------------------------------------------------------------------- */
 enum {
@@ -430,7 +438,9 @@ enum {
   RENO_VOP_ORTH = 2,
   RENO_VOP_SCALE_INV = 3,
   RENO_VOP_LINCOMB = 4,
-  RENO_VOP_ALLCLOSE = 5
+  RENO_VOP_ALLCLOSE = 5,
+  RENO_VOP_STEP = 6,
+  RENO_VOP_CHECK = 7
 };
 #define RENO_VEC_GROUP_MAX 128
 typedef struct {

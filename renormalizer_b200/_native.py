@@ -58,7 +58,7 @@ class VecItem(ctypes.Structure):
 
 
 VEC_GROUP_MAX = 128
-VOP_NORM, VOP_ALPHA, VOP_ORTH, VOP_SCALE_INV, VOP_LINCOMB, VOP_ALLCLOSE = range(6)
+VOP_NORM, VOP_ALPHA, VOP_ORTH, VOP_SCALE_INV, VOP_LINCOMB, VOP_ALLCLOSE, VOP_STEP, VOP_CHECK = range(8)
 
 
 class EnvDesc(ctypes.Structure):

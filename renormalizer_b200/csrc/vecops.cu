@@ -4,6 +4,10 @@
 // and the diagonal preconditioner.  Reductions are two-pass with a fixed
 // block count and fixed summation order, so results are bitwise
 // reproducible run to run (no atomics).
+#include <algorithm>
+#include <cooperative_groups.h>
+#include <type_traits>
+#include <vector>
 #include "reno_common.cuh"
 
 namespace reno {
@@ -125,16 +129,46 @@ __device__ __forceinline__ void lincomb_body(int64_t n, int k, bool cplx, const 
   }
 }
 
+// numpy's allclose of one element: |a - b| <= atol + rtol |b|
+__device__ __forceinline__ bool close_(double2 x, double2 y, bool cplx, double rtol, double atol) {
+  const double dx = x.x - y.x, dy = x.y - y.y;
+  const double diff = cplx ? hypot(dx, dy) : fabs(dx);
+  const double mag = cplx ? hypot(y.x, y.y) : fabs(y.x);
+  return diff <= fma_(rtol, mag, atol);
+}
+
+// out = sum_{j<k} coef[j] V[j], and the count of its elements that the
+// combination of the first k - 2 vectors (coefficients after the k) is not
+// close to: both combinations from one read of the vectors
+__device__ __forceinline__ double2 check_body(int64_t n, int k, bool cplx, const void* V, int64_t ldv,
+                                              const double* coef, void* out, double rtol, double atol, int64_t b,
+                                              int64_t nb) {
+  double2 bad = make_double2(0.0, 0.0);
+  for (int64_t i = b * VT + threadIdx.x; i < n; i += nb * VT) {
+    double2 cur = make_double2(0.0, 0.0), prev = make_double2(0.0, 0.0);
+    for (int j = 0; j < k; ++j) {
+      const double2 v = ld2(V, (int64_t)j * ldv + i, cplx);
+      const double cr = coef[2 * j], ci = coef[2 * j + 1];
+      cur.x = add_(cur.x, fma_(cr, v.x, -mul_(ci, v.y)));
+      cur.y = add_(cur.y, fma_(cr, v.y, mul_(ci, v.x)));
+      if (j < k - 2) {
+        const double pr = coef[2 * (k + j)], pi = coef[2 * (k + j) + 1];
+        prev.x = add_(prev.x, fma_(pr, v.x, -mul_(pi, v.y)));
+        prev.y = add_(prev.y, fma_(pr, v.y, mul_(pi, v.x)));
+      }
+    }
+    st2(out, i, cplx, cur);
+    if (!close_(prev, cur, cplx, rtol, atol)) bad.x += 1.0;
+  }
+  return bad;
+}
+
 // count of elements violating |a-b| <= atol + rtol |b|
 __device__ __forceinline__ double2 allclose_body(int64_t n, bool cplx, const void* a, const void* b_, double rtol,
                                                  double atol, int64_t b, int64_t nb) {
   double2 acc = make_double2(0.0, 0.0);
   for (int64_t i = b * VT + threadIdx.x; i < n; i += nb * VT) {
-    const double2 x = ld2(a, i, cplx), y = ld2(b_, i, cplx);
-    const double dx = x.x - y.x, dy = x.y - y.y;
-    const double diff = cplx ? hypot(dx, dy) : fabs(dx);
-    const double mag = cplx ? hypot(y.x, y.y) : fabs(y.x);
-    if (!(diff <= fma_(rtol, mag, atol))) acc.x += 1.0;
+    if (!close_(ld2(a, i, cplx), ld2(b_, i, cplx), cplx, rtol, atol)) acc.x += 1.0;
   }
   return acc;
 }
@@ -228,6 +262,8 @@ __global__ void vec_group_partial(const __grid_constant__ VecGroup g, double2* p
     acc = dot_body(it.n, cplx, it.x, it.y, 0, b, nb);
   else if (g.op == RENO_VOP_ORTH)
     acc = orth_body(it.n, cplx, it.out, it.x, it.y, it.scalars, it.j, b, nb);
+  else if (g.op == RENO_VOP_CHECK)
+    acc = check_body(it.n, it.j, cplx, it.x, it.ldv, it.s, it.out, g.rtol, g.atol, b, nb);
   else
     acc = allclose_body(it.n, cplx, it.x, it.y, g.rtol, g.atol, b, nb);
   const double2 r = block_sum(acc);
@@ -259,6 +295,116 @@ __global__ void vec_group_elementwise(const __grid_constant__ VecGroup g) {
     scale_inv_body(it.n, cplx, it.x, it.s, it.out, b, nb);
   else
     lincomb_body(it.n, it.j, cplx, it.x, it.ldv, it.s, it.out, b, nb);
+}
+
+// ---------------------------------------------------------------- whole Lanczos step
+// alpha_j = Re vdot(w, v); w -= alpha_j v + beta_{j-1} vprev; beta_j = ||w||;
+// V[j+1] = w / beta_j for vectors that fit one cluster's shared memory, in one
+// launch instead of five.  What bounds a small step is launches and the two
+// dependent reductions, not the megabyte it moves: the cluster keeps w in
+// shared memory between the passes, and each CTA pushes its partial sum to
+// all eight, so a reduction is one cluster barrier.  Each item's partition
+// depends on its own length only, so a batch rounds like a single call.
+// Kernel time against that of the five launches (which have four more gaps):
+// 4.1 / 13.8 us at 1000 complex elements, 5.6 / 12.2 at 10240, 10.4 / 12.3 at
+// 65536; at 102400 eight SMs are the slower side, 15.4 / 12.4, so the line is
+// drawn at 65536 (128 KB of w per CTA).
+constexpr int SCL = 8, ST = 512;
+constexpr int64_t STEP_BYTES = 128 * 1024;
+
+static bool step_fits(const reno_vec_item& it) {
+  return ceil_div(it.n, SCL) * (it.dtype == RENO_C128 ? 16 : 8) <= STEP_BYTES;
+}
+
+__device__ __forceinline__ double cluster_total(double v, double* red, double (*part)[SCL], int par,
+                                                cooperative_groups::cluster_group& cluster) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  if (threadIdx.x < SCL) {
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < ST / 32; ++w) t += red[w];
+    cluster.map_shared_rank(&part[par][0], threadIdx.x)[cluster.block_rank()] = t;
+  }
+  cluster.sync();
+  double s = 0.0;
+#pragma unroll
+  for (int q = 0; q < SCL; ++q) s += part[par][q];
+  return s;
+}
+
+template <bool C>
+__device__ __forceinline__ void step_item(const reno_vec_item& it, cooperative_groups::cluster_group& cluster,
+                                          double* red, double (*part)[SCL], unsigned char* smem) {
+  using T = typename std::conditional<C, double2, double>::type;
+  T* ws = reinterpret_cast<T*>(smem);
+  const int64_t chunk = ceil_div(it.n, SCL), i0 = (int64_t)cluster.block_rank() * chunk;
+  const int m = (int)max((int64_t)0, min(chunk, it.n - i0));
+  const T* w = reinterpret_cast<const T*>(it.out) + i0;
+  const T* v = reinterpret_cast<const T*>(it.x) + i0;
+  const T* vp = reinterpret_cast<const T*>(it.y) + i0;
+  T* vn = const_cast<T*>(reinterpret_cast<const T*>(it.x)) + it.ldv + i0;
+  const int j = it.j;
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < m; i += ST) {
+    const T a = w[i], b = v[i];
+    ws[i] = a;
+    if constexpr (C) acc = fma(a.x, b.x, fma(a.y, b.y, acc));
+    else acc = fma(a, b, acc);
+  }
+  const double alpha = cluster_total(acc, red, part, 0, cluster);
+  const double bprev = j > 0 ? it.scalars[2 * j - 1] : 0.0;
+  acc = 0.0;
+  for (int i = threadIdx.x; i < m; i += ST) {
+    T a = ws[i];
+    const T b = v[i];
+    if constexpr (C) {
+      double2 t = make_double2(alpha * b.x, alpha * b.y);
+      if (j > 0) {
+        const T p = vp[i];
+        t.x = fma(bprev, p.x, t.x);
+        t.y = fma(bprev, p.y, t.y);
+      }
+      a.x -= t.x;
+      a.y -= t.y;
+      acc = fma(a.x, a.x, fma(a.y, a.y, acc));
+    } else {
+      double t = alpha * b;
+      if (j > 0) t = fma(bprev, vp[i], t);
+      a -= t;
+      acc = fma(a, a, acc);
+    }
+    ws[i] = a;
+  }
+  const double beta = sqrt(cluster_total(acc, red, part, 1, cluster));
+  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+    it.scalars[2 * j] = alpha;
+    it.scalars[2 * j + 1] = beta;
+  }
+  for (int i = threadIdx.x; i < m; i += ST) {
+    T a = ws[i];
+    if constexpr (C) {
+      a.x /= beta;
+      a.y /= beta;
+    } else {
+      a /= beta;
+    }
+    vn[i] = a;
+  }
+}
+
+__global__ void __cluster_dims__(SCL, 1, 1) __launch_bounds__(ST, 1)
+    krylov_step_kernel(const __grid_constant__ VecGroup g) {
+  extern __shared__ __align__(16) unsigned char step_smem[];
+  __shared__ double red[ST / 32];
+  __shared__ double part[2][SCL];
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.sync();  // no CTA pushes into another before that one runs
+  const reno_vec_item& it = g.it[blockIdx.y];
+  if (it.dtype == RENO_C128) step_item<true>(it, cluster, red, part, step_smem);
+  else step_item<false>(it, cluster, red, part, step_smem);
 }
 
 __global__ void axpy_kernel(int64_t n, bool cplx, void* y, const void* x, const double* c, double sgn) {
@@ -397,13 +543,62 @@ extern "C" int reno_vec_grouped_workspace_bytes(int32_t count, size_t* bytes) {
   return RENO_OK;
 }
 
+// RENO_VOP_STEP: the items that fit a cluster in one launch, the others as the
+// three operations it stands for
+static int krylov_steps(reno_ctx* ctx, int32_t count, const reno_vec_item* items, void* ws, size_t ws_bytes) {
+  VecGroup g;
+  g.count = 0;
+  g.op = RENO_VOP_STEP;
+  g.rtol = g.atol = 0.0;
+  std::vector<reno_vec_item> big, scale;
+  int64_t bytes = 0;
+  for (int p = 0; p < count; ++p) {
+    const reno_vec_item& it = items[p];
+    if (!dt_ok(it.dtype) || it.n < 1 || !it.out || !it.x || !it.scalars || it.j < 0 || (it.j > 0 && !it.y) ||
+        it.ldv < it.n)
+      return set_error(ctx, RENO_ERR_INVALID, "reno_vec_grouped: bad item " + std::to_string(p));
+    if (step_fits(it)) {
+      g.it[g.count++] = it;
+      bytes = std::max(bytes, ceil_div(it.n, SCL) * (it.dtype == RENO_C128 ? 16 : 8));
+    } else {
+      big.push_back(it);
+      scale.push_back(it);
+      reno_vec_item& q = scale.back();
+      q.x = it.out;
+      q.out = const_cast<char*>(static_cast<const char*>(it.x)) + it.ldv * (it.dtype == RENO_C128 ? 16 : 8);
+      q.s = it.scalars + 2 * it.j + 1;
+    }
+  }
+  if (g.count) {
+    static std::atomic<unsigned long long> set{0};
+    int rc = check_cuda(ctx, smem_optin_once(krylov_step_kernel, (int)STEP_BYTES, set), "reno_vec_grouped: step");
+    if (rc != RENO_OK) return rc;
+    count_launch();
+    krylov_step_kernel<<<dim3(SCL, g.count), ST, (size_t)bytes, ctx->stream>>>(g);
+    rc = check_cuda(ctx, cudaGetLastError(), "reno_vec_grouped: step");
+    if (rc != RENO_OK) return rc;
+  }
+  if (big.empty()) return RENO_OK;
+  const int m = (int)big.size();
+  std::vector<reno_vec_item> dot = big;
+  for (reno_vec_item& q : dot) {
+    q.y = q.x;
+    q.x = q.out;
+  }
+  int rc = reno_vec_grouped(ctx, RENO_VOP_ALPHA, m, dot.data(), 0.0, 0.0, ws, ws_bytes);
+  if (rc == RENO_OK) rc = reno_vec_grouped(ctx, RENO_VOP_ORTH, m, big.data(), 0.0, 0.0, ws, ws_bytes);
+  if (rc == RENO_OK) rc = reno_vec_grouped(ctx, RENO_VOP_SCALE_INV, m, scale.data(), 0.0, 0.0, ws, ws_bytes);
+  return rc;
+}
+
 extern "C" int reno_vec_grouped(reno_ctx* ctx, int32_t op, int32_t count, const reno_vec_item* items, double rtol,
                                 double atol, void* ws, size_t ws_bytes) {
   if (!ctx) return RENO_ERR_INVALID;
-  if (op < RENO_VOP_NORM || op > RENO_VOP_ALLCLOSE || count < 0 || count > RENO_VEC_GROUP_MAX ||
+  if (op < RENO_VOP_NORM || op > RENO_VOP_CHECK || count < 0 || count > RENO_VEC_GROUP_MAX ||
       (count > 0 && !items))
     return set_error(ctx, RENO_ERR_INVALID, "reno_vec_grouped: bad op or count");
   if (count == 0) return RENO_OK;
+  if (op == RENO_VOP_STEP) return krylov_steps(ctx, count, items, ws, ws_bytes);
   const bool reduces = op != RENO_VOP_SCALE_INV && op != RENO_VOP_LINCOMB;
   if (reduces && (!ws || ws_bytes < (size_t)count * VMAX_BLOCKS * sizeof(double2)))
     return set_error(ctx, RENO_ERR_WORKSPACE, "reno_vec_grouped: workspace too small");
@@ -422,6 +617,9 @@ extern "C" int reno_vec_grouped(reno_ctx* ctx, int32_t op, int32_t count, const 
       case RENO_VOP_ORTH: ok = ok && it.out && it.x && it.scalars && it.j >= 0 && (it.j == 0 || it.y); break;
       case RENO_VOP_SCALE_INV: ok = ok && it.x && it.s && it.out; break;
       case RENO_VOP_LINCOMB: ok = ok && it.x && it.s && it.out && it.j >= 0 && it.ldv >= it.n; break;
+      case RENO_VOP_CHECK:
+        ok = ok && it.x && it.s && it.out && it.scalars && it.j >= 2 && it.ldv >= it.n;
+        break;
       default: ok = ok && it.x && it.y && it.scalars; break;
     }
     if (!ok) return set_error(ctx, RENO_ERR_INVALID, "reno_vec_grouped: bad item " + std::to_string(p));

@@ -21,7 +21,7 @@ import numpy as np
 import torch
 from scipy.linalg import eigh_tridiagonal
 
-from ._native import Engine, h2d
+from ._native import Engine, VOP_STEP, dtype_code, h2d
 from .hop_expr import as_device
 
 EPS = np.finfo(float).eps
@@ -139,7 +139,8 @@ def _expm_krylov_steps(dt, vstart, block_size=50):
             w = w.to(work_dtype)
         if not w.is_contiguous():
             w = w.contiguous()
-        eng.krylov_alpha(w, K.V[j], K.ab, j)
+        if j == n - 1 or not v.is_cuda:
+            eng.krylov_alpha(w, K.V[j], K.ab, j)
         if j == n - 1:
             alpha, beta = host_scalars(j)
             i = breakdown_before(j, beta)
@@ -148,8 +149,11 @@ def _expm_krylov_steps(dt, vstart, block_size=50):
         if K.V.shape[0] == j + 1:
             K.grow(block_size)
         vprev = K.V[j - 1] if j > 0 else None
-        eng.krylov_orth(w, K.V[j], vprev, K.ab, j)       # w -= ...; beta_j = ||w||
-        eng.scale_inv(w, K.ab[2 * j + 1:], K.V[j + 1])   # V[j+1] = w / beta_j
+        if v.is_cuda:  # alpha_j, w -= ..., beta_j = ||w|| and V[j+1] = w / beta_j in one operation
+            eng.vec_grouped(VOP_STEP, [(n, dtype_code(v), j, K.V[j], vprev, w, K.ab, None, n)])
+        else:
+            eng.krylov_orth(w, K.V[j], vprev, K.ab, j)
+            eng.scale_inv(w, K.ab[2 * j + 1:], K.V[j + 1])
         if 3 < j and j % 2 == 0:
             alpha, beta = host_scalars(j)
             i = breakdown_before(j + 1, beta)
@@ -307,16 +311,19 @@ class _LockstepKrylov:
                 if not w.is_contiguous():
                     w = w.contiguous()
                 W[p] = w
-            self._op(VOP_ALPHA, [(p, j, W[p], self.V[p][j], None, self.AB[p], None) for p in active])
             term = [p for p in active if j == self.n[p] - 1]
             cont = [p for p in active if j < self.n[p] - 1]
+            cuda = self.device.type == "cuda"
+            self._op(VOP_ALPHA, [(p, j, W[p], self.V[p][j], None, self.AB[p], None)
+                                 for p in (term if cuda else active)])
             for p in cont:
                 if self.V[p].shape[0] == j + 1:
                     self._grow(p)
-            self._op(VOP_ORTH, [(p, j, self.V[p][j], self.V[p][j - 1] if j > 0 else None, W[p], self.AB[p], None)
-                                for p in cont])
-            self._op(VOP_SCALE_INV, [(p, 0, W[p], None, self.V[p][j + 1], None, self.AB[p][2 * j + 1:])
-                                     for p in cont])
+            self._op(VOP_STEP if cuda else VOP_ORTH,
+                     [(p, j, self.V[p][j], self.V[p][j - 1] if j > 0 else None, W[p], self.AB[p], None) for p in cont])
+            if not cuda:
+                self._op(VOP_SCALE_INV, [(p, 0, W[p], None, self.V[p][j + 1], None, self.AB[p][2 * j + 1:])
+                                         for p in cont])
             check = cont if (3 < j and j % 2 == 0) else []
             finished = set()
             if term or check:
