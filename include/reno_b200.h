@@ -257,13 +257,29 @@ int reno_qr_blocks(reno_ctx* ctx, int32_t count, const reno_qr_block* blocks,
  * breakdown beta_j < 100 n eps) and count, returned in out_k.  The host
  * synchronises at those checks only.  Fails with RENO_ERR_WORKSPACE when more
  * than kmax Krylov vectors would be needed.  Workspace from
- * reno_lanczos_workspace_bytes(desc, kmax). */
+ * reno_lanczos_workspace_bytes(desc, kmax).
+ * reno_lanczos_expm_to leaves psi as it is and writes to `out` (which may be
+ * psi).
+ * reno_lanczos_coefficients is the exponential's small host problem
+ * (krylov.py:15-24), for count of them: row i of scal (ld doubles) holds the
+ * start norm and the tridiagonal matrix of order k[i] as alpha_0, beta_0,
+ * alpha_1, ..., dt its step (re, im); coef receives, one problem after the
+ * other, k[i] (re, im) pairs u (norm exp(dt w) u[0]).  RENO_ERR_NONFINITE
+ * when one is not finite.  Needs no GPU. */
+int reno_lanczos_coefficients(int32_t count, const int32_t* k,
+                              const double* scal, int64_t ld, const double* dt,
+                              double* coef);
 int reno_lanczos_workspace_bytes(const reno_heff_desc* desc, int32_t kmax,
                                  size_t* bytes);
 int reno_lanczos_expm(reno_ctx* ctx, const reno_heff_desc* desc, const void* L,
                       const void* W1, const void* W2, const void* R,
                       double dt_re, double dt_im, void* psi, int32_t kmax,
                       int32_t* out_k, void* ws, size_t ws_bytes);
+int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc,
+                         const void* L, const void* W1, const void* W2,
+                         const void* R, double dt_re, double dt_im,
+                         const void* psi, void* out, int32_t kmax,
+                         int32_t* out_k, void* ws, size_t ws_bytes);
 
 /* QN-blocked truncation of one coefficient matrix (rows x cols, row-major):
  * svd_qn.py:99-240 with select_basis lib.py:253-322 (percent 0) and

@@ -10,6 +10,7 @@ import threading
 from pathlib import Path
 from typing import Optional
 
+import numpy as np
 import torch
 
 PKG_DIR = Path(__file__).resolve().parent
@@ -61,6 +62,12 @@ VEC_GROUP_MAX = 128
 VOP_NORM, VOP_ALPHA, VOP_ORTH, VOP_SCALE_INV, VOP_LINCOMB, VOP_ALLCLOSE, VOP_STEP, VOP_CHECK = range(8)
 
 
+# VecItem as a numpy record, for tables filled by whole columns
+VEC_ITEM = np.dtype([("n", "<i8"), ("dtype", "<i4"), ("j", "<i4"), ("x", "<u8"), ("y", "<u8"), ("out", "<u8"),
+                     ("scalars", "<u8"), ("s", "<u8"), ("ldv", "<i8")])
+assert VEC_ITEM.itemsize == ctypes.sizeof(VecItem)
+
+
 class EnvDesc(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int32) for n in
                 ("side", "d", "w_in", "w_out", "mk_in", "mk_out", "mb_in", "mb_out", "env_dtype", "ket_dtype",
@@ -85,6 +92,9 @@ _SIGS = {
     "reno_lanczos_workspace_bytes": (_c_int, [ctypes.POINTER(HeffDesc), _c_int, ctypes.POINTER(_c_sz)]),
     "reno_lanczos_expm": (_c_int, [_vp, ctypes.POINTER(HeffDesc), _vp, _vp, _vp, _vp, ctypes.c_double, ctypes.c_double,
                                    _vp, _c_int, ctypes.POINTER(ctypes.c_int32), _vp, _c_sz]),
+    "reno_lanczos_expm_to": (_c_int, [_vp, ctypes.POINTER(HeffDesc), _vp, _vp, _vp, _vp, ctypes.c_double,
+                                      ctypes.c_double, _vp, _vp, _c_int, ctypes.POINTER(ctypes.c_int32), _vp, _c_sz]),
+    "reno_lanczos_coefficients": (_c_int, [_c_int, _vp, _vp, _c_i64, _vp, _vp]),
     "reno_qn_svd_truncate_workspace_bytes": (_c_int, [ctypes.POINTER(TruncDesc), ctypes.POINTER(_c_sz)]),
     "reno_qn_svd_truncate": (_c_int, [_vp, ctypes.POINTER(TruncDesc), _vp, _vp, _vp, _c_int, _vp, _vp,
                                       ctypes.POINTER(ctypes.c_int32), _vp, _c_sz]),
@@ -191,6 +201,13 @@ def ptr(t: Optional[torch.Tensor]):
     # torch's lazy conjugate / negative views keep unconjugated memory behind a flag
     assert not (t.is_conj() or t.is_neg()), "resolve_conj()/resolve_neg() before passing a view to the engine"
     return ctypes.c_void_p(t.data_ptr())
+
+
+def addresses(ts) -> np.ndarray:
+    """the device addresses of tensors, with ptr's checks"""
+    assert all([t.is_cuda and t.is_contiguous() and not (t.is_conj() or t.is_neg()) for t in ts]), \
+        "sweep-engine tensors are C-contiguous, on the GPU and without lazy conj / neg bits"
+    return np.array([t.data_ptr() for t in ts], dtype=np.uint64)
 
 
 def h2d(arr, device, dtype=None) -> torch.Tensor:
@@ -350,16 +367,24 @@ class Engine:
 
     def heff_apply_grouped(self, descs, Ls, W1s, W2s, Rs, psis, ys):
         """reno_heff_apply_grouped (FP64): lists of equal length; W1s / W2s
-        entries None below one / two active sites"""
+        entries None below one / two active sites.  An operand's list may be an
+        array of addresses (``addresses``) instead of tensors."""
         m = len(descs)
         arr = (HeffDesc * m)(*descs)
         n = _c_sz()
         self.check(self.lib.reno_heff_grouped_workspace_bytes(m, arr, ctypes.byref(n)),
                    "reno_heff_grouped_workspace_bytes")
         ws = self.workspace(int(n.value))
-        pa = lambda ts: (_vp * m)(*[_vp(t.data_ptr()) if t is not None else None for t in ts])
-        for t in list(Ls) + list(Rs) + list(psis) + list(ys) + [w for w in list(W1s) + list(W2s) if w is not None]:
-            ptr(t)  # contiguity / lazy-view checks
+
+        def pa(ts):
+            if isinstance(ts, np.ndarray):
+                assert ts.dtype == np.uint64 and ts.flags.c_contiguous and len(ts) == m
+                return ctypes.cast(ts.ctypes.data, ctypes.POINTER(_vp))
+            for t in ts:
+                if t is not None:
+                    ptr(t)  # contiguity / lazy-view checks
+            return (_vp * m)(*[t.data_ptr() if t is not None else None for t in ts])
+
         self.check(self.lib.reno_heff_apply_grouped(self.ctx, m, arr, pa(Ls), pa(W1s), pa(W2s), pa(Rs), pa(psis),
                                                     pa(ys), ptr(ws), ws.numel()), "reno_heff_apply_grouped")
         self.launches += 1
@@ -488,6 +513,38 @@ class Engine:
                 self._vec_gws = torch.empty(int(nbytes.value), dtype=torch.uint8, device=f"cuda:{self.device}")
             self.check(self.lib.reno_vec_grouped(self.ctx, op, len(chunk), arr, rtol, atol, ptr(self._vec_gws),
                                                  self._vec_gws.numel()), "reno_vec_grouped")
+
+    def vec_grouped_table(self, op, table, rtol=0.0, atol=0.0):
+        """vec_grouped on a contiguous VEC_ITEM array of device addresses that
+        the caller has checked and keeps alive until the work has run"""
+        for c0 in range(0, len(table), VEC_GROUP_MAX):
+            m = min(VEC_GROUP_MAX, len(table) - c0)
+            nbytes = _c_sz()
+            self.check(self.lib.reno_vec_grouped_workspace_bytes(m, ctypes.byref(nbytes)),
+                       "reno_vec_grouped_workspace_bytes")
+            if self._vec_gws is None or self._vec_gws.numel() < nbytes.value:
+                self._vec_gws = torch.empty(int(nbytes.value), dtype=torch.uint8, device=f"cuda:{self.device}")
+            arr = ctypes.cast(table[c0:].ctypes.data, ctypes.POINTER(VecItem))
+            self.check(self.lib.reno_vec_grouped(self.ctx, op, m, arr, rtol, atol, ptr(self._vec_gws),
+                                                 self._vec_gws.numel()), "reno_vec_grouped")
+
+    def lanczos_expm(self, desc: HeffDesc, L, W1, W2, R, dt, psi, kmax):
+        """reno_lanczos_expm_to: (exp(dt H_eff) psi, number of matvecs), or None
+        where its kmax vectors do not suffice or its scalars are not finite"""
+        n = _c_sz()
+        self.check(self.lib.reno_lanczos_workspace_bytes(ctypes.byref(desc), kmax, ctypes.byref(n)),
+                   "reno_lanczos_workspace_bytes")
+        ws = torch.empty(int(n.value), dtype=torch.uint8, device=psi.device)
+        out = torch.empty_like(psi)
+        k = ctypes.c_int32(0)
+        st = self.lib.reno_lanczos_expm_to(self.ctx, ctypes.byref(desc), ptr(L), ptr(W1), ptr(W2), ptr(R),
+                                           float(dt.real), float(dt.imag), ptr(psi), ptr(out), kmax, ctypes.byref(k),
+                                           ptr(ws), ws.numel())
+        if st in (RENO_ERR_WORKSPACE, RENO_ERR_NONFINITE):
+            return None
+        self.check(st, "reno_lanczos_expm")
+        self.launches += int(k.value)
+        return out, int(k.value)
 
     # quantum-number block movers
     def qn_gather(self, mat, rows, cols, out):

@@ -35,7 +35,8 @@ class Backend:
 
     @property
     def device(self) -> torch.device:
-        if not torch.cuda.is_available():
+        # is_available() asks the driver; once it has said yes a context exists
+        if not torch.cuda.is_initialized() and not torch.cuda.is_available():
             raise RuntimeError("renormalizer_b200 needs a CUDA device (B200, sm_100a); none is visible")
         idx = self._device_index if self._device_index is not None else torch.cuda.current_device()
         return torch.device("cuda", idx)

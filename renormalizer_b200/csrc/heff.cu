@@ -301,12 +301,22 @@ static Fused2 fused2_layout(const reno_heff_desc* d, char* base) {
 }
 
 static cudaError_t fused2_run(const reno_heff_desc* d, const Fused2& f, const void* L, const void* Wt1,
-                              const void* Wt2, const void* R, const void* psi, void* y, cudaStream_t st) {
+                              const void* Wt2, const void* R, const void* psi, void* y, bool packed,
+                              cudaStream_t st) {
   const int64_t ml = d->ml, mr = d->mr, wl = d->wl, wm = d->wm, wr = d->wr, d1 = d->d1, d2 = d->d2;
   const int ev = d->env_dtype, pv = d->psi_dtype, pr = d->prec;
   const bool c = ev == RENO_C128;
   const int64_t x2 = c ? 2 : 1;
-  cudaError_t e = split_pack(opnd(L, ev, ml, 1), (int)(ml * wl), (int)ml, 1, SplitRows{}, f.s1a, pr, st);
+  cudaError_t e = cudaSuccess;
+  if (!packed) {
+    e = split_pack(opnd(L, ev, ml, 1), (int)(ml * wl), (int)ml, 1, SplitRows{}, f.s1a, pr, st);
+    if (e == cudaSuccess)
+      e = split_pack(opnd(Wt1, RENO_F64, wl * d1, 1), (int)(d1 * wm), (int)(wl * d1), 1, SplitRows{}, f.s2a, pr, st);
+    if (e == cudaSuccess)
+      e = split_pack(opnd(Wt2, RENO_F64, wm * d2, 1), (int)(d2 * wr), (int)(wm * d2), 1, SplitRows{}, f.s3a, pr, st);
+    if (e == cudaSuccess)
+      e = split_pack(opnd(R, ev, wr * mr, 1), (int)mr, (int)(wr * mr), 1, SplitRows{}, f.s4b, pr, st);
+  }
   // psi rows in (k, h, e) order: e at stride d2*mr, h at mr, k at 1; K = c at d1*d2*mr
   SplitRows khe;
   khe.D0 = (int)d1;
@@ -315,12 +325,6 @@ static cudaError_t fused2_run(const reno_heff_desc* d, const Fused2& f, const vo
   khe.s_r2 = 1;
   if (e == cudaSuccess)
     e = split_pack(opnd(psi, pv, d2 * mr, d1 * d2 * mr), (int)(d1 * d2 * mr), (int)ml, 1, khe, f.s1b, pr, st);
-  if (e == cudaSuccess)
-    e = split_pack(opnd(Wt1, RENO_F64, wl * d1, 1), (int)(d1 * wm), (int)(wl * d1), 1, SplitRows{}, f.s2a, pr, st);
-  if (e == cudaSuccess)
-    e = split_pack(opnd(Wt2, RENO_F64, wm * d2, 1), (int)(d2 * wr), (int)(wm * d2), 1, SplitRows{}, f.s3a, pr, st);
-  if (e == cudaSuccess)
-    e = split_pack(opnd(R, ev, wr * mr, 1), (int)mr, (int)(wr * mr), 1, SplitRows{}, f.s4b, pr, st);
   if (e != cudaSuccess) return e;
   // S1: rows (a, b) of L, columns (k, h, e) -> S2's B[a][(k, h) re/im][(b, e)]
   SplitPackOut o1{f.s2b.hi, f.s2b.lo, 0, f.s2b.rows * f.s2b.pitch, d1, x2 * f.s2b.pitch, 1, f.s2b.pitch,
@@ -397,11 +401,18 @@ static Fused1 fused1_layout(const reno_heff_desc* d, char* base) {
 }
 
 static cudaError_t fused1_run(const reno_heff_desc* d, const Fused1& f, const void* L, const void* Wt,
-                              const void* R, const void* psi, void* y, cudaStream_t st) {
+                              const void* R, const void* psi, void* y, bool packed, cudaStream_t st) {
   const int64_t ml = d->ml, mr = d->mr, wl = d->wl, wr = d->wr, dd = d->d1;
   const int ev = d->env_dtype, pv = d->psi_dtype, pr = d->prec;
   const int64_t x2 = ev == RENO_C128 ? 2 : 1;
-  cudaError_t e = split_pack(opnd(L, ev, ml, 1), (int)(ml * wl), (int)ml, 1, SplitRows{}, f.s1a, pr, st);
+  cudaError_t e = cudaSuccess;
+  if (!packed) {
+    e = split_pack(opnd(L, ev, ml, 1), (int)(ml * wl), (int)ml, 1, SplitRows{}, f.s1a, pr, st);
+    if (e == cudaSuccess)
+      e = split_pack(opnd(Wt, RENO_F64, wl * dd, 1), (int)(dd * wr), (int)(wl * dd), 1, SplitRows{}, f.s2a, pr, st);
+    if (e == cudaSuccess)
+      e = split_pack(opnd(R, ev, wr * mr, 1), (int)mr, (int)(wr * mr), 1, SplitRows{}, f.s3b, pr, st);
+  }
   // psi rows in (k, e) order: e at stride mr, k at 1; K = c at dd*mr
   SplitRows ke;
   ke.D0 = (int)dd;
@@ -409,10 +420,6 @@ static cudaError_t fused1_run(const reno_heff_desc* d, const Fused1& f, const vo
   ke.s_r1 = 1;
   ke.s_r2 = 0;
   if (e == cudaSuccess) e = split_pack(opnd(psi, pv, mr, dd * mr), (int)(dd * mr), (int)ml, 1, ke, f.s1b, pr, st);
-  if (e == cudaSuccess)
-    e = split_pack(opnd(Wt, RENO_F64, wl * dd, 1), (int)(dd * wr), (int)(wl * dd), 1, SplitRows{}, f.s2a, pr, st);
-  if (e == cudaSuccess)
-    e = split_pack(opnd(R, ev, wr * mr, 1), (int)mr, (int)(wr * mr), 1, SplitRows{}, f.s3b, pr, st);
   if (e != cudaSuccess) return e;
   // S1: rows (a, b) of L, columns (k, e) -> S2's B[a][k re/im][(b, e)]
   SplitPackOut o1{f.s2b.hi, f.s2b.lo, 0, f.s2b.rows * f.s2b.pitch, dd, x2 * f.s2b.pitch, 1, f.s2b.pitch,
@@ -430,13 +437,15 @@ static cudaError_t fused1_run(const reno_heff_desc* d, const Fused1& f, const vo
   return e;
 }
 
-static size_t heff_total(const reno_heff_desc* d) {
+static size_t heff_needed(const reno_heff_desc* d) {
   const HeffLayout lay = heff_layout(d);
   if (fused2_eligible(d)) return lay.off_t1 + fused2_layout(d, nullptr).bytes;
   if (fused1_eligible(d)) return lay.off_t1 + fused1_layout(d, nullptr).bytes;
   char* nul = nullptr;
-  return lay.off_split + align256(split_need(heff_stages(d, lay, nul, nullptr, nullptr, nullptr, nullptr)));
+  return lay.off_split + split_need(heff_stages(d, lay, nul, nullptr, nullptr, nullptr, nullptr));
 }
+
+static size_t heff_total(const reno_heff_desc* d) { return align256(heff_needed(d)); }
 
 }  // namespace reno
 
@@ -448,50 +457,51 @@ extern "C" int reno_heff_workspace_bytes(const reno_heff_desc* d, size_t* bytes)
   return RENO_OK;
 }
 
-extern "C" int reno_heff_apply(reno_ctx* ctx, const reno_heff_desc* d, const void* L, const void* W1,
-                               const void* W2, const void* R, const void* psi, void* y, void* ws,
-                               size_t ws_bytes) {
+// reno_heff_apply; with `prepared` the workspace still holds what an earlier
+// call of the same operator put there (the transposed MPO tensors and, on the
+// fused split chains, the packed L, W and R), and only psi is new: the
+// matvecs of one Lanczos exponential.
+int reno::heff_apply_prepared(reno_ctx* ctx, const reno_heff_desc* d, const void* L, const void* W1, const void* W2,
+                              const void* R, const void* psi, void* y, void* ws, size_t ws_bytes, bool prepared) {
   if (!ctx) return RENO_ERR_INVALID;
   if (validate_heff(d) != RENO_OK) return set_error(ctx, RENO_ERR_INVALID, "reno_heff_apply: invalid descriptor");
   if (!L || !R || !psi || !y || (d->nsite >= 1 && !W1) || (d->nsite == 2 && !W2))
     return set_error(ctx, RENO_ERR_INVALID, "reno_heff_apply: null tensor pointer");
   const HeffLayout lay = heff_layout(d);
   char* w = static_cast<char*>(ws);
+  if (!ws || ws_bytes < heff_needed(d))
+    return set_error(ctx, RENO_ERR_WORKSPACE, "reno_heff_apply: workspace too small");
+  cudaStream_t st = ctx->stream;
+  cudaError_t e = cudaSuccess;
+  if (!prepared) {
+    if (d->nsite == 1) e = launch_wt(W1, w + lay.off_wt1, d->mpo_dtype, d->wl, d->d1, d->wr, 0, st);
+    if (d->nsite == 2) {
+      e = launch_wt(W1, w + lay.off_wt1, d->mpo_dtype, d->wl, d->d1, d->wm, 0, st);
+      if (e == cudaSuccess) e = launch_wt(W2, w + lay.off_wt2, d->mpo_dtype, d->wm, d->d2, d->wr, 0, st);
+    }
+    if (e != cudaSuccess) return check_cuda(ctx, e, "reno_heff_apply");
+  }
   if (fused1_eligible(d)) {
-    const Fused1 f = fused1_layout(d, w ? w + lay.off_t1 : nullptr);
-    if (ws_bytes < lay.off_t1 + f.bytes || !ws)
-      return set_error(ctx, RENO_ERR_WORKSPACE, "reno_heff_apply: workspace too small");
-    cudaStream_t st = ctx->stream;
-    cudaError_t e = launch_wt(W1, w + lay.off_wt1, d->mpo_dtype, d->wl, d->d1, d->wr, 0, st);
-    if (e == cudaSuccess) e = fused1_run(d, f, L, w + lay.off_wt1, R, psi, y, st);
+    e = fused1_run(d, fused1_layout(d, w + lay.off_t1), L, w + lay.off_wt1, R, psi, y, prepared, st);
     return check_cuda(ctx, e, "reno_heff_apply");
   }
   if (fused2_eligible(d)) {
-    const Fused2 f = fused2_layout(d, w ? w + lay.off_t1 : nullptr);
-    if (ws_bytes < lay.off_t1 + f.bytes || !ws)
-      return set_error(ctx, RENO_ERR_WORKSPACE, "reno_heff_apply: workspace too small");
-    cudaStream_t st = ctx->stream;
-    cudaError_t e = launch_wt(W1, w + lay.off_wt1, d->mpo_dtype, d->wl, d->d1, d->wm, 0, st);
-    if (e == cudaSuccess) e = launch_wt(W2, w + lay.off_wt2, d->mpo_dtype, d->wm, d->d2, d->wr, 0, st);
-    if (e == cudaSuccess) e = fused2_run(d, f, L, w + lay.off_wt1, w + lay.off_wt2, R, psi, y, st);
+    e = fused2_run(d, fused2_layout(d, w + lay.off_t1), L, w + lay.off_wt1, w + lay.off_wt2, R, psi, y, prepared, st);
     return check_cuda(ctx, e, "reno_heff_apply");
   }
   const std::vector<Stage> stages = heff_stages(d, lay, w, L, R, psi, y);
   const size_t need_split = split_need(stages);
-  if (ws_bytes < lay.off_split + need_split || !ws)
-    return set_error(ctx, RENO_ERR_WORKSPACE, "reno_heff_apply: workspace too small");
-  cudaStream_t st = ctx->stream;
-  cudaError_t e = cudaSuccess;
-  if (d->nsite == 1) e = launch_wt(W1, w + lay.off_wt1, d->mpo_dtype, d->wl, d->d1, d->wr, 0, st);
-  if (d->nsite == 2) {
-    e = launch_wt(W1, w + lay.off_wt1, d->mpo_dtype, d->wl, d->d1, d->wm, 0, st);
-    if (e == cudaSuccess) e = launch_wt(W2, w + lay.off_wt2, d->mpo_dtype, d->wm, d->d2, d->wr, 0, st);
-  }
   for (const Stage& s : stages) {
     if (e != cudaSuccess) break;
     e = run_stage(s, w + lay.off_split, need_split, st);
   }
   return check_cuda(ctx, e, "reno_heff_apply");
+}
+
+extern "C" int reno_heff_apply(reno_ctx* ctx, const reno_heff_desc* d, const void* L, const void* W1,
+                               const void* W2, const void* R, const void* psi, void* y, void* ws,
+                               size_t ws_bytes) {
+  return heff_apply_prepared(ctx, d, L, W1, W2, R, psi, y, ws, ws_bytes, false);
 }
 
 // ---------------------------------------------------------------- grouped FP64 matvec

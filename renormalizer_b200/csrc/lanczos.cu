@@ -3,16 +3,18 @@
 // operator) behind one C call, so that a host without Python can drive the
 // local updates of a sweep.
 //
-// Every matvec (reno_heff_apply) and vector operation (norm, alpha, the
-// three-term recurrence, the combination V c, allclose) runs on the device in
-// FP64.  The host reads the Lanczos scalars only where the reference makes a
-// decision with them: at its convergence checks (every even j > 3), where the
-// breakdown test beta_i < 100 n eps is also applied to every beta since the
-// previous check -- the Krylov vectors up to a breakdown do not depend on
-// what came after it, so the result and the count are the reference's.  The
+// Every matvec (reno_heff_apply) and vector operation (norm, the Lanczos
+// step, the combination V c, allclose) runs on the device in FP64.  The host
+// reads the Lanczos scalars only where the reference makes a decision with
+// them: at its convergence tests (every even j > 5; its first approximation,
+// at j = 4, has none to be compared with), where the breakdown test
+// beta_i < 100 n eps is also applied to every beta since the previous one --
+// the Krylov vectors up to a breakdown do not depend on what came after it,
+// so the result and the count are the reference's.  The
 // small tridiagonal eigenproblem of krylov.py:15-24 is solved on the host by
 // implicit QL iterations with shifts (the EISPACK tql2 method of Bowdler,
 // Martin, Reinsch and Wilkinson, Numer. Math. 11, 1968).
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <vector>
@@ -30,29 +32,26 @@ int64_t psi_elems(const reno_heff_desc* d) {
   return (int64_t)d->ml * d->d1 * d->d2 * d->mr;
 }
 
+// scal: the start norm, the allclose flag, then (alpha_0, beta_0, alpha_1, ...)
 struct LzLayout {
-  size_t V, w, ra, rb, ab, scal, heff, vec, total;
+  size_t V, w, scal, coef, heff, vec, total;
 };
 
 int lz_layout(const reno_heff_desc* d, int kmax, LzLayout& L) {
   size_t hb = 0, vb = 0;
   if (reno_heff_workspace_bytes(d, &hb) != RENO_OK) return RENO_ERR_INVALID;
   const int64_t n = psi_elems(d);
-  if (reno_vec_workspace_bytes(n, &vb) != RENO_OK) return RENO_ERR_INVALID;
+  if (reno_vec_grouped_workspace_bytes(1, &vb) != RENO_OK) return RENO_ERR_INVALID;
   const size_t vbytes = (size_t)n * 16;
   size_t o = 0;
   L.V = o;
   o = al256(o + (size_t)(kmax + 1) * vbytes);
   L.w = o;
   o = al256(o + vbytes);
-  L.ra = o;
-  o = al256(o + vbytes);
-  L.rb = o;
-  o = al256(o + vbytes);
-  L.ab = o;
-  o = al256(o + (2 * (size_t)kmax + 4) * sizeof(double));
   L.scal = o;
-  o = al256(o + 4 * sizeof(double));
+  o = al256(o + (2 * (size_t)kmax + 4) * sizeof(double));
+  L.coef = o;
+  o = al256(o + 4 * ((size_t)kmax + 1) * sizeof(double));
   L.heff = o;
   o = al256(o + hb);
   L.vec = o;
@@ -120,15 +119,19 @@ bool tridiag_eig(int k, std::vector<double>& d, std::vector<double> e, std::vect
 
 // krylov.py:15-24: coefficients u (nrmv exp(dt w) u[0]) of the Krylov vectors
 // for the leading tridiagonal block of order k, as (re, im) pairs
-bool tridiag_coeffs(int k, const std::vector<double>& alpha, const std::vector<double>& beta, double nrmv,
-                    double dt_re, double dt_im, std::vector<double>& coef) {
-  std::vector<double> d(alpha.begin(), alpha.begin() + k), e(beta.begin(), beta.begin() + (k > 0 ? k - 1 : 0)), Z;
+// (ab = alpha_0, beta_0, alpha_1, ...)
+bool tridiag_coeffs(int k, const double* ab, double nrmv, double dt_re, double dt_im, double* coef) {
+  std::vector<double> d(k), e(k > 0 ? k - 1 : 0), Z;
+  for (int i = 0; i < k; ++i) {
+    d[i] = ab[2 * i];
+    if (i + 1 < k) e[i] = ab[2 * i + 1];
+  }
   for (double x : d)
     if (!std::isfinite(x)) return false;
   for (double x : e)
     if (!std::isfinite(x)) return false;
   if (!tridiag_eig(k, d, e, Z)) return false;
-  coef.assign(2 * (size_t)k, 0.0);
+  std::fill(coef, coef + 2 * (size_t)k, 0.0);
   for (int j = 0; j < k; ++j) {
     const double mag = nrmv * std::exp(dt_re * d[j]) * Z[j];  // Z[0][j]
     const double cr = mag * std::cos(dt_im * d[j]), ci = mag * std::sin(dt_im * d[j]);
@@ -151,11 +154,33 @@ extern "C" int reno_lanczos_workspace_bytes(const reno_heff_desc* desc, int32_t 
   return RENO_OK;
 }
 
+extern "C" int reno_lanczos_coefficients(int32_t count, const int32_t* k, const double* scal, int64_t ld,
+                                         const double* dt, double* coef) {
+  if (count < 0 || (count > 0 && (!k || !scal || !dt || !coef))) return RENO_ERR_INVALID;
+  for (int i = 0; i < count; ++i) {
+    if (k[i] < 1 || ld < 2 * (int64_t)k[i]) return RENO_ERR_INVALID;
+    const double* s = scal + i * ld;
+    if (!tridiag_coeffs(k[i], s + 1, s[0], dt[2 * i], dt[2 * i + 1], coef)) return RENO_ERR_NONFINITE;
+    coef += 2 * (size_t)k[i];
+  }
+  return RENO_OK;
+}
+
 extern "C" int reno_lanczos_expm(reno_ctx* ctx, const reno_heff_desc* desc, const void* L, const void* W1,
                                  const void* W2, const void* R, double dt_re, double dt_im, void* psi, int32_t kmax,
                                  int32_t* out_k, void* ws, size_t ws_bytes) {
+  return reno_lanczos_expm_to(ctx, desc, L, W1, W2, R, dt_re, dt_im, psi, psi, kmax, out_k, ws, ws_bytes);
+}
+
+// The host's share of an exponential is one read of the scalars, one upload
+// of coefficients and one read of the flag per convergence test, and tests
+// begin at j = 6: the reference's first approximation (j = 4) is only compared
+// at j = 6, where RENO_VOP_CHECK forms both from one read of the vectors.
+extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, const void* L, const void* W1,
+                                    const void* W2, const void* R, double dt_re, double dt_im, const void* psi,
+                                    void* out, int32_t kmax, int32_t* out_k, void* ws, size_t ws_bytes) {
   if (!ctx) return RENO_ERR_INVALID;
-  if (!desc || !psi || !out_k || !ws || kmax < 1)
+  if (!desc || !psi || !out || !out_k || !ws || kmax < 1)
     return set_error(ctx, RENO_ERR_INVALID, "reno_lanczos_expm: null argument or kmax < 1");
   if (desc->psi_dtype != RENO_C128)
     return set_error(ctx, RENO_ERR_INVALID, "reno_lanczos_expm: psi must be complex128");
@@ -166,14 +191,14 @@ extern "C" int reno_lanczos_expm(reno_ctx* ctx, const reno_heff_desc* desc, cons
   char* base = static_cast<char*>(ws);
   double2* V = reinterpret_cast<double2*>(base + Lz.V);
   double2* w = reinterpret_cast<double2*>(base + Lz.w);
-  double2* res[2] = {reinterpret_cast<double2*>(base + Lz.ra), reinterpret_cast<double2*>(base + Lz.rb)};
-  double* ab = reinterpret_cast<double*>(base + Lz.ab);
   double* scal = reinterpret_cast<double*>(base + Lz.scal);
+  double* ab = scal + 2;
+  double* dcoef = reinterpret_cast<double*>(base + Lz.coef);
   void* hws = base + Lz.heff;
   void* vws = base + Lz.vec;
   size_t hbytes = 0, vbytes = 0;
   reno_heff_workspace_bytes(desc, &hbytes);
-  reno_vec_workspace_bytes(n, &vbytes);
+  reno_vec_grouped_workspace_bytes(1, &vbytes);
   cudaStream_t st = ctx->stream;
   const double thresh = 100.0 * (double)n * DBL_EPSILON;
   int rc;
@@ -182,78 +207,96 @@ extern "C" int reno_lanczos_expm(reno_ctx* ctx, const reno_heff_desc* desc, cons
     rc = (call);                  \
     if (rc != RENO_OK) return rc; \
   } while (0)
-  LZ_TRY(check_cuda(ctx, cudaMemsetAsync(ab, 0, (2 * (size_t)kmax + 4) * sizeof(double), st),
-                    "reno_lanczos_expm: memset"));
+  // pinned: the scalars read, then the coefficients sent
+  const size_t nscal = 2 * (size_t)kmax + 4, pinned = nscal + 4 * ((size_t)kmax + 1);
+  if (ctx->host_scalars_count < pinned) {
+    if (ctx->host_scalars) cudaFreeHost(ctx->host_scalars);
+    ctx->host_scalars = nullptr;
+    ctx->host_scalars_count = 0;
+    void* p = nullptr;
+    LZ_TRY(check_cuda(ctx, cudaMallocHost(&p, pinned * sizeof(double)), "reno_lanczos_expm: pinned scalars"));
+    ctx->host_scalars = static_cast<double*>(p);
+    ctx->host_scalars_count = pinned;
+  }
+  double* host = ctx->host_scalars;
+  double* hcoef = host + nscal;
+  reno_vec_item it{};
+  it.n = n;
+  it.dtype = RENO_C128;
+  it.ldv = n;
+  auto read = [&](const double* from, size_t count) -> int {
+    int r = check_cuda(ctx, cudaMemcpyAsync(host + (from - scal), from, count * sizeof(double), cudaMemcpyDeviceToHost,
+                                            st), "reno_lanczos_expm: scalars");
+    return r != RENO_OK ? r : check_cuda(ctx, cudaStreamSynchronize(st), "reno_lanczos_expm: sync");
+  };
+  auto send = [&](size_t count) -> int {
+    return check_cuda(ctx, cudaMemcpyAsync(dcoef, hcoef, count * sizeof(double), cudaMemcpyHostToDevice, st),
+                      "reno_lanczos_expm: coefficients");
+  };
+  auto coefficients = [&](int k, double* to) -> int {
+    return tridiag_coeffs(k, host + 2, host[0], dt_re, dt_im, to)
+               ? RENO_OK
+               : set_error(ctx, RENO_ERR_NONFINITE, "reno_lanczos_expm: Lanczos scalars are not finite");
+  };
   LZ_TRY(reno_vec_norm(ctx, n, RENO_C128, psi, scal, vws, vbytes));
   LZ_TRY(reno_vec_scale_inv(ctx, n, RENO_C128, psi, scal, V));
-  std::vector<double> hab(2 * (size_t)kmax + 4), alpha, beta, coef;
-  double nrmv = -1.0;
-  int checked = 0, last = -1;  // last: index of res[] holding the previous check's result
-  auto read_scalars = [&](int j) -> int {
-    int r = check_cuda(ctx, cudaMemcpyAsync(hab.data(), ab, (2 * (size_t)j + 2) * sizeof(double),
-                                            cudaMemcpyDeviceToHost, st), "reno_lanczos_expm: scalars");
-    if (r == RENO_OK && nrmv < 0) {
-      r = check_cuda(ctx, cudaMemcpyAsync(&nrmv, scal, sizeof(double), cudaMemcpyDeviceToHost, st),
-                     "reno_lanczos_expm: norm");
-    }
-    if (r == RENO_OK) r = check_cuda(ctx, cudaStreamSynchronize(st), "reno_lanczos_expm: sync");
-    if (r != RENO_OK) return r;
-    if (!(nrmv > 0.0) || !std::isfinite(nrmv))
-      return set_error(ctx, RENO_ERR_NONFINITE, "reno_lanczos_expm: start vector is zero or not finite");
-    alpha.assign(j + 1, 0.0);
-    beta.assign(j + 1, 0.0);
-    for (int i = 0; i <= j; ++i) {
-      alpha[i] = hab[2 * i];
-      beta[i] = hab[2 * i + 1];
-    }
-    return RENO_OK;
-  };
-  // the result (V[0:k] coef, already formed in `from`) becomes psi
-  auto finish = [&](int k, const double2* from) -> int {
-    *out_k = k;
-    return check_cuda(ctx, cudaMemcpyAsync(psi, from, (size_t)n * 16, cudaMemcpyDeviceToDevice, st),
-                      "reno_lanczos_expm: copy out");
-  };
+  int checked = 0;
   for (int j = 0; j < n; ++j) {
     if (j >= kmax)
       return set_error(ctx, RENO_ERR_WORKSPACE, "reno_lanczos_expm: no convergence within kmax = " +
                                                     std::to_string(kmax) + " Krylov vectors; raise kmax");
-    LZ_TRY(reno_heff_apply(ctx, desc, L, W1, W2, R, V + (size_t)j * n, w, hws, hbytes));
-    LZ_TRY(reno_krylov_alpha(ctx, n, RENO_C128, w, V + (size_t)j * n, ab, j, vws, vbytes));
+    double2* vj = V + (size_t)j * n;
+    LZ_TRY(heff_apply_prepared(ctx, desc, L, W1, W2, R, vj, w, hws, hbytes, j > 0));
     const bool exhausted = (j == n - 1);
-    if (!exhausted) {
-      LZ_TRY(reno_krylov_orth(ctx, n, RENO_C128, w, V + (size_t)j * n, j > 0 ? V + (size_t)(j - 1) * n : nullptr,
-                              ab, j, vws, vbytes));
-      LZ_TRY(reno_vec_scale_inv(ctx, n, RENO_C128, w, ab + 2 * (size_t)j + 1, V + (size_t)(j + 1) * n));
+    it.j = j;
+    it.scalars = ab;
+    if (exhausted) {
+      LZ_TRY(reno_krylov_alpha(ctx, n, RENO_C128, w, vj, ab, j, vws, vbytes));
+    } else {
+      it.x = vj;
+      it.y = j > 0 ? vj - n : nullptr;
+      it.out = w;
+      LZ_TRY(reno_vec_grouped(ctx, RENO_VOP_STEP, 1, &it, 0.0, 0.0, vws, vbytes));
     }
-    if (!(exhausted || (j > 3 && j % 2 == 0))) continue;
-    LZ_TRY(read_scalars(j));
-    int kk = -1;  // breakdown before this point
-    for (int i = checked; i < (exhausted ? j : j + 1); ++i)
-      if (beta[i] < thresh) {
-        kk = i;
+    const bool last_chance = j + 1 >= kmax;  // a breakdown before kmax is still found
+    if (!(exhausted || (j > 5 && j % 2 == 0) || last_chance)) continue;
+    LZ_TRY(read(scal, 2 + 2 * (size_t)j + (exhausted ? 1 : 2)));
+    if (!(host[0] > 0.0) || !std::isfinite(host[0]))
+      return set_error(ctx, RENO_ERR_NONFINITE, "reno_lanczos_expm: start vector is zero or not finite");
+    int k = exhausted ? j + 1 : 0;  // vectors of the final result, 0 = not known yet
+    const int upto = exhausted ? j : j + 1;
+    for (int i = checked; i < upto; ++i)
+      if (host[2 + 2 * i + 1] < thresh) {  // the Krylov space closed at i; nothing after it is used
+        k = i + 1;
         break;
       }
-    checked = exhausted ? j : j + 1;
-    const int k = kk >= 0 ? kk + 1 : j + 1;
-    if (!tridiag_coeffs(k, alpha, beta, nrmv, dt_re, dt_im, coef))
-      return set_error(ctx, RENO_ERR_NONFINITE, "reno_lanczos_expm: Lanczos scalars are not finite");
-    // coefficients to the device (the scalars area past the Lanczos entries)
-    double* dcoef = reinterpret_cast<double*>(w);  // w is free until the next matvec
-    LZ_TRY(check_cuda(ctx, cudaMemcpyAsync(dcoef, coef.data(), coef.size() * sizeof(double), cudaMemcpyHostToDevice,
-                                           st), "reno_lanczos_expm: coefficients"));
-    const int slot = last == 0 ? 1 : 0;
-    LZ_TRY(reno_vec_lincomb(ctx, n, k, RENO_C128, V, n, dcoef, res[slot]));
-    if (kk >= 0 || exhausted) return finish(k, res[slot]);
-    if (last >= 0) {
-      LZ_TRY(reno_vec_allclose(ctx, n, RENO_C128, res[last], res[slot], 1e-5, 1e-8, scal + 2, vws, vbytes));
-      double flag = 0.0;
-      LZ_TRY(check_cuda(ctx, cudaMemcpyAsync(&flag, scal + 2, sizeof(double), cudaMemcpyDeviceToHost, st),
-                        "reno_lanczos_expm: allclose"));
+    checked = upto;
+    if (k > 0) {
+      LZ_TRY(coefficients(k, hcoef));
+      LZ_TRY(send(2 * (size_t)k));
+      LZ_TRY(reno_vec_lincomb(ctx, n, k, RENO_C128, V, n, dcoef, out));
+      // the next exponential may refill the pinned coefficients: wait for the copy
       LZ_TRY(check_cuda(ctx, cudaStreamSynchronize(st), "reno_lanczos_expm: sync"));
-      if (flag == 1.0) return finish(k, res[slot]);
+      *out_k = k;
+      return RENO_OK;
     }
-    last = slot;
+    if (!(j > 5 && j % 2 == 0)) continue;
+    LZ_TRY(coefficients(j + 1, hcoef));
+    LZ_TRY(coefficients(j - 1, hcoef + 2 * (size_t)(j + 1)));
+    LZ_TRY(send(4 * (size_t)j));
+    it.j = j + 1;
+    it.x = V;
+    it.y = nullptr;
+    it.s = dcoef;
+    it.out = out;
+    it.scalars = scal + 1;
+    LZ_TRY(reno_vec_grouped(ctx, RENO_VOP_CHECK, 1, &it, 1e-5, 1e-8, vws, vbytes));
+    it.s = nullptr;
+    LZ_TRY(read(scal + 1, 1));
+    if (host[1] == 1.0) {
+      *out_k = j + 1;
+      return RENO_OK;
+    }
   }
 #undef LZ_TRY
   return set_error(ctx, RENO_ERR_INVALID, "reno_lanczos_expm: empty vector");

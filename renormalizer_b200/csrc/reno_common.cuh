@@ -16,8 +16,10 @@ struct reno_ctx {
   cudaStream_t stream = nullptr;
   int num_sms = 148;
   std::string last_error;
-  // pinned host slots for scalars read back by the host (Krylov alpha/beta ...)
+  // pinned host memory for scalars that cross between host and device
+  // (Krylov alpha / beta, coefficients), made on first use
   double* host_scalars = nullptr;
+  size_t host_scalars_count = 0;
 };
 
 namespace reno {
@@ -58,6 +60,9 @@ inline int check_cuda(reno_ctx* ctx, cudaError_t e, const char* what) {
   } while (0)
 
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+int heff_apply_prepared(reno_ctx* ctx, const reno_heff_desc* d, const void* L, const void* W1, const void* W2,
+                        const void* R, const void* psi, void* y, void* ws, size_t ws_bytes, bool prepared);
 
 // Opt a kernel into `bytes` of dynamic shared memory once per device:
 // function attributes belong to each device's context, so a process that

@@ -10,12 +10,13 @@ arithmetic (FP64 DMMA or BF16x3 / TF32x3 split products).
 from __future__ import annotations
 
 import ctypes
+import math
 from typing import List, Sequence
 
 import numpy as np
 import torch
 
-from ._native import Engine, HeffDesc, PREC, dtype_code
+from ._native import Engine, HeffDesc, PREC, RENO_C128, addresses, dtype_code
 from .backend import backend
 
 
@@ -24,7 +25,7 @@ def as_device(t, device=None, dtype=None) -> torch.Tensor:
     if device is None:
         device = backend.device
     if isinstance(t, torch.Tensor):
-        out = t.to(device=device)
+        out = t if t.device == device else t.to(device=device)
     else:
         out = torch.from_numpy(np.ascontiguousarray(np.asarray(t))).to(device=device)
     if dtype is not None:
@@ -112,12 +113,58 @@ class HeffOperator:
 MAX_GROUP = 128  # problems per grouped launch (reno_heff_apply_grouped)
 
 
+class Rows(list):
+    """1-D complex128 device tensors cut from one buffer, with their addresses
+    (``ptrs``, uint64): what a lockstep exponential hands to its operators and
+    apply_grouped hands back, so that neither side looks at each tensor."""
+
+    def __init__(self, tensors, ptrs):
+        super().__init__(tensors)
+        self.ptrs = ptrs
+
+    def intact(self) -> bool:
+        """whether the list still holds the vectors it was made of"""
+        return len(self) == len(self.ptrs) and [t.data_ptr() for t in self] == self.ptrs.tolist()
+
+
+def _apply_rows(ops: Sequence["HeffOperator"], psis: Rows) -> "Rows":
+    """apply_grouped for FP64 operators of one kind on checked vectors, or None"""
+    if len(ops) != len(psis) or not psis.intact():
+        return None
+    d0 = ops[0].desc
+    kind = (d0.nsite, d0.env_dtype, d0.mpo_dtype)
+    if any(o.prec != "fp64" or (o.desc.nsite, o.desc.env_dtype, o.desc.mpo_dtype) != kind or o.engine is not ops[0].engine
+           for o in ops):
+        return None
+    eng = ops[0].engine
+    eng.sync_stream()
+    sizes = [p.numel() for p in psis]
+    if any(n != math.prod(o.cshape) for n, o in zip(sizes, ops)):
+        return None
+    flat = torch.empty(sum(sizes), dtype=torch.complex128, device=psis[0].device)
+    ends = np.cumsum(sizes)
+    ptrs = np.uint64(flat.data_ptr()) + (16 * (ends - sizes)).astype(np.uint64)
+    for o in ops:
+        o.desc.psi_dtype = RENO_C128
+    none = np.zeros(len(ops), dtype=np.uint64)
+    fixed = [addresses([o.L for o in ops]), addresses([o.W[0] for o in ops]) if d0.nsite else none,
+             addresses([o.W[1] for o in ops]) if d0.nsite == 2 else none, addresses([o.R for o in ops])]
+    for c0 in range(0, len(ops), MAX_GROUP):
+        part = slice(c0, c0 + MAX_GROUP)
+        eng.heff_apply_grouped([o.desc for o in ops[part]], *[f[part] for f in fixed], psis.ptrs[part], ptrs[part])
+    return Rows([y.view(o.cshape) for y, o in zip(flat.split(sizes), ops)], ptrs)
+
+
 def apply_grouped(ops: Sequence["HeffOperator"], psis: Sequence[torch.Tensor]) -> List[torch.Tensor]:
     """[op.apply(psi) for op, psi in zip(ops, psis)] for independent local
     problems.  FP64 operators with the same number of sites and dtypes go
     through reno_heff_apply_grouped, up to 128 per launch; split-precision
     operators (whose fused chains are not grouped) are applied one by one.
     Each result equals that operator's own apply."""
+    if isinstance(psis, Rows) and len(ops):
+        ys = _apply_rows(ops, psis)
+        if ys is not None:
+            return ys
     ys: List[torch.Tensor] = [None] * len(ops)
     batch = {}
     for i, (op, psi) in enumerate(zip(ops, psis)):

@@ -4,8 +4,9 @@ renormalizer/lib/krylov/krylov.py:27-84 (``expm_krylov``).
 The Krylov basis V, the matvecs and every vector operation (vdot, norm,
 three-term recurrence, V @ coeffs, allclose) stay in HBM and run in
 libreno_b200; alpha/beta are produced on the device in FP64.  The small
-tridiagonal eigenproblem is solved in FP64 on the host with the same SciPy
-routine the reference uses (krylov.py:15-24).
+tridiagonal eigenproblem (krylov.py:15-24) is solved in FP64 on the host.  A
+HeffOperator's whole exponential is one call of the library
+(reno_lanczos_expm_to); other operators are driven from here.
 
 Host synchronisation happens only where the reference makes a decision that
 needs the scalars: at its convergence checks (every even j > 3) and when the
@@ -17,12 +18,14 @@ the ones the reference returns.
 """
 from __future__ import annotations
 
+import math
+
 import numpy as np
 import torch
-from scipy.linalg import eigh_tridiagonal
 
-from ._native import Engine, VOP_STEP, dtype_code, h2d
-from .hop_expr import as_device
+from ._native import (RENO_C128, RENO_OK, VEC_ITEM, VOP_ALPHA, VOP_CHECK, VOP_LINCOMB, VOP_NORM, VOP_SCALE_INV, VOP_STEP,
+                      Engine, addresses, dtype_code, h2d, load_library, raw_view)
+from .hop_expr import HeffOperator, Rows, as_device
 
 EPS = np.finfo(float).eps
 
@@ -47,14 +50,35 @@ class KrylovTolerance:
 tolerance = KrylovTolerance()
 
 
+def _coefficients(rows, ks, dts):
+    """The Krylov vectors' coefficients (krylov.py:15-24:
+    u_hess @ (v_norm * exp(dt * w_hess) * u_hess[0])) of several problems, one
+    after the other as (re, im) pairs; row i of ``rows`` holds the start norm,
+    then alpha_0, beta_0, alpha_1, ..."""
+    rows = np.ascontiguousarray(rows, dtype=np.float64)
+    ks = np.asarray(ks, dtype=np.int32)
+    steps = np.asarray(dts, dtype=np.complex128)
+    coef = np.empty(2 * int(ks.sum()))
+    st = load_library().reno_lanczos_coefficients(len(ks), ks.ctypes.data, rows.ctypes.data, rows.shape[1],
+                                                  steps.ctypes.data, coef.ctypes.data)
+    if st == RENO_OK:
+        return coef
+    out = []
+    for r, k, dt in zip(rows, ks.tolist(), steps.tolist()):
+        a, b = r[1:2 * k:2], r[2:2 * k - 1:2]
+        # entries past a breakdown may be garbage; only the used ones must be finite
+        if not (np.all(np.isfinite(a)) and np.all(np.isfinite(b))):
+            raise FloatingPointError("expm_krylov: Lanczos scalars are not finite")
+        w, u = np.linalg.eigh(np.diag(a) + np.diag(b, k=-1) + np.diag(b, k=1))
+        out.append((u @ (r[0] * np.exp(dt * w) * u[0])).astype(np.complex128).view(np.float64))
+    return np.concatenate(out)
+
+
 def _tridiag_coeffs(alpha, beta, v_norm, dt):
-    """krylov.py:15-24 : u_hess @ (v_norm * exp(dt * w_hess) * u_hess[0])."""
-    try:
-        w_hess, u_hess = eigh_tridiagonal(alpha, beta)
-    except np.linalg.LinAlgError:
-        h = np.diag(alpha) + np.diag(beta, k=-1) + np.diag(beta, k=1)
-        w_hess, u_hess = np.linalg.eigh(h)
-    return u_hess @ (v_norm * np.exp(dt * w_hess) * u_hess[0])
+    """_coefficients of one problem, complex"""
+    row = np.zeros(2 * len(alpha))
+    row[0], row[1::2], row[2::2] = v_norm, alpha, beta
+    return _coefficients(row[None], [len(alpha)], [dt]).view(np.complex128)
 
 
 class _Krylov:
@@ -101,6 +125,7 @@ def _expm_krylov_steps(dt, vstart, block_size=50):
     work_dtype = torch.complex128 if (v.is_complex() or dt_cplx) else torch.float64
     if v.dtype != work_dtype:
         v = v.to(work_dtype)
+    native = isinstance(eng, Engine)  # a stand-in engine has the single operations only
     K = _Krylov(eng, n, work_dtype, v.device, block_size)
     eng.vec_norm(v, K.scal)                  # nrmv = ||vstart||
     eng.scale_inv(v, K.scal, K.V[0])         # V[0] = vstart / nrmv
@@ -119,11 +144,7 @@ def _expm_krylov_steps(dt, vstart, block_size=50):
         return ab[0::2], ab[1::2]
 
     def coeffs_for(alpha, beta, k):
-        # entries past a breakdown may be garbage; only the used ones must be finite
-        a, b = alpha[: k + 1], beta[:k]
-        if not (np.all(np.isfinite(a)) and np.all(np.isfinite(b))):
-            raise FloatingPointError("expm_krylov: Lanczos scalars are not finite")
-        return _tridiag_coeffs(a, b, state["nrmv"], dt)
+        return _tridiag_coeffs(alpha[: k + 1], beta[:k], state["nrmv"], dt)
 
     def breakdown_before(j, beta):
         # first unchecked i < j with beta_i below the reference's threshold
@@ -139,7 +160,7 @@ def _expm_krylov_steps(dt, vstart, block_size=50):
             w = w.to(work_dtype)
         if not w.is_contiguous():
             w = w.contiguous()
-        if j == n - 1 or not v.is_cuda:
+        if j == n - 1 or not native:
             eng.krylov_alpha(w, K.V[j], K.ab, j)
         if j == n - 1:
             alpha, beta = host_scalars(j)
@@ -149,7 +170,7 @@ def _expm_krylov_steps(dt, vstart, block_size=50):
         if K.V.shape[0] == j + 1:
             K.grow(block_size)
         vprev = K.V[j - 1] if j > 0 else None
-        if v.is_cuda:  # alpha_j, w -= ..., beta_j = ||w|| and V[j+1] = w / beta_j in one operation
+        if native:  # alpha_j, w -= ..., beta_j = ||w|| and V[j+1] = w / beta_j in one operation
             eng.vec_grouped(VOP_STEP, [(n, dtype_code(v), j, K.V[j], vprev, w, K.ab, None, n)])
         else:
             eng.krylov_orth(w, K.V[j], vprev, K.ab, j)
@@ -169,11 +190,41 @@ def _expm_krylov_steps(dt, vstart, block_size=50):
             state["res"] = new_res
 
 
+_APPLY = HeffOperator.apply
+
+
+def _native_expm(op, dt, vstart, kmax):
+    """The exponential in one library call, or None where the generic driver
+    serves it: real results, an operator whose ``apply`` was replaced, other
+    tolerances than the reference's, more than kmax vectors, scalars that are
+    not finite (the driver raises for those)."""
+    if not isinstance(op, HeffOperator) or type(op).apply is not _APPLY or "apply" in vars(op) \
+            or not isinstance(op.engine, Engine):
+        return None
+    if (tolerance.rtol, tolerance.atol) != (1e-5, 1e-8):
+        return None
+    v = as_device(vstart).reshape(-1)
+    if not v.is_cuda or v.device != op.L.device or v.numel() != math.prod(op.cshape):
+        return None
+    dt = complex(dt)
+    if not v.is_complex():
+        if dt.imag == 0.0:
+            return None
+        v = v.to(torch.complex128)
+    op.desc.psi_dtype = RENO_C128
+    op.engine.sync_stream()
+    return op.engine.lanczos_expm(op.desc, op.L, op.W[0] if op.W else None, op.W[1] if op.nsite == 2 else None, op.R,
+                                  dt, v, kmax)
+
+
 def expm_krylov(Afunc, dt, vstart, block_size=50):
     """Krylov approximation of expm(dt*A) @ vstart for Hermitian A.
 
     Returns (vector, number of matvecs) like the reference.  ``Afunc`` maps a
     1-D device vector to a device vector (e.g. a HeffOperator)."""
+    res = _native_expm(Afunc, dt, vstart, block_size)
+    if res is not None:
+        return res
     gen = _expm_krylov_steps(dt, vstart, block_size)
     try:
         x = next(gen)
@@ -201,11 +252,166 @@ def expm_krylov_batch(group_apply, dts, vstarts, block_size=50):
         dts = [dts] * m
     if m == 0:
         return []
-    return _LockstepKrylov(dts, vstarts, block_size).run(group_apply)
+    vs = [as_device(v).reshape(-1) for v in vstarts]
+    if isinstance(Engine.get(vs[0].device), Engine) and all(
+            v.is_cuda and v.device == vs[0].device and (v.is_complex() or np.iscomplex(dt)) for v, dt in zip(vs, dts)):
+        return _LockstepRows(dts, vs, block_size).run(group_apply)
+    return _LockstepKrylov(dts, vs, block_size).run(group_apply)
+
+
+class _LockstepRows:
+    """_LockstepKrylov for complex vectors on the GPU, without per-problem work
+    between the checks: the vectors of all problems stand side by side in one
+    buffer (row j holds every problem's V[j], item p from element off[p] on),
+    so one operation's table of addresses is a few array expressions, and the
+    Krylov vectors handed out are one split of a row.  A problem that ends
+    leaves the table; its columns stay where they are."""
+
+    def __init__(self, dts, vs, block_size):
+        self.block_size = block_size
+        self.dts = [complex(dt) for dt in dts]
+        self.vs = [v if v.is_complex() else v.to(torch.complex128) for v in vs]
+        self.device = vs[0].device
+        self.eng = Engine.get(self.device)
+        m = len(vs)
+        self.sizes = [v.numel() for v in vs]
+        self.n = np.array(self.sizes, dtype=np.int64)
+        self.off = np.concatenate([[0], np.cumsum(self.n)[:-1]])
+        self.total = int(self.n.sum())
+        self.rows = block_size
+        self.V = torch.empty((self.rows, self.total), dtype=torch.complex128, device=self.device)
+        self.ab_len = 2 * block_size + 2
+        # per problem: allclose flag, start norm, then (alpha_0, beta_0, alpha_1, ...)
+        self.S = torch.zeros((m, 2 + self.ab_len), dtype=torch.float64, device=self.device)
+        self.checked = np.zeros(m, dtype=np.int64)
+        every = np.arange(m)
+        start = self._table(every)
+        start["x"], start["scalars"] = addresses(self.vs), self._scalar(1, every)
+        self.eng.vec_grouped_table(VOP_NORM, start)
+        start["s"], start["out"] = self._scalar(1, every), self._vec(0, every)
+        self.eng.vec_grouped_table(VOP_SCALE_INV, start)
+
+    def _table(self, idx):
+        t = np.zeros(len(idx), dtype=VEC_ITEM)
+        t["n"], t["dtype"], t["ldv"] = self.n[idx], RENO_C128, self.total
+        return t
+
+    def _vec(self, j, idx):
+        """addresses of the problems' V[j]"""
+        return np.uint64(self.V.data_ptr()) + (16 * (j * self.total + self.off[idx])).astype(np.uint64)
+
+    def _scalar(self, k, idx):
+        return np.uint64(self.S.data_ptr()) + (8 * (idx * self.S.shape[1] + k)).astype(np.uint64)
+
+    def _grow(self):
+        V = torch.empty((self.rows + self.block_size, self.total), dtype=torch.complex128, device=self.device)
+        V[: self.rows] = self.V
+        S = torch.zeros((self.S.shape[0], self.S.shape[1] + 2 * self.block_size), dtype=torch.float64,
+                        device=self.device)
+        S[:, : self.S.shape[1]] = self.S
+        self.V, self.S, self.rows = V, S, V.shape[0]
+
+    def _images(self, group_apply, active, j):
+        """group_apply on the active problems' V[j]: the images (kept alive) and their addresses"""
+        row = self.V[j].split(self.sizes)
+        xs = Rows([row[p] for p in active], self._vec(j, active))
+        ws = group_apply(active.tolist(), xs)
+        if isinstance(ws, Rows) and ws.intact():
+            return ws, ws.ptrs
+        out = []
+        for p, w in zip(active, ws):
+            w = w.reshape(-1)
+            if w.dtype != torch.complex128:
+                w = w.to(torch.complex128)
+            assert w.device == self.device and w.numel() == self.sizes[p]
+            out.append(raw_view(w).contiguous())
+        return out, np.array([w.data_ptr() for w in out], dtype=np.uint64)
+
+    def run(self, group_apply):
+        m = len(self.vs)
+        result = [None] * m
+        buf = [torch.empty(self.total, dtype=torch.complex128, device=self.device) for _ in range(2)]
+        active = np.arange(m)
+        j = 0
+        while len(active):
+            if self.rows == j + 1:
+                self._grow()
+            ws, wp = self._images(group_apply, active, j)
+            ends = self.n[active] == j + 1
+            for op, sel in ((VOP_ALPHA, ends), (VOP_STEP, ~ends)):
+                if not sel.any():
+                    continue
+                idx = active[sel]
+                t = self._table(idx)
+                t["j"], t["scalars"] = j, self._scalar(2, idx)
+                if op == VOP_ALPHA:
+                    t["x"], t["y"] = wp[sel], self._vec(j, idx)
+                else:
+                    t["x"], t["out"] = self._vec(j, idx), wp[sel]
+                    if j:
+                        t["y"] = self._vec(j - 1, idx)
+                self.eng.vec_grouped_table(op, t)
+            test = 3 < j and j % 2 == 0
+            if test or ends.any():
+                active = self._decide(active, ends, j, test, result, buf)
+            else:
+                active = active[~ends]
+            j += 1
+        return result
+
+    def _decide(self, active, ends, j, test, result, buf):
+        """The reference's decisions at step j: problems at the end of their
+        space, breakdowns since the last look, and (test) the convergence of
+        the others; returns those that go on."""
+        sc = self.S.cpu().numpy()
+        look = active if test else active[ends]
+        assert np.all(sc[look, 1] > 0)
+        if not np.all(np.isfinite(sc[look, 1])):
+            raise FloatingPointError("expm_krylov: start vector is not finite")
+        final, checks = [], []  # (problem, vectors)
+        for p in look.tolist():
+            end = self.n[p] == j + 1
+            upto = j if end else j + 1
+            beta = sc[p, 3 + 2 * self.checked[p]:3 + 2 * upto:2]
+            low = np.flatnonzero(beta < 100 * self.n[p] * EPS)
+            if len(low):
+                final.append((p, int(self.checked[p]) + int(low[0]) + 1))
+            elif end:
+                final.append((p, j + 1))
+            elif j > 4:
+                checks.append((p, j + 1))
+            self.checked[p] = upto
+        # of the final ones, then of each test's two approximations
+        jobs = final + [(p, q) for p, k in checks for q in (k, k - 2)]
+        if jobs:
+            who, ks = np.array([p for p, _ in jobs]), np.array([k for _, k in jobs])
+            dev = h2d(_coefficients(sc[who, 1:], ks, [self.dts[p] for p in who]), self.device)
+            at = np.uint64(dev.data_ptr()) + (16 * (np.cumsum(ks) - ks)).astype(np.uint64)
+            at = np.concatenate([at[:len(final)], at[len(final)::2]])
+        out = buf[(j // 2) % 2]
+        done = set()
+        for op, which, first in ((VOP_LINCOMB, final, 0), (VOP_CHECK, checks, len(final))):
+            if not which:
+                continue
+            idx = np.array([p for p, _ in which])
+            t = self._table(idx)
+            t["j"] = [k for _, k in which]
+            t["x"], t["s"] = self._vec(0, idx), at[first:first + len(which)]
+            t["out"] = np.uint64(out.data_ptr()) + (16 * self.off[idx]).astype(np.uint64)
+            t["scalars"] = self._scalar(0, idx)
+            self.eng.vec_grouped_table(op, t, tolerance.rtol, tolerance.atol)
+        if checks:
+            flags = self.S[:, 0].cpu().numpy()
+            final = final + [(p, k) for p, k in checks if flags[p] == 1.0]
+        for p, k in final:
+            # its own memory: the row buffer is written again while other problems go on
+            result[p] = (out[self.off[p]:self.off[p] + self.sizes[p]].clone(), k)
+            done.add(p)
+        return np.array([p for p in active.tolist() if p not in done], dtype=np.int64)
 
 
 class _LockstepKrylov:
-    """The state of expm_krylov (_expm_krylov_steps) for m problems, with the
+    """The general form (real vectors, other devices): the state of expm_krylov (_expm_krylov_steps) for m problems, with the
     alpha/beta arrays of all problems in one device array AB (row p) and the
     start norms / allclose flags in SC (columns 0 / 2)."""
 
@@ -264,10 +470,7 @@ class _LockstepKrylov:
             self.AB = AB
 
     def _coeffs(self, p, alpha, beta, k):
-        a, b = alpha[: k + 1], beta[:k]
-        if not (np.all(np.isfinite(a)) and np.all(np.isfinite(b))):
-            raise FloatingPointError("expm_krylov: Lanczos scalars are not finite")
-        return _tridiag_coeffs(a, b, self.nrmv[p], self.dts[p])
+        return _tridiag_coeffs(alpha[: k + 1], beta[:k], self.nrmv[p], self.dts[p])
 
     def _breakdown_before(self, p, j, beta):
         for i in range(self.checked[p], j):
@@ -313,15 +516,15 @@ class _LockstepKrylov:
                 W[p] = w
             term = [p for p in active if j == self.n[p] - 1]
             cont = [p for p in active if j < self.n[p] - 1]
-            cuda = self.device.type == "cuda"
+            native = isinstance(self.eng, Engine)
             self._op(VOP_ALPHA, [(p, j, W[p], self.V[p][j], None, self.AB[p], None)
-                                 for p in (term if cuda else active)])
+                                 for p in (term if native else active)])
             for p in cont:
                 if self.V[p].shape[0] == j + 1:
                     self._grow(p)
-            self._op(VOP_STEP if cuda else VOP_ORTH,
+            self._op(VOP_STEP if native else VOP_ORTH,
                      [(p, j, self.V[p][j], self.V[p][j - 1] if j > 0 else None, W[p], self.AB[p], None) for p in cont])
-            if not cuda:
+            if not native:
                 self._op(VOP_SCALE_INV, [(p, 0, W[p], None, self.V[p][j + 1], None, self.AB[p][2 * j + 1:])
                                          for p in cont])
             check = cont if (3 < j and j % 2 == 0) else []

@@ -943,7 +943,7 @@ class Mps:
             return stop.value
 
     def _krylov(self, op: HeffOperator, dt, vec: torch.Tensor):
-        return expm_krylov(lambda y: op.apply(y), dt, vec.reshape(-1))
+        return expm_krylov(op, dt, vec.reshape(-1))
 
     def _evolve_tdvp_ps(self, mpo: Mpo, evolve_dt) -> "Mps":
         return self._drive(self._evolve_tdvp_ps_steps(mpo, evolve_dt))

@@ -75,29 +75,33 @@ class QNBlock:
     vpad: int = 0
 
 
-def _i64_many(arrays, device, float_last=False):
-    """several int64 index lists (the last one float64, carried as its bits,
-    when ``float_last``) in one host-to-device transfer; returns one device
-    view per list"""
-    host = [np.asarray(a, dtype=np.int64) for a in (arrays[:-1] if float_last else arrays)]
-    if float_last:
-        host.append(np.ascontiguousarray(arrays[-1], dtype=np.float64).view(np.int64))
+def _i64_many(arrays, device):
+    """several int64 index lists in one host-to-device transfer; returns one
+    device view per list"""
+    host = [np.asarray(a, dtype=np.int64) for a in arrays]
     flat = np.concatenate(host) if host else np.zeros(0, np.int64)
-    dev = h2d(flat, device, np.int64) if device.type == "cuda" else torch.as_tensor(flat, device=device)
-    out, off = [], 0
-    for h in host:
-        out.append(dev[off: off + h.size])
-        off += h.size
-    if float_last:
-        out[-1] = out[-1].view(torch.float64)
-    return out
+    dev = h2d(flat, device) if device.type == "cuda" else torch.as_tensor(flat, device=device)
+    return list(dev.split([h.size for h in host]))
 
 
-def _gather(eng: Engine, mat: torch.Tensor, lset, rset) -> torch.Tensor:
-    out = torch.empty((len(lset), len(rset)), dtype=mat.dtype, device=mat.device)
-    rows, cols = _i64_many([lset, rset], mat.device)
+def _gather(eng: Engine, mat: torch.Tensor, rows, cols) -> torch.Tensor:
+    """mat[rows, :][:, cols] for device index lists"""
+    out = torch.empty((rows.numel(), cols.numel()), dtype=mat.dtype, device=mat.device)
     eng.qn_gather(mat, rows, cols, out)
     return out
+
+
+def _sectors(lq, rq, qntot):
+    """(nl, nr, lset, rset) of every QN sector with rows and columns, in the reference's order"""
+    found = []
+    for nl in qn_sectors(lq):
+        nr = tuple(qntot - np.array(nl))
+        rset = np.where(get_qn_mask(rq, nr))[0]
+        if len(rset):
+            found.append((nl, nr, np.where(get_qn_mask(lq, nl))[0], rset))
+    if not found:
+        raise ValueError("Invalid quantum number")
+    return found
 
 
 def _pad_counts(m, n, full_matrices=True, opt_full_matrices=True):
@@ -124,18 +128,13 @@ def qn_block_svd(coef: torch.Tensor, qnbigl, qnbigr, qntot, full_matrices=True, 
     lq = qnbigl.reshape(-1, qs)
     rq = qnbigr.reshape(-1, qs)
     blocks: List[QNBlock] = []
-    for nl in qn_sectors(lq):
-        nr = tuple(qntot - np.array(nl))
-        rset = np.where(get_qn_mask(rq, nr))[0]
-        if len(rset) == 0:
-            continue
-        lset = np.where(get_qn_mask(lq, nl))[0]
-        blk = _gather(eng, mat, lset, rset)
+    found = _sectors(lq, rq, qntot)
+    dev = _i64_many([x for f in found for x in f[2:]], mat.device)
+    for i, (nl, nr, lset, rset) in enumerate(found):
+        blk = _gather(eng, mat, dev[2 * i], dev[2 * i + 1])
         U, S, Vh = torch.linalg.svd(blk, full_matrices=False)
         upad, vpad = _pad_counts(len(lset), len(rset), full_matrices, opt_full_matrices)
         blocks.append(QNBlock(nl, nr, lset, rset, U, None, S, Vh, upad, vpad))
-    if not blocks:
-        raise ValueError("Invalid quantum number")
     Sh = torch.cat([b.S_dev for b in blocks]).cpu().numpy() if blocks else np.zeros(0)
     off = 0
     for b in blocks:
@@ -145,10 +144,27 @@ def qn_block_svd(coef: torch.Tensor, qnbigl, qnbigr, qntot, full_matrices=True, 
     return blocks, rows, cols
 
 
+@dataclass
+class _QrBlock:
+    """One QN block of a QR ("L") or RQ ("R").  For RQ the block is gathered
+    with both index lists reversed and then conjugate-transposed, so that it
+    goes to the same QR; rows / cols are the lists as gathered, place the
+    result's columns in the assembled factors, and the *_d their device
+    copies."""
+    nl: tuple
+    nr: tuple
+    rows: np.ndarray
+    cols: np.ndarray
+    place: np.ndarray
+    rows_d: torch.Tensor
+    cols_d: torch.Tensor
+    place_d: torch.Tensor
+    blk: torch.Tensor
+
+
 def _qr_begin(coef: torch.Tensor, qnbigl, qnbigr, qntot, system: str):
-    """The QN blocks of one QR / RQ (qn_block_qr) gathered and, for RQ,
-    reversed and conjugate-transposed: (found, rows, cols), found holding
-    (nl, nr, lset, rset, block to factorise) per block."""
+    """The QN blocks of one QR / RQ (qn_block_qr), gathered: (blocks, rows,
+    cols, arange), all index lists in one transfer."""
     if system not in ("L", "R"):
         raise AssertionError("system must be L or R for QR")
     eng = Engine.get(coef.device)
@@ -157,33 +173,22 @@ def _qr_begin(coef: torch.Tensor, qnbigl, qnbigr, qntot, system: str):
     mat = coef.reshape(rows, cols).contiguous()
     qntot = np.asarray(qntot)
     qs = len(qntot)
-    lq = qnbigl.reshape(-1, qs)
-    rq = qnbigr.reshape(-1, qs)
-    found = []
-    for nl in qn_sectors(lq):
-        nr = tuple(qntot - np.array(nl))
-        rset = np.where(get_qn_mask(rq, nr))[0]
-        if len(rset) == 0:
-            continue
-        lset = np.where(get_qn_mask(lq, nl))[0]
-        blk = _gather(eng, mat, lset, rset)
-        if system == "R":
-            blk = blk.flip([0, 1]).mH.resolve_conj().contiguous()
-        found.append((nl, nr, lset, rset, blk))
-    if not found:
-        raise ValueError("Invalid quantum number")
-    return found, rows, cols
-
-
-def _qr_end(found, Qs, Rs, system: str):
+    found = _sectors(qnbigl.reshape(-1, qs), qnbigr.reshape(-1, qs), qntot)
+    flip = -1 if system == "R" else 1
+    lists, off, kmax = [], 0, 0
+    for _, _, lset, rset in found:
+        k = min(len(lset), len(rset))
+        lists += [lset[::flip], rset[::flip], np.arange(off, off + k)[::flip]]
+        off, kmax = off + k, max(kmax, k)
+    dev = _i64_many(lists + [np.arange(kmax)], mat.device)
     blocks = []
-    for (nl, nr, lset, rset, _), Q, R in zip(found, Qs, Rs):
-        if system == "L":
-            blocks.append(QNBlock(nl, nr, lset, rset, Q, None, None, R))
-        else:
-            blocks.append(QNBlock(nl, nr, lset, rset, R.mH.flip([0, 1]).resolve_conj().contiguous(), None, None,
-                                  Q.mH.flip([0, 1]).resolve_conj().contiguous()))
-    return blocks
+    for i, (nl, nr, _, _) in enumerate(found):
+        blk = _gather(eng, mat, dev[3 * i], dev[3 * i + 1])
+        if system == "R":
+            out = torch.empty((blk.shape[1], blk.shape[0]), dtype=blk.dtype, device=blk.device)
+            blk = torch.conj_physical(blk.transpose(0, 1), out=out)
+        blocks.append(_QrBlock(nl, nr, *lists[3 * i:3 * i + 3], *dev[3 * i:3 * i + 3], blk))
+    return blocks, rows, cols, dev[-1]
 
 
 def qn_block_qr(coef: torch.Tensor, qnbigl, qnbigr, qntot, system: str):
@@ -195,29 +200,39 @@ def qn_block_qr(coef: torch.Tensor, qnbigl, qnbigr, qntot, system: str):
     same order as LAPACK's RQ (last row first, pivot on its last entry), so R
     and Q agree with scipy.linalg.rq including the signs, not only up to a
     rotation."""
-    found, rows, cols = _qr_begin(coef, qnbigl, qnbigr, qntot, system)
-    Qs, Rs = Engine.get(coef.device).qr_blocks([f[4] for f in found])
-    return _qr_end(found, Qs, Rs, system), rows, cols
+    found, rows, cols, _ = _qr_begin(coef, qnbigl, qnbigr, qntot, system)
+    Qs, Rs = Engine.get(coef.device).qr_blocks([f.blk for f in found])
+    blocks = []
+    for f, Q, R in zip(found, Qs, Rs):
+        if system == "L":
+            blocks.append(QNBlock(f.nl, f.nr, f.rows, f.cols, Q, None, None, R))
+        else:
+            blocks.append(QNBlock(f.nl, f.nr, f.rows[::-1], f.cols[::-1],
+                                  R.mH.flip([0, 1]).resolve_conj().contiguous(), None, None,
+                                  Q.mH.flip([0, 1]).resolve_conj().contiguous()))
+    return blocks, rows, cols
 
 
-def _scatter(eng: Engine, src: torch.Tensor, rows, scols, dcols, sigma, dst: torch.Tensor, dst_rs, dst_cs):
-    """dst[rows[i]*dst_rs + dcols[j]*dst_cs] = sigma_j * src[i, scols[j]] (src: any 2-D view)"""
-    if len(rows) == 0 or len(scols) == 0:
-        return
-    # the kernel does not bound-check its index lists: check them here
-    r, c = np.asarray(rows, dtype=np.int64), np.asarray(scols, dtype=np.int64)
-    dc = np.asarray(dcols, dtype=np.int64)
+def _check_scatter(src, r, c, dc, dst, dst_rs, dst_cs):
+    """the scatter kernel does not bound-check its index lists: check them here"""
     if (len(r) > src.shape[0] or len(dc) != len(c) or c.min() < 0 or c.max() >= src.shape[1] or r.min() < 0
             or dc.min() < 0 or int(r.max()) * dst_rs + int(dc.max()) * dst_cs >= dst.numel()):
         raise IndexError(f"qn scatter out of range: src {tuple(src.shape)}, {len(r)} rows (max {r.max()}), "
                          f"source columns up to {c.max()}, dst {tuple(dst.shape)}")
-    dev = dst.device
-    if sigma is None:
-        ri, ci, di = _i64_many([r, c, dc], dev)
-        sig = None
-    else:
-        ri, ci, di, sig = _i64_many([r, c, dc, sigma], dev, float_last=True)
-    eng.qn_scatter(src, ri, ci, di, sig, dst, dst_rs, dst_cs)
+
+
+def _scatter_all(eng: Engine, jobs):
+    """dst[rows[i]*dst_rs + dcols[j]*dst_cs] = src[i, scols[j]] (src: any 2-D
+    view) for every job (src, rows, scols, dcols, dst, dst_rs, dst_cs), the
+    index lists of all of them in one transfer"""
+    jobs = [(s, np.asarray(r, dtype=np.int64), np.asarray(c, dtype=np.int64), np.asarray(dc, dtype=np.int64), *d)
+            for s, r, c, dc, *d in jobs if len(r) and len(c)]
+    for s, r, c, dc, *d in jobs:
+        _check_scatter(s, r, c, dc, *d)
+    if jobs:
+        dev = _i64_many([x for j in jobs for x in j[1:4]], jobs[0][4].device)
+        for i, (s, _, _, _, dst, rs, cs) in enumerate(jobs):
+            eng.qn_scatter(s, *dev[3 * i:3 * i + 3], None, dst, rs, cs)
 
 
 def _select_by_code(sset: np.ndarray, codes: np.ndarray, visit: List[int], Mmax: int, percent=0) -> List[int]:
@@ -692,13 +707,10 @@ def _trunc_begin(coef, qnbigl, qnbigr, qntot, keep_left, m_trunc_fn, percent=0, 
     rq = qnbigr.reshape(-1, qs)
     blocks = []
     pending = []
-    for nl in qn_sectors(lq):
-        nr = tuple(qntot - np.array(nl))
-        rset = np.where(get_qn_mask(rq, nr))[0]
-        if len(rset) == 0:
-            continue
-        lset = np.where(get_qn_mask(lq, nl))[0]
-        X = _gather(eng, mat, lset, rset)
+    found = _sectors(lq, rq, qntot)
+    lists = _i64_many([x for f in found for x in f[2:]], mat.device)
+    for i, (nl, nr, lset, rset) in enumerate(found):
+        X = _gather(eng, mat, lists[2 * i], lists[2 * i + 1])
         m, n = X.shape
         dim = min(m, n)
         upad, vpad = _pad_counts(m, n, full_matrices)
@@ -715,8 +727,6 @@ def _trunc_begin(coef, qnbigl, qnbigr, qntot, keep_left, m_trunc_fn, percent=0, 
         blk = dict(nl=nl, nr=nr, lset=lset, rset=rset, dim=dim, npad=npad, X=X, ktop=ktop)
         blocks.append(blk)
         pending.append(blk)
-    if not blocks:
-        raise ValueError("Invalid quantum number")
     return dict(eng=eng, coef=coef, rows=rows, cols=cols, keep_left=keep_left, m_trunc_fn=m_trunc_fn,
                 refine_floor=refine_floor,
                 percent=percent, blocks=blocks, pending=pending)
@@ -952,6 +962,7 @@ def _trunc_place(st, sel):
         per_block.setdefault(bi, ([], []))
         per_block[bi][0].append(j)
         per_block[bi][1].append(out_col)
+    jobs = []
     for bi, (kc, oc) in per_block.items():
         b = blocks[bi]
         if max(kc) >= b["K"].shape[1]:
@@ -959,19 +970,18 @@ def _trunc_place(st, sel):
             # svd_qn.py:52-63 from numpy's global RNG, built only when selected
             b["K"] = torch.cat([b["K"], _completion(b["K"], max(kc) + 1 - b["K"].shape[1])], dim=1)
         nz = [(j, o) for j, o in zip(kc, oc) if j < b["dim"]]
+        pj, po = [j for j, _ in nz], [o for _, o in nz]
         if keep_left:
             # left[lset[i], out] = K[i, j] (kept basis incl. completion columns)
-            _scatter(eng, b["K"], b["lset"], kc, oc, None, left, mdim, 1)
-            if nz:
-                # right[out, rset[i]] = P[j, i]  (= sigma_j Vh[j, i]); completion rows stay 0
-                _scatter(eng, b["P"].transpose(0, 1), b["rset"], [j for j, _ in nz], [o for _, o in nz], None, right,
-                         1, cols)
+            jobs.append((b["K"], b["lset"], kc, oc, left, mdim, 1))
+            # right[out, rset[i]] = P[j, i]  (= sigma_j Vh[j, i]); completion rows stay 0
+            jobs.append((b["P"].transpose(0, 1), b["rset"], pj, po, right, 1, cols))
         else:
             # right[out, rset[i]] = conj(K[i, j]) : the reference's v = Vt.T rows
-            _scatter(eng, b["K"].conj().resolve_conj() if b["K"].is_complex() else b["K"], b["rset"], kc, oc, None,
-                     right, 1, cols)
-            if nz:
-                _scatter(eng, b["P"], b["lset"], [j for j, _ in nz], [o for _, o in nz], None, left, mdim, 1)
+            K = b["K"].conj().resolve_conj() if b["K"].is_complex() else b["K"]
+            jobs.append((K, b["rset"], kc, oc, right, 1, cols))
+            jobs.append((b["P"], b["lset"], pj, po, left, mdim, 1))
+    _scatter_all(eng, jobs)
     qn_new = np.array([qkey[bi] for bi in blk[sidx].tolist()]).reshape(mdim, -1)
     return TruncatedSplit(left, right, qn_new, mdim, sig[sidx])
 
@@ -979,8 +989,7 @@ def _trunc_place(st, sel):
 def qr_split(coef: torch.Tensor, qnbigl, qnbigr, qntot, system: str):
     """svd_qn(QR=True, full_matrices=False) of mp.py:890-908 / mps.py:1318-1327:
     returns (u (rows, k), qnl list, vt (k, cols), qnr list) as device tensors."""
-    blocks, rows, cols = qn_block_qr(coef, qnbigl, qnbigr, qntot, system)
-    return _qr_assemble(blocks, rows, cols, coef)
+    return qr_split_batch([dict(coef=coef, qnbigl=qnbigl, qnbigr=qnbigr, qntot=qntot, system=system)])[0]
 
 
 def qr_split_batch(calls):
@@ -988,36 +997,41 @@ def qr_split_batch(calls):
     QN blocks of all of them in shared batched QR launches (lockstep
     realisations); every result is that call's own qr_split."""
     begun = [_qr_begin(**c) for c in calls]
-    mats = [f[4] for found, _, _ in begun for f in found]
+    mats = [f.blk for b in begun for f in b[0]]
     if not mats:
         return []
     Qs, Rs = Engine.get(mats[0].device).qr_blocks(mats)
     out, off = [], 0
-    for c, (found, rows, cols) in zip(calls, begun):
-        k = len(found)
-        blocks = _qr_end(found, Qs[off:off + k], Rs[off:off + k], c["system"])
+    for c, b in zip(calls, begun):
+        k = len(b[0])
+        out.append(_qr_assemble(*b, Qs[off:off + k], Rs[off:off + k], c["coef"], c["system"]))
         off += k
-        out.append(_qr_assemble(blocks, rows, cols, c["coef"]))
     return out
 
 
-def _qr_assemble(blocks, rows, cols, coef):
+def _qr_assemble(blocks, rows, cols, arange, Qs, Rs, coef, system):
+    """u (rows, k) and vt (k, cols) from the blocks' factors.  For RQ, with the
+    block's QR Q1 R1 (see _QrBlock), u = J R1^H J and vt = J Q1^H J: the
+    reversals are in the blocks' index lists, the conjugation is done here and
+    the transposition is the scatter's strides."""
     eng = Engine.get(coef.device)
-    ks = [min(len(b.lset), len(b.rset)) for b in blocks]
+    ks = [len(b.place) for b in blocks]
     ktot = sum(ks)
     u = torch.zeros((rows, ktot), dtype=coef.dtype, device=coef.device)
     vt = torch.zeros((ktot, cols), dtype=coef.dtype, device=coef.device)
     qnl, qnr = [], []
-    off = 0
-    for b, k in zip(blocks, ks):
-        cidx = list(range(k))
-        out = list(range(off, off + k))
-        _scatter(eng, b.U, b.lset, cidx, out, None, u, ktot, 1)
-        # vt rows: dst (row=off+j, col=rset[i]) <- Vh[j, i]
-        _scatter(eng, b.Vh.transpose(0, 1), b.rset, cidx, out, None, vt, 1, cols)
+    for b, k, Q, R in zip(blocks, ks, Qs, Rs):
+        U, V = Q, R.transpose(0, 1)
+        if system == "R":
+            if coef.is_complex():
+                Q, R = Q.conj_physical_(), R.conj_physical_()
+            U, V = R.transpose(0, 1), Q
+        sc = np.arange(k)
+        for src, r, r_d, dst, rs, cs in ((U, b.rows, b.rows_d, u, ktot, 1), (V, b.cols, b.cols_d, vt, 1, cols)):
+            _check_scatter(src, r, sc, b.place, dst, rs, cs)
+            eng.qn_scatter(src, r_d, arange[:k], b.place_d, None, dst, rs, cs)
         qnl += [b.nl] * k
         qnr += [b.nr] * k
-        off += k
     return u, qnl, vt, qnr
 
 
@@ -1037,11 +1051,11 @@ def svd_qn(coef_array, qnbigl, qnbigr, qntot, QR=False, system=None, full_matric
     v = torch.zeros((cols, sum(vcols)), dtype=coef.dtype, device=coef.device)
     su, sv, qnl, qnr = [], [], [], []
     off = 0
+    jobs = []
     for b in blocks:
         k = b.S.size
-        _scatter(eng, b.U, b.lset, list(range(k)), list(range(off, off + k)), None, u, u.shape[1], 1)
-        _scatter(eng, b.Vh.transpose(0, 1), b.rset, list(range(k)), list(range(off, off + k)), None, v,
-                 v.shape[1], 1)
+        jobs.append((b.U, b.lset, range(k), range(off, off + k), u, u.shape[1], 1))
+        jobs.append((b.Vh.transpose(0, 1), b.rset, range(k), range(off, off + k), v, v.shape[1], 1))
         su.append(b.S)
         sv.append(b.S)
         qnl += [b.nl] * k
@@ -1051,16 +1065,17 @@ def svd_qn(coef_array, qnbigl, qnbigr, qntot, QR=False, system=None, full_matric
     for b in blocks:
         if b.upad:
             pad = _completion(b.U, b.upad)
-            _scatter(eng, pad, b.lset, list(range(b.upad)), list(range(uo, uo + b.upad)), None, u, u.shape[1], 1)
+            jobs.append((pad, b.lset, range(b.upad), range(uo, uo + b.upad), u, u.shape[1], 1))
             uo += b.upad
         su.append(np.zeros(b.upad))
         qnl += [b.nl] * b.upad
         if b.vpad:
             pad = _completion(b.Vh.transpose(0, 1).contiguous(), b.vpad).contiguous()
-            _scatter(eng, pad, b.rset, list(range(b.vpad)), list(range(vo, vo + b.vpad)), None, v, v.shape[1], 1)
+            jobs.append((pad, b.rset, range(b.vpad), range(vo, vo + b.vpad), v, v.shape[1], 1))
             vo += b.vpad
         sv.append(np.zeros(b.vpad))
         qnr += [b.nr] * b.vpad
+    _scatter_all(eng, jobs)
     su = np.concatenate(su)
     sv = np.concatenate(sv)
     if not full_matrices:
