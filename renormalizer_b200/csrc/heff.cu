@@ -13,6 +13,7 @@
 //                                  mirrored chain)
 #include "reno_common.cuh"
 #include "gemm_fp64.cuh"
+#include "mpo_stage.cuh"
 #include "split_gemm.cuh"
 #include <algorithm>
 #include <memory>
@@ -130,7 +131,7 @@ struct Stage {
 };
 
 static cudaError_t run_stage(const Stage& s, void* split_ws, size_t split_ws_bytes, cudaStream_t st) {
-  if (s.prec == RENO_PREC_FP64) return gemm_fp64(s.p, st);
+  if (s.prec == RENO_PREC_FP64) return mpo_stage_applies(s.p) ? mpo_stage(s.p, st) : gemm_fp64(s.p, st);
   return split_gemm(s.p, s.prec, split_ws, split_ws_bytes, st);
 }
 
@@ -308,15 +309,7 @@ static cudaError_t fused2_run(const reno_heff_desc* d, const Fused2& f, const vo
   const bool c = ev == RENO_C128;
   const int64_t x2 = c ? 2 : 1;
   cudaError_t e = cudaSuccess;
-  if (!packed) {
-    e = split_pack(opnd(L, ev, ml, 1), (int)(ml * wl), (int)ml, 1, SplitRows{}, f.s1a, pr, st);
-    if (e == cudaSuccess)
-      e = split_pack(opnd(Wt1, RENO_F64, wl * d1, 1), (int)(d1 * wm), (int)(wl * d1), 1, SplitRows{}, f.s2a, pr, st);
-    if (e == cudaSuccess)
-      e = split_pack(opnd(Wt2, RENO_F64, wm * d2, 1), (int)(d2 * wr), (int)(wm * d2), 1, SplitRows{}, f.s3a, pr, st);
-    if (e == cudaSuccess)
-      e = split_pack(opnd(R, ev, wr * mr, 1), (int)mr, (int)(wr * mr), 1, SplitRows{}, f.s4b, pr, st);
-  }
+  if (!packed) e = split_pack(opnd(L, ev, ml, 1), (int)(ml * wl), (int)ml, 1, SplitRows{}, f.s1a, pr, st);
   // psi rows in (k, h, e) order: e at stride d2*mr, h at mr, k at 1; K = c at d1*d2*mr
   SplitRows khe;
   khe.D0 = (int)d1;
@@ -325,6 +318,15 @@ static cudaError_t fused2_run(const reno_heff_desc* d, const Fused2& f, const vo
   khe.s_r2 = 1;
   if (e == cudaSuccess)
     e = split_pack(opnd(psi, pv, d2 * mr, d1 * d2 * mr), (int)(d1 * d2 * mr), (int)ml, 1, khe, f.s1b, pr, st);
+  // the small constant operands after the large one, which they queue up behind
+  if (!packed) {
+    if (e == cudaSuccess)
+      e = split_pack(opnd(Wt1, RENO_F64, wl * d1, 1), (int)(d1 * wm), (int)(wl * d1), 1, SplitRows{}, f.s2a, pr, st);
+    if (e == cudaSuccess)
+      e = split_pack(opnd(Wt2, RENO_F64, wm * d2, 1), (int)(d2 * wr), (int)(wm * d2), 1, SplitRows{}, f.s3a, pr, st);
+    if (e == cudaSuccess)
+      e = split_pack(opnd(R, ev, wr * mr, 1), (int)mr, (int)(wr * mr), 1, SplitRows{}, f.s4b, pr, st);
+  }
   if (e != cudaSuccess) return e;
   // S1: rows (a, b) of L, columns (k, h, e) -> S2's B[a][(k, h) re/im][(b, e)]
   SplitPackOut o1{f.s2b.hi, f.s2b.lo, 0, f.s2b.rows * f.s2b.pitch, d1, x2 * f.s2b.pitch, 1, f.s2b.pitch,
@@ -406,13 +408,7 @@ static cudaError_t fused1_run(const reno_heff_desc* d, const Fused1& f, const vo
   const int ev = d->env_dtype, pv = d->psi_dtype, pr = d->prec;
   const int64_t x2 = ev == RENO_C128 ? 2 : 1;
   cudaError_t e = cudaSuccess;
-  if (!packed) {
-    e = split_pack(opnd(L, ev, ml, 1), (int)(ml * wl), (int)ml, 1, SplitRows{}, f.s1a, pr, st);
-    if (e == cudaSuccess)
-      e = split_pack(opnd(Wt, RENO_F64, wl * dd, 1), (int)(dd * wr), (int)(wl * dd), 1, SplitRows{}, f.s2a, pr, st);
-    if (e == cudaSuccess)
-      e = split_pack(opnd(R, ev, wr * mr, 1), (int)mr, (int)(wr * mr), 1, SplitRows{}, f.s3b, pr, st);
-  }
+  if (!packed) e = split_pack(opnd(L, ev, ml, 1), (int)(ml * wl), (int)ml, 1, SplitRows{}, f.s1a, pr, st);
   // psi rows in (k, e) order: e at stride mr, k at 1; K = c at dd*mr
   SplitRows ke;
   ke.D0 = (int)dd;
@@ -420,6 +416,12 @@ static cudaError_t fused1_run(const reno_heff_desc* d, const Fused1& f, const vo
   ke.s_r1 = 1;
   ke.s_r2 = 0;
   if (e == cudaSuccess) e = split_pack(opnd(psi, pv, mr, dd * mr), (int)(dd * mr), (int)ml, 1, ke, f.s1b, pr, st);
+  if (!packed) {
+    if (e == cudaSuccess)
+      e = split_pack(opnd(Wt, RENO_F64, wl * dd, 1), (int)(dd * wr), (int)(wl * dd), 1, SplitRows{}, f.s2a, pr, st);
+    if (e == cudaSuccess)
+      e = split_pack(opnd(R, ev, wr * mr, 1), (int)mr, (int)(wr * mr), 1, SplitRows{}, f.s3b, pr, st);
+  }
   if (e != cudaSuccess) return e;
   // S1: rows (a, b) of L, columns (k, e) -> S2's B[a][k re/im][(b, e)]
   SplitPackOut o1{f.s2b.hi, f.s2b.lo, 0, f.s2b.rows * f.s2b.pitch, dd, x2 * f.s2b.pitch, 1, f.s2b.pitch,
@@ -437,15 +439,13 @@ static cudaError_t fused1_run(const reno_heff_desc* d, const Fused1& f, const vo
   return e;
 }
 
-static size_t heff_needed(const reno_heff_desc* d) {
+static size_t heff_total(const reno_heff_desc* d) {
   const HeffLayout lay = heff_layout(d);
   if (fused2_eligible(d)) return lay.off_t1 + fused2_layout(d, nullptr).bytes;
   if (fused1_eligible(d)) return lay.off_t1 + fused1_layout(d, nullptr).bytes;
   char* nul = nullptr;
-  return lay.off_split + split_need(heff_stages(d, lay, nul, nullptr, nullptr, nullptr, nullptr));
+  return lay.off_split + align256(split_need(heff_stages(d, lay, nul, nullptr, nullptr, nullptr, nullptr)));
 }
-
-static size_t heff_total(const reno_heff_desc* d) { return align256(heff_needed(d)); }
 
 }  // namespace reno
 
@@ -469,9 +469,24 @@ int reno::heff_apply_prepared(reno_ctx* ctx, const reno_heff_desc* d, const void
     return set_error(ctx, RENO_ERR_INVALID, "reno_heff_apply: null tensor pointer");
   const HeffLayout lay = heff_layout(d);
   char* w = static_cast<char*>(ws);
-  if (!ws || ws_bytes < heff_needed(d))
-    return set_error(ctx, RENO_ERR_WORKSPACE, "reno_heff_apply: workspace too small");
   cudaStream_t st = ctx->stream;
+  const bool one = fused1_eligible(d), two = fused2_eligible(d);
+  Fused1 f1{};
+  Fused2 f2{};
+  std::vector<Stage> stages;
+  size_t need_split = 0, need;
+  if (one) {
+    f1 = fused1_layout(d, w ? w + lay.off_t1 : nullptr);
+    need = lay.off_t1 + f1.bytes;
+  } else if (two) {
+    f2 = fused2_layout(d, w ? w + lay.off_t1 : nullptr);
+    need = lay.off_t1 + f2.bytes;
+  } else {
+    stages = heff_stages(d, lay, w, L, R, psi, y);
+    need_split = split_need(stages);
+    need = lay.off_split + need_split;
+  }
+  if (!ws || ws_bytes < need) return set_error(ctx, RENO_ERR_WORKSPACE, "reno_heff_apply: workspace too small");
   cudaError_t e = cudaSuccess;
   if (!prepared) {
     if (d->nsite == 1) e = launch_wt(W1, w + lay.off_wt1, d->mpo_dtype, d->wl, d->d1, d->wr, 0, st);
@@ -479,18 +494,10 @@ int reno::heff_apply_prepared(reno_ctx* ctx, const reno_heff_desc* d, const void
       e = launch_wt(W1, w + lay.off_wt1, d->mpo_dtype, d->wl, d->d1, d->wm, 0, st);
       if (e == cudaSuccess) e = launch_wt(W2, w + lay.off_wt2, d->mpo_dtype, d->wm, d->d2, d->wr, 0, st);
     }
-    if (e != cudaSuccess) return check_cuda(ctx, e, "reno_heff_apply");
   }
-  if (fused1_eligible(d)) {
-    e = fused1_run(d, fused1_layout(d, w + lay.off_t1), L, w + lay.off_wt1, R, psi, y, prepared, st);
-    return check_cuda(ctx, e, "reno_heff_apply");
-  }
-  if (fused2_eligible(d)) {
-    e = fused2_run(d, fused2_layout(d, w + lay.off_t1), L, w + lay.off_wt1, w + lay.off_wt2, R, psi, y, prepared, st);
-    return check_cuda(ctx, e, "reno_heff_apply");
-  }
-  const std::vector<Stage> stages = heff_stages(d, lay, w, L, R, psi, y);
-  const size_t need_split = split_need(stages);
+  if (e == cudaSuccess && one) e = fused1_run(d, f1, L, w + lay.off_wt1, R, psi, y, prepared, st);
+  if (e == cudaSuccess && two)
+    e = fused2_run(d, f2, L, w + lay.off_wt1, w + lay.off_wt2, R, psi, y, prepared, st);
   for (const Stage& s : stages) {
     if (e != cudaSuccess) break;
     e = run_stage(s, w + lay.off_split, need_split, st);
@@ -616,8 +623,17 @@ extern "C" int reno_heff_apply_grouped(reno_ctx* ctx, int32_t count, const reno_
   }
   std::unique_ptr<fp64gemm::GemmGroup> g(new fp64gemm::GemmGroup());
   for (size_t s = 0; s < stages[0].size(); ++s) {
-    g->count = count;
-    for (int i = 0; i < count; ++i) g->p[i] = stages[i][s].p;
+    g->count = 0;
+    for (int i = 0; i < count; ++i) {
+      const GemmParams& q = stages[i][s].p;
+      if (!mpo_stage_applies(q)) {
+        g->p[g->count++] = q;
+        continue;
+      }
+      const int rc = check_cuda(ctx, mpo_stage(q, st), "reno_heff_apply_grouped: MPO stage");
+      if (rc != RENO_OK) return rc;
+    }
+    if (g->count == 0) continue;
     const int rc = check_cuda(ctx, gemm_fp64_grouped(*g, st), "reno_heff_apply_grouped: stage");
     if (rc != RENO_OK) return rc;
   }
