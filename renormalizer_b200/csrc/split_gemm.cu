@@ -30,8 +30,9 @@
 namespace reno {
 namespace split {
 
-constexpr int BM = 128, BN = 256, STAGES = 2, THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
-constexpr int EPI_WARPS = 8;
+constexpr int EPI_WARPS = 8;  // 16 do not gain: the stores are bound by the load/store unit, not by latency
+constexpr int BM = 128, BN = 256, STAGES = 2, THREADS = 32 * (2 + EPI_WARPS);  // warp 0 TMA, warp 1 MMA, then epilogue
+constexpr int EPI_COLS = BN * 4 / EPI_WARPS;  // columns of a tile per epilogue warp
 constexpr int KROW_BYTES = 128;  // one SW128 row of K per stage
 constexpr int A_TILE = BM * KROW_BYTES;   // 16 KB
 constexpr int B_TILE = BN * KROW_BYTES;   // 32 KB
@@ -104,47 +105,61 @@ __device__ __forceinline__ void split_store_bits(void* hi, void* lo, int64_t idx
   }
 }
 
+// one 32-byte store (p is 32-byte aligned)
+__device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+               "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+
+__device__ __forceinline__ void st_global_v4(void* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
 // 16 output values v[t*STRIDE + OFF] (t = 0..15) of one (m, ri) for columns
-// n0 .. n0+15 into the packed planes: one 32-byte (BF16) or 64-byte (TF32)
-// vector store per plane when the run is contiguous and aligned, scalar
-// stores otherwise
+// n0 .. n0+15 into the packed planes: 32-byte stores (whole sectors; 16-byte
+// ones took up to a fifth of a stage longer) when the run is contiguous and
+// aligned, scalar stores otherwise.  Lanes hold different rows, so a store
+// instruction costs a cycle of the load/store unit per lane whatever its width.
 template <int ESZ, int STRIDE, int OFF>
 __device__ __forceinline__ void pack_run(const float* v, const Epi& e, int64_t mbase, int n0, int ri) {
-  const int64_t rbase = mbase + (int64_t)ri * e.s_ri;
-  const int64_t idx0 = rbase + (int64_t)(n0 / e.Dn) * e.s_n1 + (int64_t)(n0 % e.Dn) * e.s_n0;
-  const bool vec = e.s_n0 == 1 && n0 + 16 <= e.N && (n0 % e.Dn) + 16 <= e.Dn && (idx0 % (16 / ESZ)) == 0;
+  if (n0 >= e.N) return;
+  const int nq = n0 / e.Dn;
+  int nr = n0 - nq * e.Dn;
+  const int64_t idx0 = mbase + (int64_t)ri * e.s_ri + (int64_t)nq * e.s_n1 + (int64_t)nr * e.s_n0;
+  const bool vec = e.s_n0 == 1 && n0 + 16 <= e.N && nr + 16 <= e.Dn && (idx0 % (32 / ESZ)) == 0;
   if (vec) {
     uint32_t hb[16], lb[16];
 #pragma unroll
     for (int t = 0; t < 16; ++t) split_bits<ESZ>(v[t * STRIDE + OFF], hb[t], lb[t]);
-    if constexpr (ESZ == 2) {
-      uint4* ph = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(e.phi) + idx0);
-      uint4* pl = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(e.plo) + idx0);
+    // whole 32-byte sectors per store
+    uint32_t w[4 * ESZ];  // 16 elements of one plane, 32 bits at a time
+    unsigned char* planes[2] = {reinterpret_cast<unsigned char*>(e.phi) + idx0 * ESZ,
+                                reinterpret_cast<unsigned char*>(e.plo) + idx0 * ESZ};
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        ph[q] = make_uint4(hb[8 * q] | (hb[8 * q + 1] << 16), hb[8 * q + 2] | (hb[8 * q + 3] << 16),
-                           hb[8 * q + 4] | (hb[8 * q + 5] << 16), hb[8 * q + 6] | (hb[8 * q + 7] << 16));
-        pl[q] = make_uint4(lb[8 * q] | (lb[8 * q + 1] << 16), lb[8 * q + 2] | (lb[8 * q + 3] << 16),
-                           lb[8 * q + 4] | (lb[8 * q + 5] << 16), lb[8 * q + 6] | (lb[8 * q + 7] << 16));
-      }
-    } else {
-      uint4* ph = reinterpret_cast<uint4*>(reinterpret_cast<uint32_t*>(e.phi) + idx0);
-      uint4* pl = reinterpret_cast<uint4*>(reinterpret_cast<uint32_t*>(e.plo) + idx0);
+    for (int pl = 0; pl < 2; ++pl) {
+      const uint32_t* src = pl == 0 ? hb : lb;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        ph[q] = make_uint4(hb[4 * q], hb[4 * q + 1], hb[4 * q + 2], hb[4 * q + 3]);
-        pl[q] = make_uint4(lb[4 * q], lb[4 * q + 1], lb[4 * q + 2], lb[4 * q + 3]);
-      }
+      for (int q = 0; q < 4 * ESZ; ++q) w[q] = ESZ == 2 ? src[2 * q] | (src[2 * q + 1] << 16) : src[q];
+#pragma unroll
+      for (int q = 0; q < ESZ / 2; ++q) st_global_v8(planes[pl] + 32 * q, w + 8 * q);
     }
   } else {
+    // the index moves along with n: with a division per element this branch took 220 cycles a value, and
+    // the third stage of an M = 192 two-site matvec 649 us (206 now)
+    const int64_t wrap = e.s_n1 - (int64_t)e.Dn * e.s_n0;
+    int64_t idx = idx0;
 #pragma unroll
     for (int t = 0; t < 16; ++t) {
-      const int n = n0 + t;
-      if (n < e.N) {
+      if (n0 + t < e.N) {
         uint32_t hb, lb;
         split_bits<ESZ>(v[t * STRIDE + OFF], hb, lb);
-        split_store_bits<ESZ>(e.phi, e.plo, rbase + (int64_t)(n / e.Dn) * e.s_n1 + (int64_t)(n % e.Dn) * e.s_n0,
-                              hb, lb);
+        split_store_bits<ESZ>(e.phi, e.plo, idx, hb, lb);
+        idx += e.s_n0;
+        if (++nr == e.Dn) {
+          nr = 0;
+          idx += wrap;
+        }
       }
     }
   }
@@ -290,6 +305,15 @@ __device__ __forceinline__ void epilogue_store(const Epi& epi, const float* v, i
     } else if (epi.mode == OUT_COLS_CPLX) {
       if (rp < epi.M) {
         const int64_t base = (int64_t)bz * epi.sCb + (int64_t)rp * epi.sCm;
+        const int64_t first = base + cp / 2;
+        if (epi.sCn == 1 && !epi.c_f32 && !epi.accumulate && cp / 2 + 16 <= epi.N &&
+            (reinterpret_cast<uintptr_t>(epi.C) + 16 * (uint64_t)first) % 32 == 0) {
+          // two complex numbers, one whole 32-byte sector, per store
+          double2* p = reinterpret_cast<double2*>(epi.C) + first;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) st_global_v4(p + 2 * j, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          return;
+        }
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int n = cp / 2 + j;
@@ -334,6 +358,7 @@ __device__ __forceinline__ void epilogue_store(const Epi& epi, const float* v, i
 template <int ESZ>
 __device__ __forceinline__ void epilogue_tile(const Epi& epi, uint32_t tacc, int q, int lane, int m_tile, int n_tile,
                                               int bz, int c_begin, int c_end) {
+  c_end = min(c_end, epi.cols_p - n_tile * BN);  // columns past the operand's last row hold nothing
   for (int c0 = c_begin; c0 < c_end; c0 += 32) {
     uint32_t r[32];
     const uint32_t taddr = tacc + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
@@ -524,12 +549,12 @@ __global__ void __launch_bounds__(THREADS, 1)
   } else if (warp >= 2) {
     // ---------------- epilogue
     const int q = warp % 4;                      // TMEM lane quarter this warp may access
-    const int c_begin = ((warp - 2) / 4) * (BN / 2);  // warps 2-5: columns [0, BN/2), warps 6-9: the rest
+    const int c_begin = ((warp - 2) / 4) * EPI_COLS;  // four warps (one per quarter) share a column range
     int i = 0;
     if constexpr (PROMOTE) {
       bool ok = true;
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        float acc[BN / 2];  // this thread's row, columns c_begin .. c_begin + BN/2 - 1
+        float acc[EPI_COLS];  // this thread's row, columns c_begin .. c_begin + EPI_COLS - 1
         for (int k0 = 0; k0 < num_k_tiles; k0 += kc, ++i) {
           const int b = i & 1;
           const uint32_t use = (uint32_t)(i >> 1);
@@ -540,7 +565,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           asm volatile("tcgen05.fence::after_thread_sync;");
           const uint32_t tacc = tmem + (uint32_t)(b * TMEM_COLS) + ((uint32_t)(q * 32) << 16) + (uint32_t)c_begin;
 #pragma unroll
-          for (int p = 0; p < BN / 64; ++p) {
+          for (int p = 0; p < EPI_COLS / 32; ++p) {
             uint32_t r[32];
             TMEM_LD32(tacc + (uint32_t)(32 * p), r);
             asm volatile("tcgen05.wait::ld.sync.aligned;");
@@ -556,7 +581,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         int m_tile, n_tile, bz;
         tile_coords(t, mt, nt, m_fast, m_tile, n_tile, bz);
 #pragma unroll
-        for (int p = 0; p < BN / 64; ++p) epilogue_store<ESZ>(epi, acc + 32 * p, q, lane, m_tile, n_tile, bz, c_begin + 32 * p);
+        for (int p = 0; p < EPI_COLS / 32; ++p) epilogue_store<ESZ>(epi, acc + 32 * p, q, lane, m_tile, n_tile, bz, c_begin + 32 * p);
       }
     } else {
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++i) {
@@ -568,7 +593,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       int m_tile, n_tile, bz;
       tile_coords(t, mt, nt, m_fast, m_tile, n_tile, bz);
       epilogue_tile<ESZ>(epi, tmem + (uint32_t)(b * TMEM_COLS), q, lane, m_tile, n_tile, bz, c_begin,
-                         c_begin + BN / 2);
+                         c_begin + EPI_COLS);
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[b]);
@@ -592,15 +617,18 @@ enum PackMode {
   P_DBL_SPLIT = 3   // out[2r][k] = re, out[2r+1][k] = im             K' = K,  2R rows
 };
 
+// Rows are packed in groups: row r = g + i * rstep, i = 0 .. ceil((R - g) / rstep) - 1,
+// sits at (g % D0) * s_g0 + (g / D0) * s_g1 + i * s_i.  A plain row stride is one
+// group; an operand whose rows run over several of the source's indices is
+// cut into groups along the index that is contiguous in the source.
 struct PackArgs {
   const void* src;
   int src_complex, conj, src_f32;
-  int64_t s_r, s_k, s_b;  // element strides of rows, K and batch
-  // row r = (r2 * D1 + r1) * D0 + r0 sits at r0*s_r + r1*s_r1 + r2*s_r2
-  // (a single-strided row index has D0 >= R)
-  int D0, D1;
-  int64_t s_r1, s_r2;
-  int R, K, nbatch, mode;
+  int64_t s_k, s_b;  // element strides of K and batch
+  int D0, rstep;
+  int64_t s_g0, s_g1, s_i;
+  int R, K;
+  int rtiles, ktiles;
   void* hi;
   void* lo;
   int64_t pitch;        // row pitch of the packed buffer (elements, 16-byte multiple)
@@ -626,78 +654,154 @@ __device__ __forceinline__ void split_store(void* hi, void* lo, int64_t idx, dou
   }
 }
 
-// one 32 x 32 (rows x K) source tile per block, staged through shared memory so
+// |x| is 0 or in a range in which x and x - BF16(x) (0, or at most 53 binary
+// orders below x) are both normal FP32 numbers or 0
+__device__ __forceinline__ bool float_range(double x) {
+  const uint32_t mag = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+  return mag - (960u << 20) < ((1150u - 960u) << 20) || (mag | (uint32_t)__double2loint(x)) == 0;
+}
+
+// x as FP32 rounded to odd (truncated, last bit set when that was inexact): a
+// later rounding to BF16 then gives what rounding x itself would.  For x in
+// FP32's normal range or 0, in integer operations: conversions from FP64 and
+// back kept the whole pack from running at the memory's rate.
+__device__ __forceinline__ float float_to_odd(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t mag = __funnelshift_l(lo, max(hi & 0x7fffffffu, 896u << 20) - (896u << 20), 3);
+  return __uint_as_float((hi & 0x80000000u) | mag | min(lo & 0x1fffffffu, 1u));
+}
+
+// elements idx and idx + 1 (n = 2; one when n = 1) of a packed row: one store
+// per plane when the pair is aligned.  FAST: both values are in float_range.
+template <int ESZ, bool FAST>
+__device__ __forceinline__ void split_store_pair(void* hi, void* lo, int64_t idx, double x0, double x1, int n) {
+  if (n == 2 && (idx & 1) == 0) {
+    if constexpr (FAST) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(float_to_odd(x0), float_to_odd(x1));
+      reinterpret_cast<__nv_bfloat162*>(hi)[idx >> 1] = h;
+      reinterpret_cast<__nv_bfloat162*>(lo)[idx >> 1] = __floats2bfloat162_rn(
+          float_to_odd(x0 - (double)__low2float(h)), float_to_odd(x1 - (double)__high2float(h)));
+      return;
+    }
+    if constexpr (ESZ == 4) {
+      float h[2], l[2];
+      split_store<ESZ>(h, l, 0, x0);
+      split_store<ESZ>(h, l, 1, x1);
+      reinterpret_cast<float2*>(hi)[idx >> 1] = make_float2(h[0], h[1]);
+      reinterpret_cast<float2*>(lo)[idx >> 1] = make_float2(l[0], l[1]);
+      return;
+    }
+  }
+  split_store<ESZ>(hi, lo, idx, x0);
+  if (n == 2) split_store<ESZ>(hi, lo, idx + 1, x1);
+}
+
+constexpr int PACK_R = 32, PACK_K = 64;
+
+// rows i0 + ty, i0 + ty + 8, ... of a staged tile -> the packed planes
+template <int ESZ, int MODE, bool FAST>
+__device__ __forceinline__ void pack_rows(const PackArgs& a, const double2 (*tile)[PACK_K + 1], int64_t base, int rows,
+                                          int64_t r, int k) {
+  const int n = min(a.K - k, 2), tx = threadIdx.x;
+  if (n <= 0) return;
+  constexpr bool DBL = MODE == P_DBL_CPLX || MODE == P_DBL_SPLIT;
+  int64_t at = base + (DBL ? 2 * r : r) * a.pitch + k;
+  const int64_t step = (DBL ? 16 : 8) * (int64_t)a.rstep * a.pitch;
+  for (int i = threadIdx.y; i < rows; i += 8, at += step) {
+    const double2 p = tile[i][2 * tx], q = tile[i][2 * tx + 1];
+    split_store_pair<ESZ, FAST>(a.hi, a.lo, at, p.x, q.x, n);
+    if constexpr (MODE == P_CAT) {
+      split_store_pair<ESZ, FAST>(a.hi, a.lo, at + a.K, p.y, q.y, n);
+    } else if constexpr (MODE == P_DBL_CPLX) {
+      split_store_pair<ESZ, FAST>(a.hi, a.lo, at + a.K, -p.y, -q.y, n);
+      split_store_pair<ESZ, FAST>(a.hi, a.lo, at + a.pitch, p.y, q.y, n);
+      split_store_pair<ESZ, FAST>(a.hi, a.lo, at + a.pitch + a.K, p.x, q.x, n);
+    } else if constexpr (MODE == P_DBL_SPLIT) {
+      split_store_pair<ESZ, FAST>(a.hi, a.lo, at + a.pitch, p.y, q.y, n);
+    }
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ double2 pack_value(T x, double) { return make_double2((double)x, 0.0); }
+__device__ __forceinline__ double2 pack_value(double2 x, double s) { return make_double2(x.x, s * x.y); }
+__device__ __forceinline__ double2 pack_value(float2 x, double s) { return make_double2(x.x, s * x.y); }
+
+// the 32 x 64 source tile into shared memory, eight loads of each thread in
+// flight at once; returns whether all of the thread's values are in float_range
+template <typename T>
+__device__ __forceinline__ bool pack_load(const PackArgs& a, double2 (*tile)[PACK_K + 1], int64_t src0, int rows,
+                                          int cols, bool k_fast) {
+  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
+  // value j sits (j >> 1) big and (j & 1) small steps from the thread's first
+  const int i0 = k_fast ? ty : tx, c0 = k_fast ? tx : ty;
+  const int di = k_fast ? 8 : 0, dc = k_fast ? 0 : 16, ec = k_fast ? 32 : 8;
+  const int64_t big = di * a.s_i + dc * a.s_k, small = ec * a.s_k;
+  const T* src = reinterpret_cast<const T*>(a.src) + src0 + (int64_t)i0 * a.s_i + (int64_t)c0 * a.s_k;
+  T v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    v[j] = T{};
+    if (i0 + (j >> 1) * di < rows && c0 + (j >> 1) * dc + (j & 1) * ec < cols) v[j] = src[(j >> 1) * big + (j & 1) * small];
+  }
+  const double sgn = a.conj ? -1.0 : 1.0;
+  double2* t = &tile[i0][c0];
+  const int tbig = di * (PACK_K + 1) + dc;
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const double2 x = pack_value(v[j], sgn);
+    ok = ok && float_range(x.x) && float_range(x.y);
+    t[(j >> 1) * tbig + (j & 1) * ec] = x;
+  }
+  return ok;
+}
+
+// One 32 x 64 (rows x K) source tile per block, staged through shared memory so
 // that both the strided reads (FP64, or FP32 intermediates) and the
 // K-contiguous packed writes coalesce.  Packed rows hold K' elements at a
 // 16-byte pitch; the tensor maps end at K', so the TMA loads zero-fill the
-// rest of the last 128-byte K tile and no padding is ever written.
-template <int ESZ>
-__global__ void pack_kernel(PackArgs a) {
-  __shared__ double2 tile[32][33];
+// rest of the last 128-byte K tile and no padding is ever written.  Each
+// thread has its eight loads in flight at once, and a warp writes 128 bytes of
+// a BF16 row.  Bound by instruction issue (2.8 a cycle; 52% of the memory's
+// rate): the psi operand of the M = 256 two-site matvec, 16.8 M complex
+// numbers, 403 MB moved, takes 87 us, 63 at the copy rate.  With rows read
+// across the source's contiguous index and every pair rounded by FP64
+// conversions it took 127 us.
+template <int ESZ, int MODE>
+__global__ void __launch_bounds__(256, 5) pack_kernel(PackArgs a) {
+  __shared__ double2 tile[PACK_R][PACK_K + 1];
   const int b = blockIdx.z;
-  const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-  const bool k_fast = (a.s_k == 1) || (a.s_r != 1);
-  for (int i = ty; i < 32; i += 8) {
-    const int r = k_fast ? r0 + i : r0 + tx;
-    const int k = k_fast ? k0 + tx : k0 + i;
-    double2 v = make_double2(0.0, 0.0);
-    if (r < a.R && k < a.K) {
-      const int r0 = r % a.D0, rq = r / a.D0;
-      const int64_t roff = (int64_t)r0 * a.s_r + (int64_t)(rq % a.D1) * a.s_r1 + (int64_t)(rq / a.D1) * a.s_r2;
-      const int64_t off = (int64_t)b * a.s_b + roff + (int64_t)k * a.s_k;
-      if (a.src_complex) {
-        if (a.src_f32) {
-          const float2 f = reinterpret_cast<const float2*>(a.src)[off];
-          v = make_double2(f.x, f.y);
-        } else {
-          v = reinterpret_cast<const double2*>(a.src)[off];
-        }
-        if (a.conj) v.y = -v.y;
-      } else {
-        v.x = a.src_f32 ? (double)reinterpret_cast<const float*>(a.src)[off] : reinterpret_cast<const double*>(a.src)[off];
-      }
-    }
-    if (k_fast)
-      tile[i][tx] = v;
-    else
-      tile[tx][i] = v;
-  }
-  __syncthreads();
+  // row tiles fastest: neighbouring blocks read on along the source's contiguous index
+  int x = blockIdx.x;
+  const int i0 = (x % a.rtiles) * PACK_R;
+  x /= a.rtiles;
+  const int g = x % a.rstep;
+  const int k0 = (x / a.rstep) * PACK_K;
+  const int rows = min(PACK_R, (a.R - g + a.rstep - 1) / a.rstep - i0);  // of this group, in this tile
+  const int64_t src0 = (int64_t)b * a.s_b + (int64_t)(g % a.D0) * a.s_g0 + (int64_t)(g / a.D0) * a.s_g1 +
+                       (int64_t)i0 * a.s_i + (int64_t)k0 * a.s_k;
+  const bool k_fast = (a.s_k == 1) || (a.s_i != 1);
+  const int cols = a.K - k0;
+  bool ok;
+  if (a.src_complex)
+    ok = a.src_f32 ? pack_load<float2>(a, tile, src0, rows, cols, k_fast)
+                   : pack_load<double2>(a, tile, src0, rows, cols, k_fast);
+  else
+    ok = a.src_f32 ? pack_load<float>(a, tile, src0, rows, cols, k_fast)
+                   : pack_load<double>(a, tile, src0, rows, cols, k_fast);
   const int64_t base = (int64_t)b * a.rows_out * a.pitch;
-  for (int i = ty; i < 32; i += 8) {
-    const int r = r0 + i, k = k0 + tx;
-    if (r >= a.R) continue;
-    const double2 v = tile[i][tx];
-    const bool kin = k < a.K;
-    switch (a.mode) {
-      case P_REAL:
-        if (kin) split_store<ESZ>(a.hi, a.lo, base + (int64_t)r * a.pitch + k, v.x);
-        break;
-      case P_CAT:
-        if (kin) {
-          split_store<ESZ>(a.hi, a.lo, base + (int64_t)r * a.pitch + k, v.x);
-          split_store<ESZ>(a.hi, a.lo, base + (int64_t)r * a.pitch + a.K + k, v.y);
-        }
-        break;
-      case P_DBL_CPLX:
-        if (kin) {
-          const int64_t r2 = base + (int64_t)(2 * r) * a.pitch;
-          split_store<ESZ>(a.hi, a.lo, r2 + k, v.x);
-          split_store<ESZ>(a.hi, a.lo, r2 + a.K + k, -v.y);
-          split_store<ESZ>(a.hi, a.lo, r2 + a.pitch + k, v.y);
-          split_store<ESZ>(a.hi, a.lo, r2 + a.pitch + a.K + k, v.x);
-        }
-        break;
-      default:  // P_DBL_SPLIT
-        if (kin) {
-          const int64_t r2 = base + (int64_t)(2 * r) * a.pitch;
-          split_store<ESZ>(a.hi, a.lo, r2 + k, v.x);
-          split_store<ESZ>(a.hi, a.lo, r2 + a.pitch + k, v.y);
-        }
-        break;
+  const int64_t r = (int64_t)g + (int64_t)(i0 + threadIdx.y) * a.rstep;
+  const int k = k0 + 2 * threadIdx.x;
+  if constexpr (ESZ == 2) {
+    if (__syncthreads_and(ok)) {
+      pack_rows<ESZ, MODE, true>(a, tile, base, rows, r, k);
+      return;
     }
+  } else {
+    __syncthreads();
   }
+  pack_rows<ESZ, MODE, false>(a, tile, base, rows, r, k);
 }
 
 // ------------------------------------------------------------------ host side
@@ -804,24 +908,33 @@ static cudaError_t run_pack(const GemmOperand& op, int R, int K, int nb, int mod
   a.src_complex = op.is_complex;
   a.conj = op.conj;
   a.src_f32 = op.is_f32;
-  a.s_r = op.s_outer;
   a.s_k = op.s_k;
   a.s_b = op.s_batch;
-  a.D0 = rs.D0 > 0 ? rs.D0 : std::max(R, 1);
-  a.D1 = rs.D0 > 0 ? std::max(rs.D1, 1) : 1;
-  a.s_r1 = rs.D0 > 0 ? rs.s_r1 : 0;
-  a.s_r2 = rs.D0 > 0 ? rs.s_r2 : 0;
+  // row r = (r2 * D1 + r1) * D0 + r0; tiles run along the slowest index that has more than one value
+  a.D0 = std::max(rs.D0, 1);
+  const bool levels = rs.D0 > 0, two = levels && (int64_t)rs.D0 * std::max(rs.D1, 1) >= R;
+  a.rstep = !levels ? 1 : two ? std::min(rs.D0, std::max(R, 1)) : rs.D0 * std::max(rs.D1, 1);
+  a.s_g0 = levels ? op.s_outer : 0;
+  a.s_g1 = levels && !two ? rs.s_r1 : 0;
+  a.s_i = !levels ? op.s_outer : two ? rs.s_r1 : rs.s_r2;
+  a.rtiles = (int)ceil_div(ceil_div(R, a.rstep), PACK_R);
+  a.ktiles = (int)ceil_div(K, PACK_K);
   a.R = R;
   a.K = K;
-  a.nbatch = nb;
-  a.mode = mode;
   a.hi = hi;
   a.lo = lo;
   a.pitch = pitch;
   a.rows_out = rows_out;
-  dim3 grid((unsigned)ceil_div(K, 32), (unsigned)ceil_div(R, 32), (unsigned)nb);
+  const int64_t blocks = (int64_t)a.ktiles * a.rtiles * a.rstep;
+  if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
+  dim3 grid((unsigned)blocks, 1, (unsigned)nb);
   count_launch();
-  pack_kernel<ESZ><<<grid, dim3(32, 8), 0, st>>>(a);
+  switch (mode) {
+    case P_REAL: pack_kernel<ESZ, P_REAL><<<grid, dim3(32, 8), 0, st>>>(a); break;
+    case P_CAT: pack_kernel<ESZ, P_CAT><<<grid, dim3(32, 8), 0, st>>>(a); break;
+    case P_DBL_CPLX: pack_kernel<ESZ, P_DBL_CPLX><<<grid, dim3(32, 8), 0, st>>>(a); break;
+    default: pack_kernel<ESZ, P_DBL_SPLIT><<<grid, dim3(32, 8), 0, st>>>(a); break;
+  }
   return cudaGetLastError();
 }
 
