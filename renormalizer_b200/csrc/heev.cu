@@ -14,11 +14,15 @@
 //                     column; each CTA recomputes v_k and w_k itself from
 //                     row k and y (bitwise identical in every CTA: same data,
 //                     same reduction order).  Reflector k is stored in row k.
+//                     Matrices that fit the shared memory of a cluster
+//                     (n <= 424) are reduced there (hetrd_cluster_kernel).
 //   2. bisect_kernel  eigenvalues of T by Sturm-count multisection, one warp
-//                     per eigenvalue, 32 points per round.
+//                     per eigenvalue, 32 points per round, signs of the leading
+//                     minors without a division.
 //   3. inviter_kernel eigenvectors of T by inverse iteration, one thread per
 //                     eigenvalue: LU of T - lambda I with partial pivoting,
-//                     three solves from a hashed start vector.  The host
+//                     three solves from a hashed start vector, in shared
+//                     memory (inviter_smem_kernel) but for the largest.  The host
 //                     orthonormalises the block (CholeskyQR2) and checks the
 //                     residuals ||T z - lambda z||.
 //   4. back-transformation K = Q Z in blocks of 64 reflectors (compact WY
@@ -770,160 +774,221 @@ __global__ void __launch_bounds__(HT, 1) hetrd_lower_kernel(const __grid_constan
 }
 
 // ---------------------------------------------------------------- small matrices
-// n <= 256: the same lagged one-barrier-per-column reduction on one
-// thread-block cluster of CL CTAs whose shared memories hold the matrix
-// (row r in CTA r % CL, slot r / CL).  Row k is read from its owner through
-// distributed shared memory, y_r and the partial dots are pushed to every CTA
-// (double-buffered by column parity, so a CTA that runs ahead never
-// overwrites a buffer another is still reading), and the hardware cluster
-// barrier, which every CTA executes the same number of times, separates the
-// columns.  Reflector k is written to row k of Aout (which may alias Gin: all
-// of Gin is read before the first barrier).  blockIdx.y = matrix.
-constexpr int CL = 8, CT = 256, CW = CT / 32, NMAX_C = 256, RL = NMAX_C / CL;
+// The same lagged reduction on one thread-block cluster of CL CTAs whose
+// shared memories hold the matrix (row r in CTA r % CL, slot r / CL): 8 CTAs up
+// to n = 256, 16 up to NMAX_C16 = 424 (27 rows beside the vectors fill the
+// shared memory) where the device can place such a cluster.  Thread c owns entry
+// c of v_k and w_k in every CTA and keeps it in registers.  Per column:
+//   1  row k (loaded from its owner through distributed shared memory while
+//      phase 3 of the column before still ran), update k-1 applied, the norm of
+//      its tail; a CTA barrier
+//   2  the owned rows: update k-1 and (row . unscaled reflector, entry k+1),
+//      pushed to every CTA (double-buffered by column parity, so a CTA that runs
+//      ahead never overwrites a buffer another is still reading); 3, 2 or 1 rows per warp at
+//      a time share the loads of w, v and the reflector.  The last warp computes
+//      tau, beta and the reflector's scale meanwhile.  Then the hardware
+//      cluster barrier, which every CTA executes the same number of times
+//   3  y_k and v_k scaled, y^H v (a CTA barrier), w_k
+// Bound by that chain of latencies (2 us a column at n = 32), with the rows' traffic in
+// shared memory beside it from n = 200 on: 59 / 269 / 734 us at n = 32 / 128 /
+// 256 on 8 CTAs (16 take 72 / 399 / 997), 957 at 300 on 16; with a barrier
+// for each of the scalars, the reflector and w_k, and one row per warp at a time,
+// n = 240 took 821 us (623 now), and the grid 2830 for n = 416.
+// Reflector k is written to row k of Aout (which may alias Gin: all of Gin is
+// read before the first barrier).  blockIdx.y = matrix.
+constexpr int CT = 512, CW = CT / 32, NMAX_C8 = 256, NMAX_C16 = 424;
 
-inline size_t cluster_smem_bytes(int n) {
-  return ((size_t)RL * n + 5 * (size_t)n + 2 * CL) * sizeof(double2);
+inline size_t cluster_smem_bytes(int n, int cl) {
+  return ((size_t)ceil_div(n, cl) * n + 7 * (size_t)n) * sizeof(double2);
 }
 
-__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
-    hetrd_cluster_kernel(const __grid_constant__ EigTable tab) {
+// update k-1 of the CTA's rows from slot s0 on and their sums with the
+// reflector, RB rows per warp at a time, by all warps but the last
+template <int CL, int RB>
+__device__ __forceinline__ void cluster_rows(cg::cluster_group& cluster, int rank, int n, int k, int s0, int act,
+                                             double2* rows, const double2* vp, const double2* wp, const double2* vc,
+                                             double2* ya, double2* yf) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int g = warp * RB; g < act; g += (CW - 1) * RB) {
+    double2* row[RB];
+    double2 vpr[RB], wpr[RB], acc[RB], first[RB];
+#pragma unroll
+    for (int u = 0; u < RB; ++u) {
+      const int sl = s0 + min(g + u, act - 1);  // past the end: the last row again, not written
+      row[u] = rows + (size_t)sl * n;
+      vpr[u] = vp[sl * CL + rank];
+      wpr[u] = wp[sl * CL + rank];
+      acc[u] = first[u] = make_double2(0.0, 0.0);
+    }
+    for (int c = k + 1 + lane; c < n; c += 32) {
+      const double2 w = wp[c], v = vp[c], q = vc[c];
+#pragma unroll
+      for (int u = 0; u < RB; ++u) {
+        const double2 x = csub(csub(row[u][c], cmulc(vpr[u], w)), cmulc(wpr[u], v));
+        if (g + u < act) row[u][c] = x;
+        if (c == k + 1) first[u] = x;  // the reflector is 1 there
+        else acc[u] = cadd(acc[u], cmul(x, q));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < RB; ++u) {
+      if (g + u >= act) break;
+      const int r = (s0 + g + u) * CL + rank;
+      const double2 f = make_double2(__shfl_sync(0xffffffffu, first[u].x, 0), __shfl_sync(0xffffffffu, first[u].y, 0));
+      const double2 y = warp_sum(acc[u]);
+      if (lane < CL) {
+        cluster.map_shared_rank(ya, lane)[r] = y;
+        cluster.map_shared_rank(yf, lane)[r] = f;
+      }
+    }
+  }
+}
+
+template <int CL>
+__global__ void __launch_bounds__(CT, 1) hetrd_cluster_kernel(const __grid_constant__ EigTable tab) {
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const EigProb& PR = tab.p[blockIdx.y];
-  const double2* __restrict__ Gin = PR.a;
+  const double2* Gin = PR.a;
   double2* Aout = PR.a;
   const int n = PR.n;
+  const int nslots = (n - rank + CL - 1) / CL;  // rows this CTA holds
   double* __restrict__ d = PR.d;
   double* __restrict__ e = PR.e;
   double2* __restrict__ tau = PR.tau;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* rows = reinterpret_cast<double2*>(smem_raw);  // RL x n
-  double2* vp = rows + (size_t)RL * n;
+  double2* vp = reinterpret_cast<double2*>(smem_raw);
   double2* wp = vp + n;
   double2* vc = wp + n;
-  double2* yb = vc + n;      // 2 x n
-  double2* pb = yb + 2 * n;  // 2 x CL
-  __shared__ double red[CW];
+  double2* yb = vc + n;        // 2 x (row . reflector, entry k+1) x n
+  double2* rows = yb + 4 * n;  // slots x n
+  __shared__ __align__(16) double red[CW];
   __shared__ double2 redc[CW];
-  __shared__ double2 s_scale, s_tau;
+  __shared__ double2 s_sc, s_tk;
   __shared__ double s_akk;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int sl = 0; sl < RL; ++sl) {
-    const int r = sl * CL + rank;
-    if (r < n)
-      for (int c = tid; c < n; c += CT) rows[(size_t)sl * n + c] = Gin[(size_t)r * n + c];
-  }
-  for (int i = tid; i < n; i += CT) {
-    vp[i] = make_double2(0.0, 0.0);
-    wp[i] = make_double2(0.0, 0.0);
-    vc[i] = make_double2(0.0, 0.0);
-  }
+  const int c = tid;  // n <= 424 < CT
+  for (int sl = 0; sl < nslots; ++sl)
+    if (c < n) rows[(size_t)sl * n + c] = Gin[(size_t)(sl * CL + rank) * n + c];
+  if (c < n) vp[c] = wp[c] = make_double2(0.0, 0.0);
   cluster.sync();
+  const double2 zero = make_double2(0.0, 0.0), one = make_double2(1.0, 0.0);
+  double2 v_c = zero, w_c = zero, vpk = zero, wpk = zero;  // entries c and k of v_{k-1}, w_{k-1}
+  double2 nx = c < n ? cluster.map_shared_rank(rows, 0)[c] : zero;  // row k
   for (int k = 0; k < n - 1; ++k) {
-    const int par = k & 1;
-    // ---- phase 1: row k from its owner, update k-1 applied, reflector k
-    const double2* rk = cluster.map_shared_rank(rows + (size_t)(k / CL) * n, k % CL);
-    const double2 vpk = vp[k], wpk = wp[k];
+    // ---- phase 1
     double ss = 0.0;
-    for (int c = k + tid; c < n; c += CT) {
-      const double2 x = csub(csub(rk[c], cmulc(vpk, wp[c])), cmulc(wpk, vp[c]));
+    double2 xc = zero;
+    if (c >= k && c < n) {
+      const double2 x = csub(csub(nx, cmulc(vpk, w_c)), cmulc(wpk, v_c));
       if (c == k) {
         s_akk = x.x;
       } else {
-        const double2 xc = conjg(x);
+        xc = conjg(x);
         vc[c] = xc;
-        if (c >= k + 2) ss += xc.x * xc.x + xc.y * xc.y;
+        if (c >= k + 2) ss = xc.x * xc.x + xc.y * xc.y;
       }
     }
-    ss = block_sum<CW>(ss, red);
-    if (tid == 0) {
+    ss = warp_sum(ss);
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();  // vc, red, and v_{k-1}, w_{k-1} of phase 3
+    // ---- phase 2
+    double2* ya = yb + (size_t)(k & 1) * 2 * n;
+    double2* yf = ya + n;
+    const int s0 = (k + CL - rank) / CL;  // the first owned row >= k + 1
+    const int act = nslots - s0;
+    if (warp == CW - 1) {
+      double2 part = zero;
+#pragma unroll
+      for (int i = 0; i < CW / 2; ++i) part = cadd(part, reinterpret_cast<const double2*>(red)[i]);
+      ss = part.x + part.y;
       const double2 alpha = vc[k + 1];
-      double beta;
-      if (ss == 0.0 && alpha.y == 0.0) {
-        s_tau = make_double2(0.0, 0.0);
-        s_scale = make_double2(0.0, 0.0);
-        beta = alpha.x;
-      } else {
+      double2 sc = zero, tk = zero;
+      double beta = alpha.x;
+      if (ss != 0.0 || alpha.y != 0.0) {
         beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + ss), alpha.x);
-        s_tau = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
+        tk = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
         const double2 den = make_double2(alpha.x - beta, alpha.y);
         const double m2 = den.x * den.x + den.y * den.y;
-        s_scale = make_double2(den.x / m2, -den.y / m2);
+        sc = make_double2(den.x / m2, -den.y / m2);
       }
-      if (rank == 0) {
-        d[k] = s_akk;
-        e[k] = beta;
-        tau[k] = s_tau;
+      if (lane == 0) {
+        s_sc = sc;
+        s_tk = tk;
+        if (rank == 0) {
+          d[k] = s_akk;
+          e[k] = beta;
+          tau[k] = tk;
+        }
       }
-    }
-    __syncthreads();
-    const double2 sc = s_scale, tk = s_tau;
-    for (int c = k + 1 + tid; c < n; c += CT) {
-      const double2 v = (c == k + 1) ? make_double2(1.0, 0.0) : cmul(vc[c], sc);
-      vc[c] = v;
-      if (rank == 0) Aout[(size_t)k * n + c] = v;
-    }
-    __syncthreads();
-    // ---- phase 2: owned rows r >= k+1: update k-1, y_r = row . v_k, pushed to every CTA
-    double2 pdot = make_double2(0.0, 0.0);
-    for (int sl = warp; sl < RL; sl += CW) {
-      const int r = sl * CL + rank;
-      if (r <= k || r >= n) continue;
-      double2* row = rows + (size_t)sl * n;
-      const double2 vpr = vp[r], wpr = wp[r];
-      double2 acc = make_double2(0.0, 0.0);
-      for (int c = k + 1 + lane; c < n; c += 32) {
-        const double2 x = csub(csub(row[c], cmulc(vpr, wp[c])), cmulc(wpr, vp[c]));
-        row[c] = x;
-        acc = cadd(acc, cmul(x, vc[c]));
-      }
-      acc = warp_sum(acc);
-      if (lane < CL) cluster.map_shared_rank(yb + (size_t)par * n, lane)[r] = acc;
-      if (lane == 0) pdot = cadd(pdot, cmulc(vc[r], acc));
-    }
-    if (lane == 0) redc[warp] = pdot;
-    __syncthreads();
-    if (tid < CL) {
-      double2 sum = make_double2(0.0, 0.0);
-      for (int w = 0; w < CW; ++w) sum = cadd(sum, redc[w]);
-      cluster.map_shared_rank(pb + par * CL, tid)[rank] = sum;
+    } else if (act > 2 * (CW - 1)) {
+      cluster_rows<CL, 3>(cluster, rank, n, k, s0, act, rows, vp, wp, vc, ya, yf);
+    } else if (act > CW - 1) {
+      cluster_rows<CL, 2>(cluster, rank, n, k, s0, act, rows, vp, wp, vc, ya, yf);
+    } else {
+      cluster_rows<CL, 1>(cluster, rank, n, k, s0, act, rows, vp, wp, vc, ya, yf);
     }
     cluster.sync();
     // ---- phase 3: w_k = tau y - (|tau|^2 / 2)(y^H v) v
-    double2 dot = make_double2(0.0, 0.0);
-    for (int q = 0; q < CL; ++q) dot = cadd(dot, pb[par * CL + q]);
+    double2 pdot = zero, y = zero;
+    const double2 sc = s_sc, tk = s_tk;
+    if (c > k && c < n) {
+      nx = cluster.map_shared_rank(rows + (size_t)((k + 1) / CL) * n, (k + 1) % CL)[c];
+      y = cadd(cmul(ya[c], sc), yf[c]);
+      v_c = c == k + 1 ? one : cmul(xc, sc);
+      pdot = cmulc(v_c, y);
+    }
+    const double2 yk1 = cadd(cmul(ya[k + 1], sc), yf[k + 1]);
+    pdot = warp_sum(pdot);
+    if (lane == 0) redc[warp] = pdot;
+    __syncthreads();
+    double2 dot = zero;
+#pragma unroll
+    for (int q = 0; q < CW; ++q) dot = cadd(dot, redc[q]);
     const double t2 = tk.x * tk.x + tk.y * tk.y;
     const double2 alph = make_double2(-0.5 * t2 * dot.x, -0.5 * t2 * dot.y);
-    for (int c = k + 1 + tid; c < n; c += CT) {
-      const double2 v = vc[c];
-      wp[c] = cadd(cmul(tk, yb[(size_t)par * n + c]), cmul(alph, v));
-      vp[c] = v;
+    if (c > k && c < n) {
+      w_c = cadd(cmul(tk, y), cmul(alph, v_c));
+      vp[c] = v_c;
+      wp[c] = w_c;
+      if (rank == 0) Aout[(size_t)k * n + c] = v_c;
     }
-    __syncthreads();
+    vpk = one;
+    wpk = cadd(cmul(tk, yk1), alph);
   }
-  if (rank == 0 && tid == 0) {
-    if (n == 1) {
-      d[0] = rows[0].x;
-    } else {
-      const double2* rn = cluster.map_shared_rank(rows + (size_t)((n - 1) / CL) * n, (n - 1) % CL);
-      const double2 a = csub(csub(rn[n - 1], cmulc(vp[n - 1], wp[n - 1])), cmulc(wp[n - 1], vp[n - 1]));
-      d[n - 1] = a.x;
-    }
-  }
+  if (rank == 0 && c == n - 1) d[n - 1] = csub(csub(nx, cmulc(v_c, w_c)), cmulc(w_c, v_c)).x;
   cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
 // ---------------------------------------------------------------- eigenvalues
-// Number of eigenvalues of T below x (LDL^T pivots, LAPACK dstebz's guard
-// |q| >= pivmin).
-__device__ __forceinline__ int sturm_count(const double* d, const double* e2, int n, double x, double pivmin) {
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int cnt = q < 0.0;
-  for (int i = 1; i < n; ++i) {
-    q = (d[i] - x) - e2[i - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    cnt += q < 0.0;
+// Sign changes of the leading principal minors p_i of T - x I = eigenvalues of T
+// below x (Givens 1953): p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}.  The recurrence
+// has one fused multiply-add on its chain, the pivot form q_i = d_i - x - e^2 / q
+// a division.  T comes scaled by a power of two to norm <= 1 and e^2 is at
+// least 2^-140 (eigenvalues move by 2^-69 of the norm at most), so that eight steps
+// change the larger of two neighbouring minors by at most 3^8 up or 2^-560
+// down: rescaled by 2^+-560 outside [2^-400, 2^400], it never leaves FP64's
+// range.  A minor that is exactly 0 counts once whatever its sign, as the one after
+// it has the opposite sign of the one before.
+constexpr int SCH = 8;  // steps between rescalings; the arrays are padded to a multiple
+__device__ __forceinline__ int sturm_count(const double2* t, int n, double x) {
+  double p0 = 1.0, p1 = t[0].x - x;  // t[i] = (d_i, e_{i-1}^2)
+  int cnt = __double2hiint(p1) < 0;
+  for (int i0 = 1; i0 < n; i0 += SCH) {
+    double2 c[SCH];
+#pragma unroll
+    for (int u = 0; u < SCH; ++u) c[u] = t[i0 + u];
+    const int m = max(__double2hiint(p0) & 0x7fffffff, __double2hiint(p1) & 0x7fffffff);
+    const double f = m < ((1023 - 400) << 20) ? 0x1p560 : m > ((1023 + 400) << 20) ? 0x1p-560 : 1.0;
+    p0 *= f;
+    p1 *= f;
+#pragma unroll
+    for (int u = 0; u < SCH; ++u) {
+      const double p2 = fma(c[u].x - x, p1, -c[u].y * p0);
+      if (i0 + u < n) cnt += (uint32_t)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
+      p0 = p1;
+      p1 = p2;
+    }
   }
   return cnt;
 }
@@ -972,32 +1037,52 @@ __global__ void __launch_bounds__(THREADS) bounds_kernel(const __grid_constant__
   }
 }
 
-// eigenvalue i0 + j (ascending) of T for j < cnt, one warp each
-__global__ void __launch_bounds__(THREADS) bisect_kernel(const __grid_constant__ EigTable tab) {
+// the binary exponent that brings the Gershgorin interval into [-1, 1]
+__device__ __forceinline__ int norm_exponent(const double* bnd) {
+  const double tn = fmax(fabs(bnd[0]), fabs(bnd[1]));
+  int ex = 0;
+  frexp(tn, &ex);
+  return tn > 0.0 && isfinite(tn) ? ex : 0;
+}
+
+// eigenvalue i0 + j (ascending) of T for j < cnt, one warp each: the bracket is
+// cut into 33 parts per round, down to 2 ulp or 2^-64 of the norm (the reduction
+// left an error of 2^-52 of it).  Bound by the latency of the minors' chain (one
+// warp per scheduler where the matrices are small): the top half of an n = 240
+// spectrum takes 36 us, 415 with a division on the chain.
+constexpr int BW = 4, BT = 32 * BW;
+__global__ void __launch_bounds__(BT) bisect_kernel(const __grid_constant__ EigTable tab) {
   const EigProb& PR = tab.p[blockIdx.y];
   const double* __restrict__ d = PR.d;
   const double* __restrict__ e = PR.e;
   const int n = PR.n, i0 = PR.n - PR.kt, cnt = PR.kt;
+  if (blockIdx.x * BW >= cnt) return;
   const double* __restrict__ bnd = PR.bnd;
   double* __restrict__ w = PR.w;
   extern __shared__ double sh[];
-  double* sd = sh;
-  double* se2 = sh + n;
-  for (int i = threadIdx.x; i < n; i += THREADS) {
-    sd[i] = d[i];
-    if (i < n - 1) se2[i] = e[i] * e[i];
+  double2* t = reinterpret_cast<double2*>(sh);
+  const int ex = norm_exponent(bnd);
+  for (int i = threadIdx.x; i < n + SCH; i += BT) {
+    double2 c = make_double2(0.0, 0.0);
+    if (i < n) {
+      c.x = ldexp(d[i], -ex);
+      if (i > 0) {
+        const double s = ldexp(e[i - 1], -ex);
+        c.y = fmax(s * s, 0x1p-140);
+      }
+    }
+    t[i] = c;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x * WARPS + (threadIdx.x >> 5);
+  const int j = blockIdx.x * BW + (threadIdx.x >> 5);
   if (j >= cnt) return;
   const int idx = i0 + j;
-  const double pivmin = bnd[2];
-  double lo = bnd[0], hi = bnd[1];
+  double lo = ldexp(bnd[0], -ex), hi = ldexp(bnd[1], -ex);
   for (int round = 0; round < 40; ++round) {
-    if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + pivmin) break;
+    if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + 0x1p-64) break;
     const double x = lo + (hi - lo) * ((double)(lane + 1) / 33.0);
-    const int c = sturm_count(sd, se2, n, x, pivmin);
+    const int c = sturm_count(t, n, x);
     // count(x) > idx  <=>  eigenvalue idx < x
     const unsigned above = __ballot_sync(0xffffffffu, c > idx);
     const int first = above ? __ffs(above) - 1 : 32;
@@ -1009,7 +1094,7 @@ __global__ void __launch_bounds__(THREADS) bisect_kernel(const __grid_constant__
     lo = nlo;
     hi = nhi;
   }
-  if (lane == 0) w[j] = 0.5 * (lo + hi);
+  if (lane == 0) w[j] = ldexp(0.5 * (lo + hi), ex);
 }
 
 // ---------------------------------------------------------------- eigenvectors
@@ -1023,11 +1108,123 @@ __device__ __forceinline__ double hash_unit(uint32_t a, uint32_t b) {
   return (double)h * (2.0 / 4294967296.0) - 1.0;
 }
 
-// column j of Z (n x cnt row-major) = eigenvector of T for w[j]; scratch:
+constexpr int IV_THREADS = 128, CH = 8, IV_WAVES = 4;
+
+// The same iteration with every array of a vector in shared memory, V vectors
+// (lanes) per warp-sized CTA: a pass over n rows then costs the chains of its
+// arithmetic, not trips to L2 (each row 0.3 us against 1.2).  Laid out [row][lane],
+// so the lanes never share a bank.  1 / |z| is applied by the next pass.
+// 95 us for the top half of n = 240 where the form below takes 240.
+constexpr int IV_SMEM = 227 * 1024;
+inline size_t inviter_smem_bytes(int n, int V) { return ((size_t)2 * n + 5 * (size_t)n * V) * sizeof(double); }
+
+__global__ void __launch_bounds__(32) inviter_smem_kernel(const __grid_constant__ EigTable tab, int V) {
+  const EigProb& PR = tab.p[blockIdx.y];
+  const double* __restrict__ d = PR.d;
+  const double* __restrict__ e = PR.e;
+  const int n = PR.n, cnt = PR.kt;
+  const int lane = threadIdx.x, j = blockIdx.x * V + lane;
+  if (blockIdx.x * V >= cnt) return;
+  extern __shared__ double sh_iv[];
+  double* sd = sh_iv;
+  double* se = sd + n;
+  const int ex = norm_exponent(PR.bnd);  // T and lambda scaled to norm <= 1: the vectors' squares stay finite
+  for (int i = lane; i < n; i += 32) {
+    sd[i] = ldexp(d[i], -ex);
+    se[i] = i < n - 1 ? ldexp(e[i], -ex) : 0.0;
+  }
+  __syncwarp();
+  if (lane >= V || j >= cnt) return;
+  const size_t step = (size_t)n * V;
+  double* ua = se + n + lane;  // 1 / u_kk
+  double* uc = ua + step;      // u_{k,k+1}
+  double* uc2 = uc + step;     // u_{k,k+2}
+  double* ml = uc2 + step;     // multiplier (+4 when rows k, k+1 were swapped)
+  double* z = ml + step;
+  const double lam = ldexp(PR.w[j], -ex);
+  const double tn = ldexp(fmax(fabs(PR.bnd[0]), fabs(PR.bnd[1])), -ex);
+  const double tiny = DBL_EPSILON * fmax(tn, DBL_MIN);
+  double ak = sd[0] - lam;
+  double ck = se[0];
+  for (int k = 0; k < n - 1; ++k) {
+    const double bk = se[k];
+    const double ak1 = sd[k + 1] - lam;
+    const double ck1 = se[k + 1];
+    const bool swap = fabs(ak) < fabs(bk);
+    // pivot row (p, p1, p2), the other row (q, q1, q2); a pivot below tiny becomes tiny
+    const double p1 = swap ? ak1 : ck, p2 = swap ? ck1 : 0.0;
+    const double q = swap ? ak : bk, q1 = swap ? ck : ak1, q2 = swap ? 0.0 : ck1;
+    double p = swap ? bk : ak;
+    if (fabs(p) < tiny) p = copysign(tiny, p);
+    const double inv = 1.0 / p, m = q * inv;
+    ua[k * V] = inv;
+    uc[k * V] = p1;
+    uc2[k * V] = p2;
+    ml[k * V] = swap ? m + 4.0 : m;
+    ak = q1 - m * p1;
+    ck = q2 - m * p2;
+  }
+  if (fabs(ak) < tiny) ak = copysign(tiny, ak);
+  ua[(n - 1) * V] = 1.0 / ak;
+  uc[(n - 1) * V] = 0.0;
+  uc2[(n - 1) * V] = 0.0;
+  for (int i = 0; i < n; ++i) z[i * V] = hash_unit((uint32_t)j + 1u, (uint32_t)i);
+  double inv = 1.0;
+  for (int it = 0; it < 3; ++it) {
+    // forward: L^-1 with the row swaps
+    double zk = z[0] * inv;
+    for (int k0 = 0; k0 < n - 1; k0 += CH) {
+      double mm[CH], zn[CH];
+#pragma unroll
+      for (int u = 0; u < CH; ++u) {
+        const int k = min(k0 + u, n - 2);
+        mm[u] = ml[k * V];
+        zn[u] = z[(k + 1) * V] * inv;
+      }
+#pragma unroll
+      for (int u = 0; u < CH; ++u) {
+        if (k0 + u < n - 1) {
+          const bool swap = mm[u] > 2.0;
+          const double m = swap ? mm[u] - 4.0 : mm[u];
+          z[(k0 + u) * V] = swap ? zn[u] : zk;
+          zk = swap ? zk - m * zn[u] : zn[u] - m * zk;
+        }
+      }
+    }
+    z[(n - 1) * V] = zk;
+    // backward: U with two super-diagonals
+    double z1 = 0.0, z2 = 0.0, nrm = 0.0;
+    for (int k0 = n - 1; k0 >= 0; k0 -= CH) {
+      double zz[CH], c1[CH], c2[CH], ia[CH];
+#pragma unroll
+      for (int u = 0; u < CH; ++u) {
+        const int k = max(k0 - u, 0);
+        zz[u] = z[k * V];
+        c1[u] = uc[k * V];
+        c2[u] = uc2[k * V];
+        ia[u] = ua[k * V];
+      }
+#pragma unroll
+      for (int u = 0; u < CH; ++u) {
+        if (k0 - u >= 0) {
+          const double v = (zz[u] - c2[u] * z2 - c1[u] * z1) * ia[u];
+          z[(k0 - u) * V] = v;
+          z2 = z1;
+          z1 = v;
+          nrm += v * v;
+        }
+      }
+    }
+    inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
+  }
+  for (int i = 0; i < n; ++i) PR.z[(size_t)i * cnt + j] = z[i * V] * inv;
+}
+
+// column j of Z (n x cnt row-major) = eigenvector of T for w[j], for tables whose
+// vectors would take more than IV_WAVES turns of the shared-memory form; scratch:
 // 4 * n * cnt doubles laid out [i * cnt + j] (coalesced across threads).
 // d, e are staged in shared memory; every sequential loop loads the next CH
 // steps' independent inputs before running their dependent chain.
-constexpr int IV_THREADS = 128, CH = 8;
 __global__ void __launch_bounds__(IV_THREADS) inviter_kernel(const __grid_constant__ EigTable tab) {
   const EigProb& PR = tab.p[blockIdx.y];
   const double* __restrict__ d = PR.d;
@@ -1040,9 +1237,10 @@ __global__ void __launch_bounds__(IV_THREADS) inviter_kernel(const __grid_consta
   extern __shared__ double sh_de[];
   double* sd = sh_de;
   double* se = sh_de + n;
+  const int ex = norm_exponent(bnd);
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    sd[i] = d[i];
-    se[i] = i < n - 1 ? e[i] : 0.0;
+    sd[i] = ldexp(d[i], -ex);
+    se[i] = i < n - 1 ? ldexp(e[i], -ex) : 0.0;
   }
   __syncthreads();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1052,8 +1250,8 @@ __global__ void __launch_bounds__(IV_THREADS) inviter_kernel(const __grid_consta
   double* uc = scr + 1 * (size_t)n * S;   // u_{k,k+1}
   double* uc2 = scr + 2 * (size_t)n * S;  // u_{k,k+2}
   double* ml = scr + 3 * (size_t)n * S;   // multiplier (+4 when rows k, k+1 were swapped)
-  const double lam = w[j];
-  const double tn = fmax(fabs(bnd[0]), fabs(bnd[1]));
+  const double lam = ldexp(w[j], -ex);
+  const double tn = ldexp(fmax(fabs(bnd[0]), fabs(bnd[1])), -ex);
   const double tiny = DBL_EPSILON * fmax(tn, DBL_MIN);
   // LU of T - lam I with partial pivoting.  The current row k has entries
   // (ak, ck) at columns (k, k+1); the next original row is (bk, ak1, ck1) at
@@ -1172,30 +1370,66 @@ __global__ void clean_v_kernel(double2* __restrict__ A, int n) {
   else if (c == k + 1) A[idx] = make_double2(1.0, 0.0);
 }
 
-// minus the NB x NB upper-triangular T of block b from S = V^H V and tau.
-// Thread i owns row i (written and read only by itself).
-__global__ void __launch_bounds__(NB) larft_kernel(const double2* __restrict__ Sg, const double2* __restrict__ tau,
-                                                   double2* __restrict__ Tg, int n) {
-  __shared__ double2 x[NB];
-  const int b = blockIdx.x, i = threadIdx.x;
-  const int k0 = b * NB, kb = min(NB, n - 1 - k0);
-  const double2* S = Sg + (size_t)b * NB * NB;
-  double2* T = Tg + ((size_t)b * NB + i) * NB;
-  for (int c = 0; c < NB; ++c) T[c] = make_double2(0.0, 0.0);
-  for (int j = 0; j < kb; ++j) {
-    const double2 tj = tau[k0 + j];
-    if (i < j) x[i] = cmul(make_double2(-tj.x, -tj.y), S[(size_t)i * NB + j]);
-    __syncthreads();
-    if (i < j) {
+// minus the NB x NB upper-triangular T of block b from S = V^H V and tau, by
+// doubling: two neighbouring factors T1, T2 of h reflectors join into
+// [[T1, -T1 S12 T2], [0, T2]], for h = 1, 2, .. NB / 2, all pairs of a level at once in
+// shared memory.  12 barriers in the place of the 128 of a column-by-column form,
+// whose row sums also ran one after the other.  22 us a call; the
+// column form took 105 per matrix.
+constexpr int LT = 256;
+constexpr int LARFT_SMEM = (2 * NB * NB + NB * NB / 4) * (int)sizeof(double2);
+struct LarftProb {
+  const double2* S;
+  const double2* tau;
+  double2* T;
+  int n, first;  // first block of the grid
+};
+struct LarftTable {
+  int count = 0, blocks = 0;
+  LarftProb p[MAXM];
+  void add(const double2* S, const double2* tau, double2* T, int n) {
+    p[count++] = LarftProb{S, tau, T, n, blocks};
+    blocks += (int)ceil_div(n - 1, NB);
+  }
+};
+__global__ void __launch_bounds__(LT) larft_kernel(const __grid_constant__ LarftTable tab) {
+  int pi = 0;
+  while (pi + 1 < tab.count && (int)blockIdx.x >= tab.p[pi + 1].first) ++pi;
+  const double2* __restrict__ Sg = tab.p[pi].S;
+  const double2* __restrict__ tau = tab.p[pi].tau;
+  double2* __restrict__ Tg = tab.p[pi].T;
+  const int n = tab.p[pi].n;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* S = reinterpret_cast<double2*>(smem_raw);
+  double2* T = S + NB * NB;
+  double2* W = T + NB * NB;  // S12 T2 of every pair of a level: 32 h <= NB^2 / 4 entries
+  const int b = blockIdx.x - tab.p[pi].first, k0 = b * NB, kb = min(NB, n - 1 - k0);
+  for (int i = threadIdx.x; i < NB * NB; i += LT) {
+    const int r = i / NB, c = i % NB;
+    S[i] = Sg[(size_t)b * NB * NB + i];
+    T[i] = r == c && r < kb ? tau[k0 + r] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  for (int h = 1; h < NB; h *= 2) {
+    const int total = NB / 2 * h;
+    for (int i = threadIdx.x; i < total; i += LT) {
+      const int c = i % h, r = i / h % h, o = i / (h * h) * 2 * h;
       double2 acc = make_double2(0.0, 0.0);
-      for (int l = i; l < j; ++l) acc = cadd(acc, cmul(T[l], x[l]));
-      T[j] = acc;
-    } else if (i == j) {
-      T[j] = tj;
+#pragma unroll 4
+      for (int l = 0; l <= c; ++l) acc = cadd(acc, cmul(S[(o + r) * NB + o + h + l], T[(o + h + l) * NB + o + h + c]));
+      W[i] = acc;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < total; i += LT) {
+      const int c = i % h, r = i / h % h, o = i / (h * h) * 2 * h, w0 = i / (h * h) * h * h + c;
+      double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 4
+      for (int l = r; l < h; ++l) acc = cadd(acc, cmul(T[(o + r) * NB + o + l], W[w0 + l * h]));
+      T[(o + r) * NB + o + h + c] = make_double2(-acc.x, -acc.y);
     }
     __syncthreads();
   }
-  for (int c = 0; c < NB; ++c) T[c] = make_double2(-T[c].x, -T[c].y);
+  for (int i = threadIdx.x; i < NB * NB; i += LT) Tg[(size_t)b * NB * NB + i] = make_double2(-T[i].x, -T[i].y);
 }
 
 }  // namespace heev
@@ -1221,7 +1455,7 @@ HeevLayout heev_layout(int n, int kt) {
   L.p = off;
   off += align256(2 * 1024 * sizeof(double2));
   L.yp = off;  // partial sums of the lower-triangle reduction (grid path only)
-  off += n > NMAX_C ? align256((size_t)YP_G * n * sizeof(double2)) : 0;
+  off += n > NMAX_C8 ? align256((size_t)YP_G * n * sizeof(double2)) : 0;
   L.bnd = off;
   off += align256(4 * sizeof(double));
   L.scr = off;
@@ -1249,7 +1483,7 @@ GemmOperand op(const void* p, int64_t s_outer, int64_t s_k, int conj) {
 }
 }  // namespace
 
-// Cooperative launch of the reduction over the matrices of tab (n > NMAX_C):
+// Cooperative launch of the reduction over the matrices of tab (too large for a cluster):
 // one CTA per SM, the SMs shared out in proportion to each matrix's n^2.  When
 // the largest matrix has at least LOWER_MIN_N rows the lower-triangle kernel
 // runs (each matrix then needs enough CTAs that its rows' (row, chunk)
@@ -1324,26 +1558,90 @@ extern "C" int reno_heev_workspace_bytes(int32_t n, int32_t kt, size_t* bytes) {
 namespace {
 
 int heev_attrs(reno_ctx* ctx) {
-  static std::atomic<unsigned long long> bisect_set{0}, inviter_set{0}, cluster_set{0};
-  int rc = check_cuda(ctx, smem_optin_once(bisect_kernel, 2 * MAX_N * (int)sizeof(double), bisect_set),
-                      "reno_heev_top: bisect smem attribute");
-  if (rc == RENO_OK)
-    rc = check_cuda(ctx, smem_optin_once(inviter_kernel, 2 * MAX_N * (int)sizeof(double), inviter_set),
-                    "reno_heev_top: inverse iteration smem attribute");
-  if (rc == RENO_OK)
-    rc = check_cuda(ctx, smem_optin_once(hetrd_cluster_kernel, (int)cluster_smem_bytes(NMAX_C), cluster_set),
-                    "reno_heev_top: cluster smem attribute");
-  return rc;
+  static std::atomic<unsigned long long> bisect_set{0}, inviter_set{0}, iv_smem_set{0}, larft_set{0}, c8_set{0},
+      c16_set{0}, wide_set{0};
+  const char* what = "reno_heev_top: shared memory attributes";
+  cudaError_t rc = smem_optin_once(bisect_kernel, 2 * (MAX_N + SCH) * (int)sizeof(double), bisect_set);
+  if (rc == cudaSuccess) rc = smem_optin_once(inviter_kernel, 2 * MAX_N * (int)sizeof(double), inviter_set);
+  if (rc == cudaSuccess) rc = smem_optin_once(inviter_smem_kernel, IV_SMEM, iv_smem_set);
+  if (rc == cudaSuccess) rc = smem_optin_once(larft_kernel, LARFT_SMEM, larft_set);
+  if (rc == cudaSuccess) rc = smem_optin_once(hetrd_cluster_kernel<8>, (int)cluster_smem_bytes(NMAX_C8, 8), c8_set);
+  if (rc == cudaSuccess) rc = smem_optin_once(hetrd_cluster_kernel<16>, (int)cluster_smem_bytes(NMAX_C16, 16), c16_set);
+  if (rc == cudaSuccess) {
+    int dev = 0;
+    rc = cudaGetDevice(&dev);
+    const unsigned long long bit = (dev >= 0 && dev < 64) ? (1ull << dev) : 0ull;
+    if (rc == cudaSuccess && !(bit && (wide_set.load(std::memory_order_acquire) & bit))) {
+      rc = cudaFuncSetAttribute(hetrd_cluster_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (rc == cudaSuccess && bit) wide_set.fetch_or(bit, std::memory_order_release);
+    }
+  }
+  return check_cuda(ctx, rc, what);
 }
 
-// tridiagonal reduction of small matrices (n <= NMAX_C): one thread-block
-// cluster per matrix, all in one launch
-int heev_reduce_small(reno_ctx* ctx, const EigTable& tab, int nmax) {
-  if (tab.count == 0) return RENO_OK;
+int launch_larft(reno_ctx* ctx, const LarftTable& tab) {
+  const int rc = heev_attrs(ctx);
+  if (rc != RENO_OK) return rc;
   count_launch();
-  hetrd_cluster_kernel<<<dim3(CL, tab.count), CT, cluster_smem_bytes(nmax), ctx->stream>>>(tab);
-  RENO_LAUNCH_CHECK(ctx, "reno_heev_top: cluster hetrd");
+  larft_kernel<<<tab.blocks, LT, LARFT_SMEM, ctx->stream>>>(tab);
+  RENO_LAUNCH_CHECK(ctx, "reno_heev_backtransform: larft");
   return RENO_OK;
+}
+
+cudaLaunchConfig_t cluster_config(int cl, int count, int n, cudaStream_t st, cudaLaunchAttribute* at) {
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)cl;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cl, (unsigned)count);
+  cfg.blockDim = dim3(CT);
+  cfg.dynamicSmemBytes = cluster_smem_bytes(n, cl);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// 16-CTA clusters of the largest matrix that the current device can hold at
+// once (read once per device; 0 where it has no room for even one)
+int wide_clusters() {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int c = known[dev].load(std::memory_order_acquire);
+  if (c == 0) {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = cluster_config(16, 1, NMAX_C16, nullptr, &at);
+    int num = 0;
+    if (cudaOccupancyMaxActiveClusters(&num, hetrd_cluster_kernel<16>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      num = 0;
+    }
+    c = num + 1;
+    known[dev].store(c, std::memory_order_release);
+  }
+  return c - 1;
+}
+
+// tridiagonal reduction of matrices that fit a cluster: one cluster per
+// matrix, all of one cluster size in one launch
+int heev_reduce_small(reno_ctx* ctx, const EigTable& tab, int cl) {
+  if (tab.count == 0) return RENO_OK;
+  int nmax = 1;
+  for (int i = 0; i < tab.count; ++i) nmax = std::max(nmax, tab.p[i].n);
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = cluster_config(cl, tab.count, nmax, ctx->stream, &at);
+  count_launch();
+  return check_cuda(ctx,
+                    cl == 16 ? cudaLaunchKernelEx(&cfg, hetrd_cluster_kernel<16>, tab)
+                             : cudaLaunchKernelEx(&cfg, hetrd_cluster_kernel<8>, tab),
+                    "reno_heev_top: cluster hetrd");
+}
+
+// CTAs of the cluster that reduces an n x n matrix (0: the grid does)
+int cluster_of(int n) {
+  if (n <= NMAX_C8) return 8;
+  return n <= NMAX_C16 && wide_clusters() > 0 ? 16 : 0;
 }
 
 // eigenvalues n-kt .. n-1 of every T (ascending) and their inverse-iteration
@@ -1360,12 +1658,18 @@ int heev_eig(reno_ctx* ctx, const EigTable& tab) {
   bounds_kernel<<<dim3(1, tab.count), THREADS, 0, st>>>(tab);
   RENO_LAUNCH_CHECK(ctx, "reno_heev_top: bounds");
   count_launch();
-  bisect_kernel<<<dim3((unsigned)ceil_div(ktmax, WARPS), tab.count), THREADS, 2 * (size_t)nmax * sizeof(double),
+  bisect_kernel<<<dim3((unsigned)ceil_div(ktmax, BW), tab.count), BT, 2 * (size_t)(nmax + SCH) * sizeof(double),
                   st>>>(tab);
   RENO_LAUNCH_CHECK(ctx, "reno_heev_top: bisect");
+  // a turn of the shared-memory form is worth four of the other's (0.3 against 1.2 us a row)
+  const int V = (int)std::min<size_t>(32, (IV_SMEM / sizeof(double) - 2 * (size_t)nmax) / (5 * (size_t)nmax));
+  const int64_t ctas = ceil_div(ktmax, std::max(V, 1)) * (int64_t)tab.count;
   count_launch();
-  inviter_kernel<<<dim3((unsigned)ceil_div(ktmax, IV_THREADS), tab.count), IV_THREADS,
-                   2 * (size_t)nmax * sizeof(double), st>>>(tab);
+  if (V >= 1 && ctas <= (int64_t)IV_WAVES * sm_count_current_device())
+    inviter_smem_kernel<<<dim3((unsigned)ceil_div(ktmax, V), tab.count), 32, inviter_smem_bytes(nmax, V), st>>>(tab, V);
+  else
+    inviter_kernel<<<dim3((unsigned)ceil_div(ktmax, IV_THREADS), tab.count), IV_THREADS,
+                     2 * (size_t)nmax * sizeof(double), st>>>(tab);
   RENO_LAUNCH_CHECK(ctx, "reno_heev_top: inverse iteration");
   return RENO_OK;
 }
@@ -1404,8 +1708,8 @@ extern "C" int reno_heev_top(reno_ctx* ctx, int32_t n, int32_t kt, void* A, doub
   EigTable et{};
   et.count = 1;
   et.p[0] = EigProb{static_cast<double2*>(A), static_cast<double2*>(tau), d, e, n, kt, w, Z, bnd, scr};
-  if (n <= NMAX_C) {
-    rc = heev_reduce_small(ctx, et, n);
+  if (const int cl = cluster_of(n)) {
+    rc = heev_reduce_small(ctx, et, cl);
   } else {
     HetrdTable tab{};
     tab.count = 1;
@@ -1442,8 +1746,8 @@ extern "C" int reno_heev_top_batched(reno_ctx* ctx, int32_t count, const reno_he
   int rc = heev_attrs(ctx);
   if (rc != RENO_OK) return rc;
   HetrdTable tab{};
-  EigTable small{}, all{};
-  int nmax = 0, nsmall = 1;
+  EigTable small{}, wide{}, all{};
+  int nmax = 0;
   for (int i = 0; i < count; ++i) {
     const reno_heev_problem& p = probs[i];
     char* base = static_cast<char*>(ws) + batched_offset(count, probs, i);
@@ -1454,9 +1758,9 @@ extern "C" int reno_heev_top_batched(reno_ctx* ctx, int32_t count, const reno_he
     const EigProb ep{static_cast<double2*>(p.a), static_cast<double2*>(p.tau), p.d, p.e, p.n, p.kt, p.w, p.z,
                      reinterpret_cast<double*>(base + L.bnd), reinterpret_cast<double*>(base + L.scr)};
     all.p[all.count++] = ep;
-    if (p.n <= NMAX_C) {
-      small.p[small.count++] = ep;
-      nsmall = std::max(nsmall, (int)p.n);
+    if (const int cl = cluster_of(p.n)) {
+      EigTable& t = cl == 8 ? small : wide;
+      t.p[t.count++] = ep;
     } else {
       tab.p[tab.count++] = HetrdProb{static_cast<double2*>(p.a), p.n, p.d, p.e, static_cast<double2*>(p.tau),
                                      reinterpret_cast<double2*>(base + L.y), reinterpret_cast<double2*>(base + L.p),
@@ -1464,7 +1768,8 @@ extern "C" int reno_heev_top_batched(reno_ctx* ctx, int32_t count, const reno_he
       nmax = std::max(nmax, (int)p.n);
     }
   }
-  rc = heev_reduce_small(ctx, small, nsmall);
+  rc = heev_reduce_small(ctx, small, 8);
+  if (rc == RENO_OK) rc = heev_reduce_small(ctx, wide, 16);
   if (rc != RENO_OK) return rc;
   if (tab.count) {
     rc = launch_hetrd(ctx, tab, nmax, "reno_heev_top_batched");
@@ -1543,9 +1848,10 @@ extern "C" int reno_heev_backtransform(reno_ctx* ctx, int32_t n, int32_t kt, voi
     rc = check_cuda(ctx, gemm_fp64(p, st), "reno_heev_backtransform: gram (last block)");
     if (rc != RENO_OK) return rc;
   }
-  count_launch();
-  larft_kernel<<<nblk, NB, 0, st>>>(Sg, static_cast<const double2*>(tau), Tg, n);
-  RENO_LAUNCH_CHECK(ctx, "reno_heev_backtransform: larft");
+  LarftTable lt;
+  lt.add(Sg, static_cast<const double2*>(tau), Tg, n);
+  rc = launch_larft(ctx, lt);
+  if (rc != RENO_OK) return rc;
   for (int b = nblk - 1; b >= 0; --b) {
     const int k0 = b * NB, kb = std::min(NB, n - 1 - k0);
     const int rows = n - k0 - 1;
@@ -1682,12 +1988,12 @@ extern "C" int reno_heev_backtransform_batched(reno_ctx* ctx, int32_t count, con
   }
   if ((rc = flush(g1, "reno_heev_backtransform_batched: gram")) != RENO_OK) return rc;
   int bmax = 0;
+  LarftTable lt;
   for (const One& o : P) {
-    count_launch();
-    larft_kernel<<<o.nblk, NB, 0, st>>>(o.Sg, o.tau, o.Tg, o.n);
-    RENO_LAUNCH_CHECK(ctx, "reno_heev_backtransform_batched: larft");
+    lt.add(o.Sg, o.tau, o.Tg, o.n);
     bmax = std::max(bmax, o.nblk);
   }
+  if ((rc = launch_larft(ctx, lt)) != RENO_OK) return rc;
   // blocks of reflectors from the last: every problem with block b advances together
   for (int b = bmax - 1; b >= 0; --b) {
     for (const One& o : P) {
