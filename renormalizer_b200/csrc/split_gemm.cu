@@ -11,7 +11,11 @@
 //
 // Pipeline (persistent: one CTA per SM walks 128 x 256 output tiles; 10 warps):
 //   warp 0     TMA producer: 4 tiles per stage (A_hi, A_lo, B_hi, B_lo),
-//              128-byte swizzled K-major boxes, mbarrier complete_tx
+//              64-byte swizzled K-major boxes, mbarrier complete_tx.  Four
+//              48 KB stages: two of 96 KB refill one while the other computes,
+//              which at 64 bytes a clock leaves no time for the latency (M = 256
+//              two-site matvec 1604 -> 1576 us, its last stage 360 -> 322; the
+//              first stays near the L2's rate, 401 us)
 //   warp 1     TMEM allocator + single-thread tcgen05.mma issuer: 3 products
 //              per stage, tcgen05.commit frees the stage
 //   warps 2-9  epilogue (two warps per TMEM lane quarter, half the columns
@@ -31,11 +35,11 @@ namespace reno {
 namespace split {
 
 constexpr int EPI_WARPS = 8;  // 16 do not gain: the stores are bound by the load/store unit, not by latency
-constexpr int BM = 128, BN = 256, STAGES = 2, THREADS = 32 * (2 + EPI_WARPS);  // warp 0 TMA, warp 1 MMA, then epilogue
+constexpr int BM = 128, BN = 256, STAGES = 4, THREADS = 32 * (2 + EPI_WARPS);  // warp 0 TMA, warp 1 MMA, then epilogue
 constexpr int EPI_COLS = BN * 4 / EPI_WARPS;  // columns of a tile per epilogue warp
-constexpr int KROW_BYTES = 128;  // one SW128 row of K per stage
-constexpr int A_TILE = BM * KROW_BYTES;   // 16 KB
-constexpr int B_TILE = BN * KROW_BYTES;   // 32 KB
+constexpr int KROW_BYTES = 64;  // one SW64 row of K per stage
+constexpr int A_TILE = BM * KROW_BYTES;   // 8 KB
+constexpr int B_TILE = BN * KROW_BYTES;   // 16 KB
 constexpr int STAGE_BYTES = 2 * A_TILE + 2 * B_TILE;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 constexpr uint32_t TMEM_COLS = 256;  // one accumulator buffer (two are allocated)
@@ -220,14 +224,14 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* tm, ui
       : "memory");
 }
 
-// K-major, 128-byte swizzle shared-memory matrix descriptor (SBO = 8 rows x 128 B)
+// K-major, 64-byte swizzle shared-memory matrix descriptor (SBO = 8 rows x 64 B)
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
   d |= (uint64_t)1u << 16;            // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024u >> 4) << 32;  // stride byte offset
+  d |= (uint64_t)(512u >> 4) << 32;   // stride byte offset
   d |= (uint64_t)1u << 46;            // descriptor version for sm_100
-  d |= (uint64_t)2u << 61;            // SWIZZLE_128B
+  d |= (uint64_t)4u << 61;            // SWIZZLE_64B
   return d;
 }
 
@@ -525,11 +529,11 @@ __global__ void __launch_bounds__(THREADS, 1)
         const uint64_t dah = sdesc(base), dal = sdesc(base + A_TILE);
         const uint64_t dbh = sdesc(base + 2 * A_TILE), dbl = sdesc(base + 2 * A_TILE + B_TILE);
         // K beyond k_elems is TMA zero fill: skip the sub-steps that only see it
-        constexpr int SUB = (KROW_BYTES / ESZ) / 4;  // elements per 32-byte instruction step
+        constexpr int STEPS = KROW_BYTES / 32, SUB = 32 / ESZ;  // 32-byte instruction steps, elements of one
         const int rem = k_elems - kt * (KROW_BYTES / ESZ);
-        const int nsub = rem >= 4 * SUB ? 4 : (rem + SUB - 1) / SUB;
+        const int nsub = rem >= STEPS * SUB ? STEPS : (rem + SUB - 1) / SUB;
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
+        for (int kk = 0; kk < STEPS; ++kk) {
           if (kk < nsub) {
             const uint64_t adv = (uint64_t)((kk * 32) >> 4);  // 32 bytes of K per instruction
             const uint32_t first = (kt == k0 && kk == 0) ? 0u : 1u;
@@ -761,7 +765,7 @@ __device__ __forceinline__ bool pack_load(const PackArgs& a, double2 (*tile)[PAC
 // that both the strided reads (FP64, or FP32 intermediates) and the
 // K-contiguous packed writes coalesce.  Packed rows hold K' elements at a
 // 16-byte pitch; the tensor maps end at K', so the TMA loads zero-fill the
-// rest of the last 128-byte K tile and no padding is ever written.  Each
+// rest of the last K tile and no padding is ever written.  Each
 // thread has its eight loads in flight at once, and a warp writes 128 bytes of
 // a BF16 row.  Bound by instruction issue (2.8 a cycle; 52% of the memory's
 // rate): the psi operand of the M = 256 two-site matvec, 16.8 M complex
@@ -834,13 +838,13 @@ static bool make_map(CUtensorMap* tm, void* base, int esz, int64_t kext, int64_t
   cuuint32_t box[3] = {(cuuint32_t)(KROW_BYTES / esz), (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(tm, esz == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims,
-                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 
 struct Plan {
-  int esz, kstep;        // element size, elements per 128-byte K row
+  int esz, kstep;        // element size, elements per K row of a stage
   int modeA, modeB, out;
   int64_t KA;            // logical K' (after re/im concatenation)
   int64_t pitch;         // packed row pitch: K' rounded up to 16 bytes
@@ -986,7 +990,7 @@ static cudaError_t launch_split(const SplitPacked& A, const SplitPacked& B, int 
   }
   const int64_t kstep = KROW_BYTES / ESZ;
   const int chunk_k = g_split_chunk_k.load(std::memory_order_relaxed);
-  const int kc = chunk_k > 0 ? (int)std::max<int64_t>(1, chunk_k / kstep) : 0;
+  const int kc = chunk_k > 0 ? (int)std::max<int64_t>(1, chunk_k / (2 * kstep)) * 2 : 0;  // whole 128-byte rows
   static std::atomic<unsigned long long> smem_set{0}, smem_set_p{0};
   {
     cudaError_t e = kc > 0 ? smem_optin_once(split_gemm_kernel<ESZ, true>, SMEM_BYTES, smem_set_p)
