@@ -159,7 +159,7 @@ class LowRankOptions:
     below 0.7 of the extrapolation the block is not tried.
 
     Truncation of a complex 4096 x 4096 coefficient with two 2048^2 blocks
-    to 256: 54 -> 16 ms with sigma falling 3.5 decades over the kept ones,
+    to 256: 54 -> 15 ms with sigma falling 3.5 decades over the kept ones,
     27 ms with 1.5 decades; a flat spectrum pays 0.5 ms for the probe."""
 
     def __init__(self, min_ratio=2.5, oversample=96, probe=32, tol=2e-14):
