@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(HT, 1) hetrd_lower_kernel(const __grid_constan
 // ---------------------------------------------------------------- small matrices
 // The same lagged reduction on one thread-block cluster of CL CTAs whose
 // shared memories hold the matrix (row r in CTA r % CL, slot r / CL): 8 CTAs up
-// to n = 256, 16 up to NMAX_C16 = 424 (27 rows beside the vectors fill the
+// to n = 256 (one each for many small matrices, see cluster_of), 16 up to NMAX_C16 = 424 (27 rows beside the vectors fill the
 // shared memory) where the device can place such a cluster.  Thread c owns entry
 // c of v_k and w_k in every CTA and keeps it in registers.  Per column:
 //   1  row k (loaded from its owner through distributed shared memory while
@@ -790,13 +790,14 @@ __global__ void __launch_bounds__(HT, 1) hetrd_lower_kernel(const __grid_constan
 //      cluster barrier, which every CTA executes the same number of times
 //   3  y_k and v_k scaled, y^H v (a CTA barrier), w_k
 // Bound by that chain of latencies (2 us a column at n = 32), with the rows' traffic in
-// shared memory beside it from n = 200 on: 59 / 269 / 734 us at n = 32 / 128 /
-// 256 on 8 CTAs (16 take 72 / 399 / 997), 957 at 300 on 16; with a barrier
+// shared memory beside it from n = 200 on: 58 / 274 / 727 us at n = 32 / 128 /
+// 256 on 8 CTAs, 942 / 1703 at 300 / 424 on 16 (which a first form found slower than
+// 8 up to 256: 997 against 916); with a barrier
 // for each of the scalars, the reflector and w_k, and one row per warp at a time,
 // n = 240 took 821 us (623 now), and the grid 2830 for n = 416.
 // Reflector k is written to row k of Aout (which may alias Gin: all of Gin is
 // read before the first barrier).  blockIdx.y = matrix.
-constexpr int CT = 512, CW = CT / 32, NMAX_C8 = 256, NMAX_C16 = 424;
+constexpr int CT = 512, CW = CT / 32, NMAX_C1 = 64, NMAX_C8 = 256, NMAX_C16 = 424;
 
 inline size_t cluster_smem_bytes(int n, int cl) {
   return ((size_t)ceil_div(n, cl) * n + 7 * (size_t)n) * sizeof(double2);
@@ -842,6 +843,19 @@ __device__ __forceinline__ void cluster_rows(cg::cluster_group& cluster, int ran
       }
     }
   }
+}
+
+// sum of CW values in shared memory, pairwise: four dependent additions
+template <typename T, int N>
+__device__ __forceinline__ T tree_sum(const T* x) {
+  T t[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) t[i] = x[i];
+#pragma unroll
+  for (int h = N / 2; h > 0; h /= 2)
+#pragma unroll
+    for (int i = 0; i < h; ++i) t[i] = cadd(t[i], t[i + h]);
+  return t[0];
 }
 
 template <int CL>
@@ -898,19 +912,19 @@ __global__ void __launch_bounds__(CT, 1) hetrd_cluster_kernel(const __grid_const
     const int s0 = (k + CL - rank) / CL;  // the first owned row >= k + 1
     const int act = nslots - s0;
     if (warp == CW - 1) {
-      double2 part = zero;
-#pragma unroll
-      for (int i = 0; i < CW / 2; ++i) part = cadd(part, reinterpret_cast<const double2*>(red)[i]);
+      const double2 part = tree_sum<double2, CW / 2>(reinterpret_cast<const double2*>(red));
       ss = part.x + part.y;
       const double2 alpha = vc[k + 1];
       double2 sc = zero, tk = zero;
       double beta = alpha.x;
       if (ss != 0.0 || alpha.y != 0.0) {
         beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + ss), alpha.x);
-        tk = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
         const double2 den = make_double2(alpha.x - beta, alpha.y);
-        const double m2 = den.x * den.x + den.y * den.y;
-        sc = make_double2(den.x / m2, -den.y / m2);
+        // one division for both: even lanes take 1 / beta, odd ones 1 / |alpha - beta|^2
+        const double r = 1.0 / ((lane & 1) ? den.x * den.x + den.y * den.y : beta);
+        const double rb = __shfl_sync(0xffffffffu, r, 0), rm = __shfl_sync(0xffffffffu, r, 1);
+        tk = make_double2((beta - alpha.x) * rb, -alpha.y * rb);
+        sc = make_double2(den.x * rm, -den.y * rm);
       }
       if (lane == 0) {
         s_sc = sc;
@@ -942,9 +956,7 @@ __global__ void __launch_bounds__(CT, 1) hetrd_cluster_kernel(const __grid_const
     pdot = warp_sum(pdot);
     if (lane == 0) redc[warp] = pdot;
     __syncthreads();
-    double2 dot = zero;
-#pragma unroll
-    for (int q = 0; q < CW; ++q) dot = cadd(dot, redc[q]);
+    const double2 dot = tree_sum<double2, CW>(redc);
     const double t2 = tk.x * tk.x + tk.y * tk.y;
     const double2 alph = make_double2(-0.5 * t2 * dot.x, -0.5 * t2 * dot.y);
     if (c > k && c < n) {
@@ -1559,12 +1571,13 @@ namespace {
 
 int heev_attrs(reno_ctx* ctx) {
   static std::atomic<unsigned long long> bisect_set{0}, inviter_set{0}, iv_smem_set{0}, larft_set{0}, c8_set{0},
-      c16_set{0}, wide_set{0};
+      c16_set{0}, c1_set{0}, wide_set{0};
   const char* what = "reno_heev_top: shared memory attributes";
   cudaError_t rc = smem_optin_once(bisect_kernel, 2 * (MAX_N + SCH) * (int)sizeof(double), bisect_set);
   if (rc == cudaSuccess) rc = smem_optin_once(inviter_kernel, 2 * MAX_N * (int)sizeof(double), inviter_set);
   if (rc == cudaSuccess) rc = smem_optin_once(inviter_smem_kernel, IV_SMEM, iv_smem_set);
   if (rc == cudaSuccess) rc = smem_optin_once(larft_kernel, LARFT_SMEM, larft_set);
+  if (rc == cudaSuccess) rc = smem_optin_once(hetrd_cluster_kernel<1>, (int)cluster_smem_bytes(NMAX_C1, 1), c1_set);
   if (rc == cudaSuccess) rc = smem_optin_once(hetrd_cluster_kernel<8>, (int)cluster_smem_bytes(NMAX_C8, 8), c8_set);
   if (rc == cudaSuccess) rc = smem_optin_once(hetrd_cluster_kernel<16>, (int)cluster_smem_bytes(NMAX_C16, 16), c16_set);
   if (rc == cudaSuccess) {
@@ -1633,13 +1646,20 @@ int heev_reduce_small(reno_ctx* ctx, const EigTable& tab, int cl) {
   const cudaLaunchConfig_t cfg = cluster_config(cl, tab.count, nmax, ctx->stream, &at);
   count_launch();
   return check_cuda(ctx,
-                    cl == 16 ? cudaLaunchKernelEx(&cfg, hetrd_cluster_kernel<16>, tab)
-                             : cudaLaunchKernelEx(&cfg, hetrd_cluster_kernel<8>, tab),
+                    cl == 16  ? cudaLaunchKernelEx(&cfg, hetrd_cluster_kernel<16>, tab)
+                    : cl == 8 ? cudaLaunchKernelEx(&cfg, hetrd_cluster_kernel<8>, tab)
+                              : cudaLaunchKernelEx(&cfg, hetrd_cluster_kernel<1>, tab),
                     "reno_heev_top: cluster hetrd");
 }
 
-// CTAs of the cluster that reduces an n x n matrix (0: the grid does)
-int cluster_of(int n) {
+// CTAs of the cluster that reduces an n x n matrix (0: the grid does), for a
+// call with `tiny` matrices of at most NMAX_C1 rows.  One matrix is done soonest by
+// 8 CTAs (120 us at n = 64, 180 on one); more matrices than 8-CTA clusters fit the GPU
+// at once go to single CTAs (24 of n = 64: 180 us against 265, 32 of n = 32: 68
+// against 179).  Every sum has the same order on any number of CTAs, so the
+// choice does not show in the results.
+int cluster_of(int n, int tiny) {
+  if (n <= NMAX_C1 && tiny > 16) return 1;
   if (n <= NMAX_C8) return 8;
   return n <= NMAX_C16 && wide_clusters() > 0 ? 16 : 0;
 }
@@ -1708,7 +1728,7 @@ extern "C" int reno_heev_top(reno_ctx* ctx, int32_t n, int32_t kt, void* A, doub
   EigTable et{};
   et.count = 1;
   et.p[0] = EigProb{static_cast<double2*>(A), static_cast<double2*>(tau), d, e, n, kt, w, Z, bnd, scr};
-  if (const int cl = cluster_of(n)) {
+  if (const int cl = cluster_of(n, 1)) {
     rc = heev_reduce_small(ctx, et, cl);
   } else {
     HetrdTable tab{};
@@ -1746,7 +1766,9 @@ extern "C" int reno_heev_top_batched(reno_ctx* ctx, int32_t count, const reno_he
   int rc = heev_attrs(ctx);
   if (rc != RENO_OK) return rc;
   HetrdTable tab{};
-  EigTable small{}, wide{}, all{};
+  EigTable single{}, small{}, wide{}, all{};
+  int tiny = 0;
+  for (int i = 0; i < count; ++i) tiny += probs[i].n <= NMAX_C1;
   int nmax = 0;
   for (int i = 0; i < count; ++i) {
     const reno_heev_problem& p = probs[i];
@@ -1758,8 +1780,8 @@ extern "C" int reno_heev_top_batched(reno_ctx* ctx, int32_t count, const reno_he
     const EigProb ep{static_cast<double2*>(p.a), static_cast<double2*>(p.tau), p.d, p.e, p.n, p.kt, p.w, p.z,
                      reinterpret_cast<double*>(base + L.bnd), reinterpret_cast<double*>(base + L.scr)};
     all.p[all.count++] = ep;
-    if (const int cl = cluster_of(p.n)) {
-      EigTable& t = cl == 8 ? small : wide;
+    if (const int cl = cluster_of(p.n, tiny)) {
+      EigTable& t = cl == 1 ? single : cl == 8 ? small : wide;
       t.p[t.count++] = ep;
     } else {
       tab.p[tab.count++] = HetrdProb{static_cast<double2*>(p.a), p.n, p.d, p.e, static_cast<double2*>(p.tau),
@@ -1768,7 +1790,8 @@ extern "C" int reno_heev_top_batched(reno_ctx* ctx, int32_t count, const reno_he
       nmax = std::max(nmax, (int)p.n);
     }
   }
-  rc = heev_reduce_small(ctx, small, 8);
+  rc = heev_reduce_small(ctx, single, 1);
+  if (rc == RENO_OK) rc = heev_reduce_small(ctx, small, 8);
   if (rc == RENO_OK) rc = heev_reduce_small(ctx, wide, 16);
   if (rc != RENO_OK) return rc;
   if (tab.count) {

@@ -93,3 +93,18 @@ def test_batch_of_all_reductions():
     kts = [max(1, n // 5) for n in ns]
     for G, kt, (w, K, chk) in zip(Gs, kts, heev_top_batched(eng, Gs, kts)):
         _check(G, kt, w, K, chk)
+
+
+def test_many_small_matrices_equal_single_calls():
+    """more small matrices than 8-CTA clusters fit: one CTA each, bit for bit the
+    results of single calls (a larger one among them stays on its cluster)"""
+    from renormalizer_b200._native import Engine
+    from renormalizer_b200.heev import heev_top, heev_top_batched
+    rng = np.random.default_rng(11)
+    ns, eng = [1, 2, 5, 8, 13, 16, 17, 30, 31, 32, 33, 40, 48, 50, 60, 63, 64, 64, 65, 3], Engine.get(0)
+    Gs = [_gram(n, rng, "generic") for n in ns]
+    kts = [max(1, n // 2) for n in ns]
+    for G, kt, (w, K, chk) in zip(Gs, kts, heev_top_batched(eng, Gs, kts)):
+        _check(G, kt, w, K, chk)
+        w1, _, _ = heev_top(eng, G, kt)
+        assert torch.equal(w, w1)
