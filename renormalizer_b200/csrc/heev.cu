@@ -776,18 +776,20 @@ __global__ void __launch_bounds__(HT, 1) hetrd_lower_kernel(const __grid_constan
 // ---------------------------------------------------------------- small matrices
 // The same lagged reduction on one thread-block cluster of CL CTAs whose
 // shared memories hold the matrix (row r in CTA r % CL, slot r / CL): 8 CTAs up
-// to n = 256 (one each for many small matrices, see cluster_of), 16 up to NMAX_C16 = 424 (27 rows beside the vectors fill the
-// shared memory) where the device can place such a cluster.  Thread c owns entry
-// c of v_k and w_k in every CTA and keeps it in registers.  Per column:
+// to n = 256 (one each for many small matrices, see cluster_of), 16 up to
+// NMAX_C16 = 424 (27 rows beside the vectors fill the shared memory) where the
+// device can place such a cluster.  Thread c owns entry c of v_k and w_k in
+// every CTA and keeps it in registers.  Per column:
 //   1  row k (loaded from its owner through distributed shared memory while
 //      phase 3 of the column before still ran), update k-1 applied, the norm of
 //      its tail; a CTA barrier
 //   2  the owned rows: update k-1 and (row . unscaled reflector, entry k+1),
 //      pushed to every CTA (double-buffered by column parity, so a CTA that runs
-//      ahead never overwrites a buffer another is still reading); 3, 2 or 1 rows per warp at
-//      a time share the loads of w, v and the reflector.  The last warp computes
-//      tau, beta and the reflector's scale meanwhile.  Then the hardware
-//      cluster barrier, which every CTA executes the same number of times
+//      ahead never overwrites a buffer another is still reading); 3, 2 or 1
+//      rows per warp at a time share the loads of w, v and the reflector.  The
+//      last warp computes tau, beta and the reflector's scale meanwhile.  Then
+//      the hardware cluster barrier, which every CTA executes the same number
+//      of times
 //   3  y_k and v_k scaled, y^H v (a CTA barrier), w_k
 // Bound by that chain of latencies (2 us a column at n = 32), with the rows' traffic in
 // shared memory beside it from n = 200 on: 58 / 274 / 727 us at n = 32 / 128 /
