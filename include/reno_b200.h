@@ -258,8 +258,9 @@ int reno_qr_blocks(reno_ctx* ctx, int32_t count, const reno_qr_block* blocks,
  * synchronises at those checks only.  Fails with RENO_ERR_WORKSPACE when more
  * than kmax Krylov vectors would be needed.  Workspace from
  * reno_lanczos_workspace_bytes(desc, kmax).
- * reno_lanczos_expm_to leaves psi as it is and writes to `out` (which may be
- * psi).
+ * reno_lanczos_expm_to leaves psi as it is and writes to `out`.  `out` may be
+ * psi (reno_lanczos_expm), and must not overlap it otherwise; psi is then still the
+ * start vector after an error.  A separate `out` is undefined after an error.
  * reno_lanczos_coefficients is the exponential's small host problem
  * (krylov.py:15-24), for count of them: row i of scal (ld doubles) holds the
  * start norm and the tridiagonal matrix of order k[i] as alpha_0, beta_0,

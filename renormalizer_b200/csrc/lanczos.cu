@@ -176,6 +176,9 @@ extern "C" int reno_lanczos_expm(reno_ctx* ctx, const reno_heff_desc* desc, cons
 // of coefficients and one read of the flag per convergence test, and tests
 // begin at j = 6: the reference's first approximation (j = 4) is only compared
 // at j = 6, where RENO_VOP_CHECK forms both from one read of the vectors.
+// The tests write their approximation to out; in place they write it to w,
+// free between a step and the next matvec, so that psi is still the start
+// vector when the call fails.
 extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, const void* L, const void* W1,
                                     const void* W2, const void* R, double dt_re, double dt_im, const void* psi,
                                     void* out, int32_t kmax, int32_t* out_k, void* ws, size_t ws_bytes) {
@@ -191,6 +194,7 @@ extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, c
   char* base = static_cast<char*>(ws);
   double2* V = reinterpret_cast<double2*>(base + Lz.V);
   double2* w = reinterpret_cast<double2*>(base + Lz.w);
+  void* approx = out == psi ? static_cast<void*>(w) : out;
   double* scal = reinterpret_cast<double*>(base + Lz.scal);
   double* ab = scal + 2;
   double* dcoef = reinterpret_cast<double*>(base + Lz.coef);
@@ -288,12 +292,15 @@ extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, c
     it.x = V;
     it.y = nullptr;
     it.s = dcoef;
-    it.out = out;
+    it.out = approx;
     it.scalars = scal + 1;
     LZ_TRY(reno_vec_grouped(ctx, RENO_VOP_CHECK, 1, &it, 1e-5, 1e-8, vws, vbytes));
     it.s = nullptr;
     LZ_TRY(read(scal + 1, 1));
     if (host[1] == 1.0) {
+      if (approx != out)
+        LZ_TRY(check_cuda(ctx, cudaMemcpyAsync(out, approx, (size_t)n * sizeof(double2), cudaMemcpyDeviceToDevice, st),
+                          "reno_lanczos_expm: copy out"));
       *out_k = j + 1;
       return RENO_OK;
     }
