@@ -114,17 +114,22 @@ MAX_GROUP = 128  # problems per grouped launch (reno_heff_apply_grouped)
 
 
 class Rows(list):
-    """1-D complex128 device tensors cut from one buffer, with their addresses
-    (``ptrs``, uint64): what a lockstep exponential hands to its operators and
-    apply_grouped hands back, so that neither side looks at each tensor."""
+    """Complex128 device tensors cut from one buffer, with their addresses
+    (``ptrs``, uint64) and sizes: what a lockstep exponential hands to its
+    operators and apply_grouped hands back, so that neither side copies or
+    converts each tensor."""
 
-    def __init__(self, tensors, ptrs):
+    def __init__(self, tensors, ptrs, sizes):
         super().__init__(tensors)
-        self.ptrs = ptrs
+        self.ptrs, self.sizes = ptrs, sizes
 
     def intact(self) -> bool:
-        """whether the list still holds the vectors it was made of"""
-        return len(self) == len(self.ptrs) and [t.data_ptr() for t in self] == self.ptrs.tolist()
+        """whether the list still holds the vectors it was made of, as they lie in
+        memory: an entry that was replaced by a view of its own memory (a lazy
+        conjugate, a transpose, a part) has the same address"""
+        return len(self) == len(self.ptrs) and all(
+            t.data_ptr() == a and t.numel() == n and t.dtype is torch.complex128 and t.is_contiguous()
+            and not (t.is_conj() or t.is_neg()) for t, a, n in zip(self, self.ptrs.tolist(), self.sizes))
 
 
 def _apply_rows(ops: Sequence["HeffOperator"], psis: Rows) -> "Rows":
@@ -138,7 +143,7 @@ def _apply_rows(ops: Sequence["HeffOperator"], psis: Rows) -> "Rows":
         return None
     eng = ops[0].engine
     eng.sync_stream()
-    sizes = [p.numel() for p in psis]
+    sizes = psis.sizes
     if any(n != math.prod(o.cshape) for n, o in zip(sizes, ops)):
         return None
     flat = torch.empty(sum(sizes), dtype=torch.complex128, device=psis[0].device)
@@ -152,7 +157,7 @@ def _apply_rows(ops: Sequence["HeffOperator"], psis: Rows) -> "Rows":
     for c0 in range(0, len(ops), MAX_GROUP):
         part = slice(c0, c0 + MAX_GROUP)
         eng.heff_apply_grouped([o.desc for o in ops[part]], *[f[part] for f in fixed], psis.ptrs[part], ptrs[part])
-    return Rows([y.view(o.cshape) for y, o in zip(flat.split(sizes), ops)], ptrs)
+    return Rows([y.view(o.cshape) for y, o in zip(flat.split(sizes), ops)], ptrs, sizes)
 
 
 def apply_grouped(ops: Sequence["HeffOperator"], psis: Sequence[torch.Tensor]) -> List[torch.Tensor]:

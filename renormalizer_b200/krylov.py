@@ -314,9 +314,10 @@ class _LockstepRows:
     def _images(self, group_apply, active, j):
         """group_apply on the active problems' V[j]: the images (kept alive) and their addresses"""
         row = self.V[j].split(self.sizes)
-        xs = Rows([row[p] for p in active], self._vec(j, active))
+        sizes = self.n[active].tolist()
+        xs = Rows([row[p] for p in active], self._vec(j, active), sizes)
         ws = group_apply(active.tolist(), xs)
-        if isinstance(ws, Rows) and ws.intact():
+        if isinstance(ws, Rows) and ws.sizes == sizes and ws.intact():
             return ws, ws.ptrs
         out = []
         for p, w in zip(active, ws):
