@@ -190,16 +190,16 @@ def _expm_krylov_steps(dt, vstart, block_size=50):
             state["res"] = new_res
 
 
-_APPLY = HeffOperator.apply
+_APPLY, _CALL = HeffOperator.apply, HeffOperator.__call__
 
 
 def _native_expm(op, dt, vstart, kmax):
     """The exponential in one library call, or None where the generic driver
-    serves it: real results, an operator whose ``apply`` was replaced, other
-    tolerances than the reference's, more than kmax vectors, scalars that are
+    serves it: real results, an operator whose ``apply`` or ``__call__`` is not
+    HeffOperator's own, other tolerances than the reference's, more than kmax vectors, scalars that are
     not finite (the driver raises for those)."""
-    if not isinstance(op, HeffOperator) or type(op).apply is not _APPLY or "apply" in vars(op) \
-            or not isinstance(op.engine, Engine):
+    if not isinstance(op, HeffOperator) or type(op).apply is not _APPLY or type(op).__call__ is not _CALL \
+            or "apply" in vars(op) or not isinstance(op.engine, Engine):
         return None
     if (tolerance.rtol, tolerance.atol) != (1e-5, 1e-8):
         return None
