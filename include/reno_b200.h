@@ -10,7 +10,8 @@
  *    the reference's index order (cited per entry point).  complex128 is
  *    interleaved (re, im) doubles, 16-byte aligned.
  *  - Hot calls never allocate: scratch memory ("workspace") is passed in by
- *    the caller and sized by the matching *_workspace_bytes query.
+ *    the caller, aligned to 16 bytes, and sized by the matching
+ *    *_workspace_bytes query.
  *  - Work is enqueued on the context's stream (reno_ctx_set_stream); calls are
  *    asynchronous unless documented otherwise.  One context per host thread.
  *

@@ -122,8 +122,10 @@ __device__ __forceinline__ void st_global_v4(void* p, double a, double b, double
 
 // 16 output values v[t*STRIDE + OFF] (t = 0..15) of one (m, ri) for columns
 // n0 .. n0+15 into the packed planes: 32-byte stores (whole sectors; 16-byte
-// ones took up to a fifth of a stage longer) when the run is contiguous and
-// aligned, scalar stores otherwise.  Lanes hold different rows, so a store
+// ones took up to a fifth of a stage longer) when the run is contiguous and its
+// address allows it, 16-byte ones where it lies on half a sector (an odd row pitch, or a
+// workspace that is itself aligned to 16 bytes, all that the tensor maps ask for),
+// scalar stores otherwise.  Lanes hold different rows, so a store
 // instruction costs a cycle of the load/store unit per lane whatever its width.
 template <int ESZ, int STRIDE, int OFF>
 __device__ __forceinline__ void pack_run(const float* v, const Epi& e, int64_t mbase, int n0, int ri) {
@@ -131,22 +133,27 @@ __device__ __forceinline__ void pack_run(const float* v, const Epi& e, int64_t m
   const int nq = n0 / e.Dn;
   int nr = n0 - nq * e.Dn;
   const int64_t idx0 = mbase + (int64_t)ri * e.s_ri + (int64_t)nq * e.s_n1 + (int64_t)nr * e.s_n0;
-  const bool vec = e.s_n0 == 1 && n0 + 16 <= e.N && nr + 16 <= e.Dn && (idx0 % (32 / ESZ)) == 0;
-  if (vec) {
+  unsigned char* planes[2] = {reinterpret_cast<unsigned char*>(e.phi) + idx0 * ESZ,
+                              reinterpret_cast<unsigned char*>(e.plo) + idx0 * ESZ};
+  const uintptr_t off = (reinterpret_cast<uintptr_t>(planes[0]) | reinterpret_cast<uintptr_t>(planes[1])) % 32;
+  if (e.s_n0 == 1 && n0 + 16 <= e.N && nr + 16 <= e.Dn && off % 16 == 0) {
     uint32_t hb[16], lb[16];
 #pragma unroll
     for (int t = 0; t < 16; ++t) split_bits<ESZ>(v[t * STRIDE + OFF], hb[t], lb[t]);
-    // whole 32-byte sectors per store
     uint32_t w[4 * ESZ];  // 16 elements of one plane, 32 bits at a time
-    unsigned char* planes[2] = {reinterpret_cast<unsigned char*>(e.phi) + idx0 * ESZ,
-                                reinterpret_cast<unsigned char*>(e.plo) + idx0 * ESZ};
 #pragma unroll
     for (int pl = 0; pl < 2; ++pl) {
       const uint32_t* src = pl == 0 ? hb : lb;
 #pragma unroll
       for (int q = 0; q < 4 * ESZ; ++q) w[q] = ESZ == 2 ? src[2 * q] | (src[2 * q + 1] << 16) : src[q];
+      if (off == 0) {
 #pragma unroll
-      for (int q = 0; q < ESZ / 2; ++q) st_global_v8(planes[pl] + 32 * q, w + 8 * q);
+        for (int q = 0; q < ESZ / 2; ++q) st_global_v8(planes[pl] + 32 * q, w + 8 * q);
+      } else {
+#pragma unroll
+        for (int q = 0; q < ESZ; ++q)
+          reinterpret_cast<uint4*>(planes[pl])[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+      }
     }
   } else {
     // the index moves along with n: with a division per element this branch took 220 cycles a value, and
