@@ -446,8 +446,9 @@ inline cudaError_t launch_one(const GemmParams& p, int S, cudaStream_t st) {
   cudaError_t e = smem_optin_once(gemm_kernel<AC, BC, TILE>, (int)sm, smem_set);
   if (e != cudaSuccess) return e;
   const int64_t nx = ceil_div(p.N, BT), ny = ceil_div(p.M, BT);
-  // walk the tiles of the smaller operand fastest, so that the larger one streams from HBM once
-  const int m_fast = p.M < p.N && nx <= 65535 ? 1 : 0;
+  // walk the tiles of the smaller operand fastest, so that the larger one streams from HBM once;
+  // the grid's y holds 65535 tiles (1.05 M rows of 16), so that a taller product has them along x
+  const int m_fast = nx <= 65535 && (p.M < p.N || ny > 65535) ? 1 : 0;
   const dim3 grid((unsigned)((m_fast ? ny : nx) * S), (unsigned)(m_fast ? nx : ny), (unsigned)p.batch);
   return launch_clustered(gemm_kernel<AC, BC, TILE>, grid, sm, S, st, p, S, m_fast);
 }
