@@ -978,13 +978,14 @@ __global__ void __launch_bounds__(CT, 1) hetrd_cluster_kernel(const __grid_const
 // Sign changes of the leading principal minors p_i of T - x I = eigenvalues of T
 // below x (Givens 1953): p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}.  The recurrence
 // has one fused multiply-add on its chain, the pivot form q_i = d_i - x - e^2 / q
-// a division.  T comes scaled by a power of two to norm <= 1 and e^2 is at
-// least 2^-140 (eigenvalues move by 2^-69 of the norm at most), so that eight steps
-// change the larger of two neighbouring minors by at most 3^8 up or 2^-560
-// down: rescaled by 2^+-560 outside [2^-400, 2^400], it never leaves FP64's
-// range.  A minor that is exactly 0 counts once whatever its sign, as the one after
-// it has the opposite sign of the one before.
-constexpr int SCH = 8;  // steps between rescalings; the arrays are padded to a multiple
+// a division.  T comes scaled by a power of two to norm <= 1, and e^2 is at least
+// E2MIN = 2^-236 (eigenvalues move by 2^-117 of the norm at most).  A step takes
+// the larger of two neighbouring minors up by at most 3 and down by at most E2MIN / 4:
+// a smaller p_i leaves p_{i+1} above E2MIN / 2 of p_{i-1}.  Four steps from a pair
+// scaled to [1, 2) therefore stay in FP64's range.  A minor that is exactly 0
+// counts once whatever its sign, as the one after it has the opposite sign of the one before.
+constexpr int SCH = 4;  // steps between rescalings; the arrays are padded to a multiple
+constexpr double E2MIN = 0x1p-236;
 __device__ __forceinline__ int sturm_count(const double2* t, int n, double x) {
   double p0 = 1.0, p1 = t[0].x - x;  // t[i] = (d_i, e_{i-1}^2)
   int cnt = __double2hiint(p1) < 0;
@@ -992,8 +993,8 @@ __device__ __forceinline__ int sturm_count(const double2* t, int n, double x) {
     double2 c[SCH];
 #pragma unroll
     for (int u = 0; u < SCH; ++u) c[u] = t[i0 + u];
-    const int m = max(__double2hiint(p0) & 0x7fffffff, __double2hiint(p1) & 0x7fffffff);
-    const double f = m < ((1023 - 400) << 20) ? 0x1p560 : m > ((1023 + 400) << 20) ? 0x1p-560 : 1.0;
+    const int m = max(__double2hiint(p0) & 0x7ff00000, __double2hiint(p1) & 0x7ff00000);
+    const double f = __hiloint2double((2046 << 20) - m, 0);  // 2^-exponent of the larger
     p0 *= f;
     p1 *= f;
 #pragma unroll
@@ -1003,6 +1004,21 @@ __device__ __forceinline__ int sturm_count(const double2* t, int n, double x) {
       p0 = p1;
       p1 = p2;
     }
+  }
+  return cnt;
+}
+
+// The same count from the pivots, for x so near 0 that E2MIN would show: e as
+// it is (s = 2^-exponent of T's norm), LAPACK dstebz's guard |q| >= pivmin.
+__device__ __forceinline__ int sturm_count_pivots(const double2* t, const double* e, int ex, int n, double x) {
+  double q = t[0].x - x;
+  if (fabs(q) < DBL_MIN) q = -DBL_MIN;
+  int cnt = q < 0.0;
+  for (int i = 1; i < n; ++i) {
+    const double s = ldexp(e[i - 1], -ex);
+    q = (t[i].x - x) - s * s / q;
+    if (fabs(q) < DBL_MIN) q = -DBL_MIN;
+    cnt += q < 0.0;
   }
   return cnt;
 }
@@ -1060,10 +1076,12 @@ __device__ __forceinline__ int norm_exponent(const double* bnd) {
 }
 
 // eigenvalue i0 + j (ascending) of T for j < cnt, one warp each: the bracket is
-// cut into 33 parts per round, down to 2 ulp or 2^-64 of the norm (the reduction
-// left an error of 2^-52 of it).  Bound by the latency of the minors' chain (one
+// cut into 33 parts per round, down to 2 ulp of the eigenvalue.  Those below
+// 2^-60 of the norm (blocks of exact zeros, graded diagonals) take their last
+// rounds with the pivot form.  Bound by the latency of the minors' chain (one
 // warp per scheduler where the matrices are small): the top half of an n = 240
-// spectrum takes 36 us, 415 with a division on the chain.
+// spectrum whose last values lie at 2^-53 of the norm (21 rounds) takes 79 us, 415
+// with a division on the chain; 37 with rounds only down to 2^-64 of the norm.
 constexpr int BW = 4, BT = 32 * BW;
 __global__ void __launch_bounds__(BT) bisect_kernel(const __grid_constant__ EigTable tab) {
   const EigProb& PR = tab.p[blockIdx.y];
@@ -1082,7 +1100,7 @@ __global__ void __launch_bounds__(BT) bisect_kernel(const __grid_constant__ EigT
       c.x = ldexp(d[i], -ex);
       if (i > 0) {
         const double s = ldexp(e[i - 1], -ex);
-        c.y = fmax(s * s, 0x1p-140);
+        c.y = fmax(s * s, E2MIN);
       }
     }
     t[i] = c;
@@ -1093,10 +1111,17 @@ __global__ void __launch_bounds__(BT) bisect_kernel(const __grid_constant__ EigT
   if (j >= cnt) return;
   const int idx = i0 + j;
   double lo = ldexp(bnd[0], -ex), hi = ldexp(bnd[1], -ex);
+  bool pivots = false;
   for (int round = 0; round < 40; ++round) {
-    if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + 0x1p-64) break;
+    const double ulps = 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi));
+    if (hi - lo <= ulps + (pivots ? DBL_MIN : 0x1p-112)) {
+      if (pivots || ulps >= 0x1p-111) break;
+      pivots = true;  // the bracket holds the eigenvalue to 2^-117
+      lo -= 0x1p-114;
+      hi += 0x1p-114;
+    }
     const double x = lo + (hi - lo) * ((double)(lane + 1) / 33.0);
-    const int c = sturm_count(t, n, x);
+    const int c = pivots ? sturm_count_pivots(t, e, ex, n, x) : sturm_count(t, n, x);
     // count(x) > idx  <=>  eigenvalue idx < x
     const unsigned above = __ballot_sync(0xffffffffu, c > idx);
     const int first = above ? __ffs(above) - 1 : 32;
