@@ -1147,6 +1147,54 @@ __device__ __forceinline__ double hash_unit(uint32_t a, uint32_t b) {
   return (double)h * (2.0 / 4294967296.0) - 1.0;
 }
 
+// The three recurrences of a vector, in fixed operations, so that both kernels
+// below round alike: which of them a matrix gets depends on what else is in the
+// call, and its vectors must not.
+//
+// Row k of the LU factors of T - lambda I with partial pivoting.  The current
+// row has entries (ak, ck) at columns (k, k+1), the next original row (bk, ak1,
+// ck1) at (k, k+1, k+2); U's row is 1 / inv, p1, p2, and ml the multiplier (+4
+// when the two were swapped, |multiplier| <= 1 either way).  A pivot below tiny becomes tiny.
+struct IvRow {
+  double inv, p1, p2, ml;
+};
+__device__ __forceinline__ IvRow iv_eliminate(double& ak, double& ck, double bk, double ak1, double ck1, double tiny) {
+  const bool swap = fabs(ak) < fabs(bk);
+  IvRow r;
+  r.p1 = swap ? ak1 : ck;
+  r.p2 = swap ? ck1 : 0.0;
+  const double q = swap ? ak : bk, q1 = swap ? ck : ak1, q2 = swap ? 0.0 : ck1;
+  double p = swap ? bk : ak;
+  if (fabs(p) < tiny) p = copysign(tiny, p);
+  r.inv = 1.0 / p;
+  const double m = __dmul_rn(q, r.inv);
+  r.ml = swap ? m + 4.0 : m;
+  ak = __fma_rn(-m, r.p1, q1);
+  ck = __fma_rn(-m, r.p2, q2);
+  return r;
+}
+// the last pivot's reciprocal
+__device__ __forceinline__ double iv_last(double ak, double tiny) {
+  return 1.0 / (fabs(ak) < tiny ? copysign(tiny, ak) : ak);
+}
+// L^-1 at row k: returns entry k, zk moves on to k+1, whose entry is zn
+__device__ __forceinline__ double iv_forward(double ml, double zn, double& zk) {
+  const bool swap = ml > 2.0;
+  const double m = swap ? ml - 4.0 : ml;
+  const double out = swap ? zn : zk;
+  zk = __fma_rn(-m, out, swap ? zk : zn);
+  return out;
+}
+// U^-1 at row k, entries k+1 and k+2 in z1 and z2; adds to the squared norm
+__device__ __forceinline__ double iv_backward(double z, double p1, double p2, double inv, double& z1, double& z2,
+                                              double& nrm) {
+  const double v = __dmul_rn(__fma_rn(-p1, z1, __fma_rn(-p2, z2, z)), inv);
+  z2 = z1;
+  z1 = v;
+  nrm = __fma_rn(v, v, nrm);
+  return v;
+}
+
 constexpr int IV_THREADS = 128, CH = 8, IV_WAVES = 4;
 
 // The same iteration with every array of a vector in shared memory, V vectors
@@ -1186,48 +1234,31 @@ __global__ void __launch_bounds__(32) inviter_smem_kernel(const __grid_constant_
   double ak = sd[0] - lam;
   double ck = se[0];
   for (int k = 0; k < n - 1; ++k) {
-    const double bk = se[k];
-    const double ak1 = sd[k + 1] - lam;
-    const double ck1 = se[k + 1];
-    const bool swap = fabs(ak) < fabs(bk);
-    // pivot row (p, p1, p2), the other row (q, q1, q2); a pivot below tiny becomes tiny
-    const double p1 = swap ? ak1 : ck, p2 = swap ? ck1 : 0.0;
-    const double q = swap ? ak : bk, q1 = swap ? ck : ak1, q2 = swap ? 0.0 : ck1;
-    double p = swap ? bk : ak;
-    if (fabs(p) < tiny) p = copysign(tiny, p);
-    const double inv = 1.0 / p, m = q * inv;
-    ua[k * V] = inv;
-    uc[k * V] = p1;
-    uc2[k * V] = p2;
-    ml[k * V] = swap ? m + 4.0 : m;
-    ak = q1 - m * p1;
-    ck = q2 - m * p2;
+    const IvRow r = iv_eliminate(ak, ck, se[k], sd[k + 1] - lam, se[k + 1], tiny);
+    ua[k * V] = r.inv;
+    uc[k * V] = r.p1;
+    uc2[k * V] = r.p2;
+    ml[k * V] = r.ml;
   }
-  if (fabs(ak) < tiny) ak = copysign(tiny, ak);
-  ua[(n - 1) * V] = 1.0 / ak;
+  ua[(n - 1) * V] = iv_last(ak, tiny);
   uc[(n - 1) * V] = 0.0;
   uc2[(n - 1) * V] = 0.0;
   for (int i = 0; i < n; ++i) z[i * V] = hash_unit((uint32_t)j + 1u, (uint32_t)i);
   double inv = 1.0;
   for (int it = 0; it < 3; ++it) {
     // forward: L^-1 with the row swaps
-    double zk = z[0] * inv;
+    double zk = __dmul_rn(z[0], inv);
     for (int k0 = 0; k0 < n - 1; k0 += CH) {
       double mm[CH], zn[CH];
 #pragma unroll
       for (int u = 0; u < CH; ++u) {
         const int k = min(k0 + u, n - 2);
         mm[u] = ml[k * V];
-        zn[u] = z[(k + 1) * V] * inv;
+        zn[u] = __dmul_rn(z[(k + 1) * V], inv);
       }
 #pragma unroll
       for (int u = 0; u < CH; ++u) {
-        if (k0 + u < n - 1) {
-          const bool swap = mm[u] > 2.0;
-          const double m = swap ? mm[u] - 4.0 : mm[u];
-          z[(k0 + u) * V] = swap ? zn[u] : zk;
-          zk = swap ? zk - m * zn[u] : zn[u] - m * zk;
-        }
+        if (k0 + u < n - 1) z[(k0 + u) * V] = iv_forward(mm[u], zn[u], zk);
       }
     }
     z[(n - 1) * V] = zk;
@@ -1245,13 +1276,7 @@ __global__ void __launch_bounds__(32) inviter_smem_kernel(const __grid_constant_
       }
 #pragma unroll
       for (int u = 0; u < CH; ++u) {
-        if (k0 - u >= 0) {
-          const double v = (zz[u] - c2[u] * z2 - c1[u] * z1) * ia[u];
-          z[(k0 - u) * V] = v;
-          z2 = z1;
-          z1 = v;
-          nrm += v * v;
-        }
+        if (k0 - u >= 0) z[(k0 - u) * V] = iv_backward(zz[u], c1[u], c2[u], ia[u], z1, z2, nrm);
       }
     }
     inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
@@ -1292,47 +1317,18 @@ __global__ void __launch_bounds__(IV_THREADS) inviter_kernel(const __grid_consta
   const double lam = ldexp(w[j], -ex);
   const double tn = ldexp(fmax(fabs(bnd[0]), fabs(bnd[1])), -ex);
   const double tiny = DBL_EPSILON * fmax(tn, DBL_MIN);
-  // LU of T - lam I with partial pivoting.  The current row k has entries
-  // (ak, ck) at columns (k, k+1); the next original row is (bk, ak1, ck1) at
-  // columns (k, k+1, k+2).  U row k is (ak, ck, 0) without a swap and
-  // (bk, ak1, ck1) with one; |multiplier| <= 1 either way.
   double ak = sd[0] - lam;
   double ck = se[0];
   for (int k = 0; k < n - 1; ++k) {
-    const double bk = se[k];
-    const double ak1 = sd[k + 1] - lam;
-    const double ck1 = se[k + 1];
-    double u_kk, u_k1, u_k2, flagged;
-    if (fabs(ak) >= fabs(bk)) {
-      u_kk = ak == 0.0 ? tiny : ak;
-      u_k1 = ck;
-      u_k2 = 0.0;
-      const double m = bk / u_kk;
-      flagged = m;
-      ak = ak1 - m * ck;
-      ck = ck1;
-    } else {
-      u_kk = bk;
-      u_k1 = ak1;
-      u_k2 = ck1;
-      const double m = ak / bk;
-      flagged = m + 4.0;
-      ak = ck - m * ak1;
-      ck = -m * ck1;
-    }
-    if (fabs(u_kk) < tiny) u_kk = copysign(tiny, u_kk);
-    ua[(size_t)k * S + j] = 1.0 / u_kk;
-    uc[(size_t)k * S + j] = u_k1;
-    uc2[(size_t)k * S + j] = u_k2;
-    ml[(size_t)k * S + j] = flagged;
+    const IvRow r = iv_eliminate(ak, ck, se[k], sd[k + 1] - lam, se[k + 1], tiny);
+    ua[(size_t)k * S + j] = r.inv;
+    uc[(size_t)k * S + j] = r.p1;
+    uc2[(size_t)k * S + j] = r.p2;
+    ml[(size_t)k * S + j] = r.ml;
   }
-  {
-    double u = ak;
-    if (fabs(u) < tiny) u = copysign(tiny, u == 0.0 ? 1.0 : u);
-    ua[(size_t)(n - 1) * S + j] = 1.0 / u;
-    uc[(size_t)(n - 1) * S + j] = 0.0;
-    uc2[(size_t)(n - 1) * S + j] = 0.0;
-  }
+  ua[(size_t)(n - 1) * S + j] = iv_last(ak, tiny);
+  uc[(size_t)(n - 1) * S + j] = 0.0;
+  uc2[(size_t)(n - 1) * S + j] = 0.0;
   double* z = Z;
 #pragma unroll 8
   for (int i = 0; i < n; ++i) z[(size_t)i * S + j] = hash_unit((uint32_t)j + 1u, (uint32_t)i);
@@ -1350,15 +1346,7 @@ __global__ void __launch_bounds__(IV_THREADS) inviter_kernel(const __grid_consta
 #pragma unroll
       for (int u = 0; u < CH; ++u) {
         const int k = k0 + u;
-        if (k < n - 1) {
-          if (mm[u] > 2.0) {  // rows k, k+1 swapped
-            z[(size_t)k * S + j] = zn[u];
-            zk = zk - (mm[u] - 4.0) * zn[u];
-          } else {
-            z[(size_t)k * S + j] = zk;
-            zk = zn[u] - mm[u] * zk;
-          }
-        }
+        if (k < n - 1) z[(size_t)k * S + j] = iv_forward(mm[u], zn[u], zk);
       }
     }
     z[(size_t)(n - 1) * S + j] = zk;
@@ -1378,13 +1366,7 @@ __global__ void __launch_bounds__(IV_THREADS) inviter_kernel(const __grid_consta
 #pragma unroll
       for (int u = 0; u < CH; ++u) {
         const int k = k0 - u;
-        if (k >= 0) {
-          const double v = (zz[u] - c1[u] * z1 - c2[u] * z2) * ia[u];
-          z[(size_t)k * S + j] = v;
-          z2 = z1;
-          z1 = v;
-          nrm += v * v;
-        }
+        if (k >= 0) z[(size_t)k * S + j] = iv_backward(zz[u], c1[u], c2[u], ia[u], z1, z2, nrm);
       }
     }
     const double inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
