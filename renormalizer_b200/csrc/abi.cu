@@ -21,7 +21,6 @@ extern "C" int reno_ctx_create(int device, reno_ctx** out) {
 }
 
 extern "C" int reno_ctx_destroy(reno_ctx* ctx) {
-  if (ctx && ctx->host_scalars) cudaFreeHost(ctx->host_scalars);
   delete ctx;
   return RENO_OK;
 }

@@ -176,6 +176,8 @@ extern "C" int reno_lanczos_expm(reno_ctx* ctx, const reno_heff_desc* desc, cons
 // of coefficients and one read of the flag per convergence test, and tests
 // begin at j = 6: the reference's first approximation (j = 4) is only compared
 // at j = 6, where RENO_VOP_CHECK forms both from one read of the vectors.
+// (Pageable host memory: the copies return once it has been read or staged, and a
+// pinned block would have to be allocated in a hot call.)
 // The tests write their approximation to out; in place they write it to w,
 // free between a step and the next matvec, so that psi is still the start
 // vector when the call fails.
@@ -211,34 +213,22 @@ extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, c
     rc = (call);                  \
     if (rc != RENO_OK) return rc; \
   } while (0)
-  // pinned: the scalars read, then the coefficients sent
-  const size_t nscal = 2 * (size_t)kmax + 4, pinned = nscal + 4 * ((size_t)kmax + 1);
-  if (ctx->host_scalars_count < pinned) {
-    if (ctx->host_scalars) cudaFreeHost(ctx->host_scalars);
-    ctx->host_scalars = nullptr;
-    ctx->host_scalars_count = 0;
-    void* p = nullptr;
-    LZ_TRY(check_cuda(ctx, cudaMallocHost(&p, pinned * sizeof(double)), "reno_lanczos_expm: pinned scalars"));
-    ctx->host_scalars = static_cast<double*>(p);
-    ctx->host_scalars_count = pinned;
-  }
-  double* host = ctx->host_scalars;
-  double* hcoef = host + nscal;
+  std::vector<double> host(2 * (size_t)kmax + 4), hcoef(4 * ((size_t)kmax + 1));  // read / sent
   reno_vec_item it{};
   it.n = n;
   it.dtype = RENO_C128;
   it.ldv = n;
   auto read = [&](const double* from, size_t count) -> int {
-    int r = check_cuda(ctx, cudaMemcpyAsync(host + (from - scal), from, count * sizeof(double), cudaMemcpyDeviceToHost,
-                                            st), "reno_lanczos_expm: scalars");
+    int r = check_cuda(ctx, cudaMemcpyAsync(host.data() + (from - scal), from, count * sizeof(double),
+                                            cudaMemcpyDeviceToHost, st), "reno_lanczos_expm: scalars");
     return r != RENO_OK ? r : check_cuda(ctx, cudaStreamSynchronize(st), "reno_lanczos_expm: sync");
   };
   auto send = [&](size_t count) -> int {
-    return check_cuda(ctx, cudaMemcpyAsync(dcoef, hcoef, count * sizeof(double), cudaMemcpyHostToDevice, st),
+    return check_cuda(ctx, cudaMemcpyAsync(dcoef, hcoef.data(), count * sizeof(double), cudaMemcpyHostToDevice, st),
                       "reno_lanczos_expm: coefficients");
   };
   auto coefficients = [&](int k, double* to) -> int {
-    return tridiag_coeffs(k, host + 2, host[0], dt_re, dt_im, to)
+    return tridiag_coeffs(k, host.data() + 2, host[0], dt_re, dt_im, to)
                ? RENO_OK
                : set_error(ctx, RENO_ERR_NONFINITE, "reno_lanczos_expm: Lanczos scalars are not finite");
   };
@@ -276,17 +266,15 @@ extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, c
       }
     checked = upto;
     if (k > 0) {
-      LZ_TRY(coefficients(k, hcoef));
+      LZ_TRY(coefficients(k, hcoef.data()));
       LZ_TRY(send(2 * (size_t)k));
       LZ_TRY(reno_vec_lincomb(ctx, n, k, RENO_C128, V, n, dcoef, out));
-      // the next exponential may refill the pinned coefficients: wait for the copy
-      LZ_TRY(check_cuda(ctx, cudaStreamSynchronize(st), "reno_lanczos_expm: sync"));
       *out_k = k;
       return RENO_OK;
     }
     if (!(j > 5 && j % 2 == 0)) continue;
-    LZ_TRY(coefficients(j + 1, hcoef));
-    LZ_TRY(coefficients(j - 1, hcoef + 2 * (size_t)(j + 1)));
+    LZ_TRY(coefficients(j + 1, hcoef.data()));
+    LZ_TRY(coefficients(j - 1, hcoef.data() + 2 * (size_t)(j + 1)));
     LZ_TRY(send(4 * (size_t)j));
     it.j = j + 1;
     it.x = V;

@@ -16,10 +16,6 @@ struct reno_ctx {
   cudaStream_t stream = nullptr;
   int num_sms = 148;
   std::string last_error;
-  // pinned host memory for scalars that cross between host and device
-  // (Krylov alpha / beta, coefficients), made on first use
-  double* host_scalars = nullptr;
-  size_t host_scalars_count = 0;
 };
 
 namespace reno {
