@@ -262,6 +262,11 @@ int reno_qr_blocks(reno_ctx* ctx, int32_t count, const reno_qr_block* blocks,
  * reno_lanczos_expm_to leaves psi as it is and writes to `out`.  `out` may be
  * psi (reno_lanczos_expm), and must not overlap it otherwise; psi is then still the
  * start vector after an error.  A separate `out` is undefined after an error.
+ * reno_lanczos_expm_resume goes on where a call with prev_kmax vectors ended
+ * with RENO_ERR_WORKSPACE for want of more (out_k is then its kmax, 0 after
+ * any other error): prev_ws is that call's workspace,
+ * unchanged, ws one for kmax > prev_kmax vectors (not overlapping it), the operator and step
+ * are the same.  The result is that of one call with kmax vectors.
  * reno_lanczos_coefficients is the exponential's small host problem
  * (krylov.py:15-24), for count of them: row i of scal (ld doubles) holds the
  * start norm and the tridiagonal matrix of order k[i] as alpha_0, beta_0,
@@ -282,6 +287,12 @@ int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc,
                          const void* R, double dt_re, double dt_im,
                          const void* psi, void* out, int32_t kmax,
                          int32_t* out_k, void* ws, size_t ws_bytes);
+int reno_lanczos_expm_resume(reno_ctx* ctx, const reno_heff_desc* desc,
+                             const void* L, const void* W1, const void* W2,
+                             const void* R, double dt_re, double dt_im,
+                             void* out, int32_t kmax, int32_t prev_kmax,
+                             const void* prev_ws, int32_t* out_k, void* ws,
+                             size_t ws_bytes);
 
 /* QN-blocked truncation of one coefficient matrix (rows x cols, row-major):
  * svd_qn.py:99-240 with select_basis lib.py:253-322 (percent 0) and

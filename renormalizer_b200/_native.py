@@ -94,6 +94,9 @@ _SIGS = {
                                    _vp, _c_int, ctypes.POINTER(ctypes.c_int32), _vp, _c_sz]),
     "reno_lanczos_expm_to": (_c_int, [_vp, ctypes.POINTER(HeffDesc), _vp, _vp, _vp, _vp, ctypes.c_double,
                                       ctypes.c_double, _vp, _vp, _c_int, ctypes.POINTER(ctypes.c_int32), _vp, _c_sz]),
+    "reno_lanczos_expm_resume": (_c_int, [_vp, ctypes.POINTER(HeffDesc), _vp, _vp, _vp, _vp, ctypes.c_double,
+                                          ctypes.c_double, _vp, _c_int, _c_int, _vp, ctypes.POINTER(ctypes.c_int32),
+                                          _vp, _c_sz]),
     "reno_lanczos_coefficients": (_c_int, [_c_int, _vp, _vp, _c_i64, _vp, _vp]),
     "reno_qn_svd_truncate_workspace_bytes": (_c_int, [ctypes.POINTER(TruncDesc), ctypes.POINTER(_c_sz)]),
     "reno_qn_svd_truncate": (_c_int, [_vp, ctypes.POINTER(TruncDesc), _vp, _vp, _vp, _c_int, _vp, _vp,
@@ -528,19 +531,28 @@ class Engine:
             self.check(self.lib.reno_vec_grouped(self.ctx, op, m, arr, rtol, atol, ptr(self._vec_gws),
                                                  self._vec_gws.numel()), "reno_vec_grouped")
 
-    def lanczos_expm(self, desc: HeffDesc, L, W1, W2, R, dt, psi, kmax):
+    def lanczos_expm(self, desc: HeffDesc, L, W1, W2, R, dt, psi, block):
         """reno_lanczos_expm_to: (exp(dt H_eff) psi, number of matvecs), or None
-        where its kmax vectors do not suffice or its scalars are not finite"""
-        n = _c_sz()
-        self.check(self.lib.reno_lanczos_workspace_bytes(ctypes.byref(desc), kmax, ctypes.byref(n)),
-                   "reno_lanczos_workspace_bytes")
-        ws = torch.empty(int(n.value), dtype=torch.uint8, device=psi.device)
+        where its scalars are not finite.  Vectors come ``block`` at a time: a call that
+        needs more is resumed in a larger workspace."""
         out = torch.empty_like(psi)
         k = ctypes.c_int32(0)
-        st = self.lib.reno_lanczos_expm_to(self.ctx, ctypes.byref(desc), ptr(L), ptr(W1), ptr(W2), ptr(R),
-                                           float(dt.real), float(dt.imag), ptr(psi), ptr(out), kmax, ctypes.byref(k),
-                                           ptr(ws), ws.numel())
-        if st in (RENO_ERR_WORKSPACE, RENO_ERR_NONFINITE):
+        head = (self.ctx, ctypes.byref(desc), ptr(L), ptr(W1), ptr(W2), ptr(R), float(dt.real), float(dt.imag))
+        kmax, prev, st = 0, None, RENO_ERR_WORKSPACE
+        while st == RENO_ERR_WORKSPACE and k.value == kmax:
+            had, kmax = kmax, kmax + block
+            n = _c_sz()
+            self.check(self.lib.reno_lanczos_workspace_bytes(ctypes.byref(desc), kmax, ctypes.byref(n)),
+                       "reno_lanczos_workspace_bytes")
+            ws = torch.empty(int(n.value), dtype=torch.uint8, device=psi.device)
+            if prev is None:
+                st = self.lib.reno_lanczos_expm_to(*head, ptr(psi), ptr(out), kmax, ctypes.byref(k), ptr(ws),
+                                                   ws.numel())
+            else:
+                st = self.lib.reno_lanczos_expm_resume(*head, ptr(out), kmax, had, ptr(prev), ctypes.byref(k), ptr(ws),
+                                                       ws.numel())
+            prev = ws
+        if st == RENO_ERR_NONFINITE:
             return None
         self.check(st, "reno_lanczos_expm")
         self.launches += int(k.value)

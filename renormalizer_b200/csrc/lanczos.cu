@@ -166,12 +166,6 @@ extern "C" int reno_lanczos_coefficients(int32_t count, const int32_t* k, const 
   return RENO_OK;
 }
 
-extern "C" int reno_lanczos_expm(reno_ctx* ctx, const reno_heff_desc* desc, const void* L, const void* W1,
-                                 const void* W2, const void* R, double dt_re, double dt_im, void* psi, int32_t kmax,
-                                 int32_t* out_k, void* ws, size_t ws_bytes) {
-  return reno_lanczos_expm_to(ctx, desc, L, W1, W2, R, dt_re, dt_im, psi, psi, kmax, out_k, ws, ws_bytes);
-}
-
 // The host's share of an exponential is one read of the scalars, one upload
 // of coefficients and one read of the flag per convergence test, and tests
 // begin at j = 6: the reference's first approximation (j = 4) is only compared
@@ -181,14 +175,20 @@ extern "C" int reno_lanczos_expm(reno_ctx* ctx, const reno_heff_desc* desc, cons
 // The tests write their approximation to out; in place they write it to w,
 // free between a step and the next matvec, so that psi is still the start
 // vector when the call fails.
-extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, const void* L, const void* W1,
-                                    const void* W2, const void* R, double dt_re, double dt_im, const void* psi,
-                                    void* out, int32_t kmax, int32_t* out_k, void* ws, size_t ws_bytes) {
+// With prev, a call with k0 vectors went before and ended with
+// RENO_ERR_WORKSPACE: its vectors and scalars are taken over from its workspace
+// and the recurrence goes on at j = k0.  No decision looks further back than
+// the scalars (both approximations of a test are formed from the vectors), so the result
+// is bit for bit that of one call with enough vectors.
+static int lanczos_run(reno_ctx* ctx, const reno_heff_desc* desc, const void* L, const void* W1, const void* W2,
+                       const void* R, double dt_re, double dt_im, const void* psi, void* out, int32_t kmax, int32_t k0,
+                       const void* prev, int32_t* out_k, void* ws, size_t ws_bytes) {
   if (!ctx) return RENO_ERR_INVALID;
-  if (!desc || !psi || !out || !out_k || !ws || kmax < 1)
-    return set_error(ctx, RENO_ERR_INVALID, "reno_lanczos_expm: null argument or kmax < 1");
+  if (!desc || !(psi || prev) || !out || !out_k || !ws || kmax < 1 || (prev && (k0 < 1 || k0 >= kmax)))
+    return set_error(ctx, RENO_ERR_INVALID, "reno_lanczos_expm: null argument or bad vector count");
   if (desc->psi_dtype != RENO_C128)
     return set_error(ctx, RENO_ERR_INVALID, "reno_lanczos_expm: psi must be complex128");
+  *out_k = 0;
   LzLayout Lz;
   if (lz_layout(desc, kmax, Lz) != RENO_OK) return set_error(ctx, RENO_ERR_INVALID, "reno_lanczos_expm: bad descriptor");
   if (ws_bytes < Lz.total) return set_error(ctx, RENO_ERR_WORKSPACE, "reno_lanczos_expm: workspace too small");
@@ -232,15 +232,28 @@ extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, c
                ? RENO_OK
                : set_error(ctx, RENO_ERR_NONFINITE, "reno_lanczos_expm: Lanczos scalars are not finite");
   };
-  LZ_TRY(reno_vec_norm(ctx, n, RENO_C128, psi, scal, vws, vbytes));
-  LZ_TRY(reno_vec_scale_inv(ctx, n, RENO_C128, psi, scal, V));
-  int checked = 0;
-  for (int j = 0; j < n; ++j) {
-    if (j >= kmax)
+  const int j0 = prev ? k0 : 0;
+  if (prev) {
+    LzLayout P;
+    lz_layout(desc, k0, P);
+    const char* from = static_cast<const char*>(prev);
+    cudaError_t e = cudaMemcpyAsync(V, from + P.V, ((size_t)k0 + 1) * n * sizeof(double2), cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(scal, from + P.scal, (2 + 2 * (size_t)k0) * sizeof(double), cudaMemcpyDeviceToDevice, st);
+    LZ_TRY(check_cuda(ctx, e, "reno_lanczos_expm_resume: copy"));
+  } else {
+    LZ_TRY(reno_vec_norm(ctx, n, RENO_C128, psi, scal, vws, vbytes));
+    LZ_TRY(reno_vec_scale_inv(ctx, n, RENO_C128, psi, scal, V));
+  }
+  int checked = j0;  // a call that ran out of vectors looked at every beta it has
+  for (int j = j0; j < n; ++j) {
+    if (j >= kmax) {
+      *out_k = kmax;
       return set_error(ctx, RENO_ERR_WORKSPACE, "reno_lanczos_expm: no convergence within kmax = " +
                                                     std::to_string(kmax) + " Krylov vectors; raise kmax");
+    }
     double2* vj = V + (size_t)j * n;
-    LZ_TRY(heff_apply_prepared(ctx, desc, L, W1, W2, R, vj, w, hws, hbytes, j > 0));
+    LZ_TRY(heff_apply_prepared(ctx, desc, L, W1, W2, R, vj, w, hws, hbytes, j > j0));
     const bool exhausted = (j == n - 1);
     it.j = j;
     it.scalars = ab;
@@ -295,4 +308,25 @@ extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, c
   }
 #undef LZ_TRY
   return set_error(ctx, RENO_ERR_INVALID, "reno_lanczos_expm: empty vector");
+}
+
+extern "C" int reno_lanczos_expm(reno_ctx* ctx, const reno_heff_desc* desc, const void* L, const void* W1,
+                                 const void* W2, const void* R, double dt_re, double dt_im, void* psi, int32_t kmax,
+                                 int32_t* out_k, void* ws, size_t ws_bytes) {
+  return reno_lanczos_expm_to(ctx, desc, L, W1, W2, R, dt_re, dt_im, psi, psi, kmax, out_k, ws, ws_bytes);
+}
+
+extern "C" int reno_lanczos_expm_to(reno_ctx* ctx, const reno_heff_desc* desc, const void* L, const void* W1,
+                                    const void* W2, const void* R, double dt_re, double dt_im, const void* psi,
+                                    void* out, int32_t kmax, int32_t* out_k, void* ws, size_t ws_bytes) {
+  return lanczos_run(ctx, desc, L, W1, W2, R, dt_re, dt_im, psi, out, kmax, 0, nullptr, out_k, ws, ws_bytes);
+}
+
+extern "C" int reno_lanczos_expm_resume(reno_ctx* ctx, const reno_heff_desc* desc, const void* L, const void* W1,
+                                        const void* W2, const void* R, double dt_re, double dt_im, void* out,
+                                        int32_t kmax, int32_t prev_kmax, const void* prev_ws, int32_t* out_k, void* ws,
+                                        size_t ws_bytes) {
+  if (!ctx) return RENO_ERR_INVALID;
+  if (!prev_ws) return set_error(ctx, RENO_ERR_INVALID, "reno_lanczos_expm_resume: null previous workspace");
+  return lanczos_run(ctx, desc, L, W1, W2, R, dt_re, dt_im, nullptr, out, kmax, prev_kmax, prev_ws, out_k, ws, ws_bytes);
 }

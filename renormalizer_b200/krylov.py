@@ -193,11 +193,12 @@ def _expm_krylov_steps(dt, vstart, block_size=50):
 _APPLY, _CALL = HeffOperator.apply, HeffOperator.__call__
 
 
-def _native_expm(op, dt, vstart, kmax):
-    """The exponential in one library call, or None where the generic driver
-    serves it: real results, an operator whose ``apply`` or ``__call__`` is not
-    HeffOperator's own, other tolerances than the reference's, more than kmax vectors, scalars that are
-    not finite (the driver raises for those)."""
+def _native_expm(op, dt, vstart, block_size):
+    """The exponential in library calls (one, and one more for each further
+    ``block_size`` vectors), or None where the generic driver serves it: real
+    results, an operator whose ``apply`` or ``__call__`` is not HeffOperator's
+    own, other tolerances than the reference's, scalars that are not finite
+    (the driver raises for those)."""
     if not isinstance(op, HeffOperator) or type(op).apply is not _APPLY or type(op).__call__ is not _CALL \
             or "apply" in vars(op) or not isinstance(op.engine, Engine):
         return None
@@ -214,7 +215,7 @@ def _native_expm(op, dt, vstart, kmax):
     op.desc.psi_dtype = RENO_C128
     op.engine.sync_stream()
     return op.engine.lanczos_expm(op.desc, op.L, op.W[0] if op.W else None, op.W[1] if op.nsite == 2 else None, op.R,
-                                  dt, v, kmax)
+                                  dt, v, block_size)
 
 
 def expm_krylov(Afunc, dt, vstart, block_size=50):
