@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import operator
 from typing import List, Sequence
 
 import numpy as np
@@ -122,14 +123,19 @@ class Rows(list):
     def __init__(self, tensors, ptrs, sizes):
         super().__init__(tensors)
         self.ptrs, self.sizes = ptrs, sizes
+        self._made = tuple(self)
 
     def intact(self) -> bool:
         """whether the list still holds the vectors it was made of, as they lie in
         memory: an entry that was replaced by a view of its own memory (a lazy
-        conjugate, a transpose, a part) has the same address"""
-        return len(self) == len(self.ptrs) and all(
-            t.data_ptr() == a and t.numel() == n and t.dtype is torch.complex128 and t.is_contiguous()
-            and not (t.is_conj() or t.is_neg()) for t, a, n in zip(self, self.ptrs.tolist(), self.sizes))
+        conjugate, a transpose, a part) has the same address.  One pass per
+        property over C methods: a lockstep round comes here twice, with 64
+        vectors 18 us a time (39 with a test per entry)."""
+        T = torch.Tensor
+        return (len(self) == len(self._made) and list(map(T.data_ptr, self)) == self.ptrs.tolist()
+                and list(map(T.numel, self)) == self.sizes and all(map(T.is_contiguous, self))
+                and (all(map(operator.is_, self, self._made)) or
+                     all(t.dtype is torch.complex128 and not (t.is_conj() or t.is_neg()) for t in self)))
 
 
 def _apply_rows(ops: Sequence["HeffOperator"], psis: Rows) -> "Rows":
