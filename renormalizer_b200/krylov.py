@@ -266,7 +266,8 @@ class _LockstepRows:
     buffer (row j holds every problem's V[j], item p from element off[p] on),
     so one operation's table of addresses is a few array expressions, and the
     Krylov vectors handed out are one split of a row.  A problem that ends
-    leaves the table; its columns stay where they are."""
+    leaves the table; when the rows run out, the problems still active move
+    to a larger buffer of their own."""
 
     def __init__(self, dts, vs, block_size):
         self.block_size = block_size
@@ -280,6 +281,7 @@ class _LockstepRows:
         self.off = np.concatenate([[0], np.cumsum(self.n)[:-1]])
         self.total = int(self.n.sum())
         self.rows = block_size
+        self.held = np.arange(m)  # the problems with columns in V, in their order there
         self.V = torch.empty((self.rows, self.total), dtype=torch.complex128, device=self.device)
         self.ab_len = 2 * block_size + 2
         # per problem: allclose flag, start norm, then (alpha_0, beta_0, alpha_1, ...)
@@ -304,19 +306,23 @@ class _LockstepRows:
     def _scalar(self, k, idx):
         return np.uint64(self.S.data_ptr()) + (8 * (idx * self.S.shape[1] + k)).astype(np.uint64)
 
-    def _grow(self):
-        V = torch.empty((self.rows + self.block_size, self.total), dtype=torch.complex128, device=self.device)
-        V[: self.rows] = self.V
+    def _grow(self, active):
+        n = self.n[active]
+        off = np.cumsum(n) - n
+        V = torch.empty((self.rows + self.block_size, int(n.sum())), dtype=torch.complex128, device=self.device)
+        for p, a in zip(active.tolist(), off.tolist()):
+            V[: self.rows, a:a + self.sizes[p]] = self.V[:, self.off[p]:self.off[p] + self.sizes[p]]
         S = torch.zeros((self.S.shape[0], self.S.shape[1] + 2 * self.block_size), dtype=torch.float64,
                         device=self.device)
         S[:, : self.S.shape[1]] = self.S
-        self.V, self.S, self.rows = V, S, V.shape[0]
+        self.off[active] = off
+        self.V, self.S, self.held, self.total, self.rows = V, S, active, V.shape[1], V.shape[0]
 
     def _images(self, group_apply, active, j):
         """group_apply on the active problems' V[j]: the images (kept alive) and their addresses"""
-        row = self.V[j].split(self.sizes)
+        row = self.V[j].split(self.n[self.held].tolist())
         sizes = self.n[active].tolist()
-        xs = Rows([row[p] for p in active], self._vec(j, active), sizes)
+        xs = Rows([row[i] for i in np.searchsorted(self.held, active)], self._vec(j, active), sizes)
         ws = group_apply(active.tolist(), xs)
         if isinstance(ws, Rows) and ws.sizes == sizes and ws.intact():
             return ws, ws.ptrs
@@ -332,14 +338,14 @@ class _LockstepRows:
     def run(self, group_apply):
         m = len(self.vs)
         result = [None] * m
-        buf = [torch.empty(self.total, dtype=torch.complex128, device=self.device) for _ in range(2)]
+        out = torch.empty(self.total, dtype=torch.complex128, device=self.device)
         active = np.arange(m)
         j = 0
         while len(active):
-            if self.rows == j + 1:
-                self._grow()
-            ws, wp = self._images(group_apply, active, j)
             ends = self.n[active] == j + 1
+            if self.rows == j + 1 and not ends.all():
+                self._grow(active)
+            ws, wp = self._images(group_apply, active, j)
             for op, sel in ((VOP_ALPHA, ends), (VOP_STEP, ~ends)):
                 if not sel.any():
                     continue
@@ -355,13 +361,13 @@ class _LockstepRows:
                 self.eng.vec_grouped_table(op, t)
             test = 3 < j and j % 2 == 0
             if test or ends.any():
-                active = self._decide(active, ends, j, test, result, buf)
+                active = self._decide(active, ends, j, test, result, out)
             else:
                 active = active[~ends]
             j += 1
         return result
 
-    def _decide(self, active, ends, j, test, result, buf):
+    def _decide(self, active, ends, j, test, result, out):
         """The reference's decisions at step j: problems at the end of their
         space, breakdowns since the last look, and (test) the convergence of
         the others; returns those that go on."""
@@ -390,7 +396,6 @@ class _LockstepRows:
             dev = h2d(_coefficients(sc[who, 1:], ks, [self.dts[p] for p in who]), self.device)
             at = np.uint64(dev.data_ptr()) + (16 * (np.cumsum(ks) - ks)).astype(np.uint64)
             at = np.concatenate([at[:len(final)], at[len(final)::2]])
-        out = buf[(j // 2) % 2]
         done = set()
         for op, which, first in ((VOP_LINCOMB, final, 0), (VOP_CHECK, checks, len(final))):
             if not which:
