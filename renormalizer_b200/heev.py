@@ -139,11 +139,20 @@ class LowRankOptions:
     kept ones has few eigenvalues above its own rounding errors (8 decades of
     sigma are 16 of lambda), while forming it and reducing all of its n
     columns to a tridiagonal matrix costs the same however few they are.  For
-    n >= ``min_ratio`` r the range is found first (Halko, Martinsson, Tropp,
-    SIAM Rev. 53, 2011): Q = orth(M^H (M Omega)) with r >= kt + ``oversample``
-    seeded Gaussian columns, B = M Q, T = B^H B.  T goes through the
-    device eigensolver, and with its eigenvectors S the wanted ones are
-    K = Q S and the projected block M K = B S, so G itself is never formed.
+    orders n >= ``min_n`` and n >= ``min_ratio`` r the range is found first
+    (Halko, Martinsson, Tropp, SIAM Rev. 53, 2011): Q1 = orth(M^H Omega) with
+    r >= kt + ``oversample`` seeded Gaussian columns Omega, Q = orth(M^H (M Q1)),
+    B = M Q, T = B^H B.  T goes through the device eigensolver, and with its
+    eigenvectors S the wanted ones are K = Q S and the projected block M K = B S,
+    so G itself is never formed.
+
+    The order of the passes is for precision.  From orth(M^H (M Omega)), what
+    rounding adds to the small columns of the second product leaves some 2e-15
+    of G outside Q, and truncated coefficients came out up to 1.24 times further from
+    64 bits than the dense route's (30 blocks of 480 to 2048 rows, mean
+    1.05).  Rounding of M^H Omega hides singular values below eps sigma_1 instead of
+    eigenvalues below eps lambda_1, M^H M maps each column of Q1 to its
+    own size, and the ratio is 1.000 or less on all of those blocks.
 
     The result is kept only where Q carries all of G to its rounding level:
     the invariance ||M^H B - Q T||_F <= ``tol`` ||T||_F, and the trace that is
@@ -154,16 +163,17 @@ class LowRankOptions:
 
     r comes from a sketch of ``probe`` columns, whose R factor's diagonal
     falls like the eigenvalues: the slope of its logarithm extrapolated to
-    rounding level (with 15 % more, for the sketch's scatter), at least
-    kt + oversample and at most n / min_ratio.  Where that upper limit is
-    below 0.7 of the extrapolation the block is not tried.
+    rounding level, at least kt + oversample and at most n / min_ratio.  Where
+    that upper limit is below 0.7 of the extrapolation the block is not tried.
 
-    Truncation of a complex 4096 x 4096 coefficient with two 2048^2 blocks
-    to 256: 54 -> 15 ms with sigma falling 3.5 decades over the kept ones,
-    27 ms with 1.5 decades; a flat spectrum pays 0.5 ms for the probe."""
+    Kept sides of two complex 2048^2 blocks, 320 vectors each: 48.7 ms by the
+    dense path, 13.4 / 21.3 / 28.3 through 416 / 608 / 800 columns; two of 600
+    rows, 128 vectors: 5.7 ms, 4.6 through 224 columns.  A probe that says no costs 0.2
+    to 0.5 ms, 4 % of a block of 480 rows and 1 % of one of 2048."""
 
-    def __init__(self, min_ratio=2.5, oversample=96, probe=32, tol=2e-14):
-        self.min_ratio, self.oversample, self.probe, self.tol = min_ratio, oversample, probe, tol
+    def __init__(self, min_n=480, min_ratio=2.5, oversample=32, probe=32, tol=2e-14):
+        self.min_n, self.min_ratio, self.oversample = min_n, min_ratio, oversample
+        self.probe, self.tol = probe, tol
         self.calls = 0
         self.missed = 0
 
@@ -176,6 +186,8 @@ def _range_columns(n: int, kt: int, diag=None) -> int:
     diagonal of its probe's R factor; 0 = dense path."""
     least = (kt + lowrank_opts.oversample + 31) // 32 * 32
     most = int(n / lowrank_opts.min_ratio) // 32 * 32
+    if n < lowrank_opts.min_n:
+        return 0
     if least > most or diag is None:
         return least if least <= most else 0
     eps = np.finfo(np.float64).eps
@@ -186,7 +198,7 @@ def _range_columns(n: int, kt: int, diag=None) -> int:
     need = -math.log(eps) / slope if slope > 0 else math.inf
     if most < 0.7 * need:
         return 0
-    return min(most, max(least, (int(1.15 * need) + 31) // 32 * 32))
+    return min(most, max(least, (int(need) + 31) // 32 * 32))
 
 
 def lowrank_top_batched(eng: Engine, Ms, kts):
@@ -198,6 +210,7 @@ def lowrank_top_batched(eng: Engine, Ms, kts):
     the dense path is to be taken."""
     out = [None] * len(Ms)
     size = lambda i: Ms[i][0].shape[0 if Ms[i][1] else 1]
+    long = lambda i: Ms[i][0].shape[1 if Ms[i][1] else 0]
     idx = [i for i, kt in enumerate(kts) if _range_columns(size(i), kt)]
     if not idx:
         return out
@@ -212,18 +225,19 @@ def lowrank_top_batched(eng: Engine, Ms, kts):
 
     dev = Ms[0][0].device
 
-    def sketch(i, cols, seed):  # seeded by its shape alone: a block's result does not depend on the batch it is in
+    def gaussian(rows, cols, seed):  # seeded by its shape alone: a block's result does not depend on the batch it is in
         gen = torch.Generator(device=dev).manual_seed(seed)
-        return back(i, fwd(i, torch.randn((size(i), cols), dtype=torch.float64, device=dev, generator=gen)))
+        return torch.randn((rows, cols), dtype=torch.float64, device=dev, generator=gen)
 
-    Rs = _qr_by_type(eng, [sketch(i, lowrank_opts.probe, 0x5EED) for i in idx])[1]
+    Rs = _qr_by_type(eng, [back(i, fwd(i, gaussian(size(i), lowrank_opts.probe, 0x5EED))) for i in idx])[1]
     diag = torch.stack([torch.diagonal(R).abs() for R in Rs]).cpu().numpy()
     rs = {i: _range_columns(size(i), kts[i], d) for i, d in zip(idx, diag)}
     idx = [i for i in idx if rs[i]]
     if not idx:
         return out
     lowrank_opts.calls += len(idx)
-    Qs = _qr_by_type(eng, [sketch(i, rs[i], 0x5EED + 1) for i in idx])[0]
+    Qs = _qr_by_type(eng, [back(i, gaussian(long(i), rs[i], 0x5EED + 1)) for i in idx])[0]
+    Qs = _qr_by_type(eng, [back(i, fwd(i, Q)) for i, Q in zip(idx, Qs)])[0]
     Bs = [fwd(i, Q) for i, Q in zip(idx, Qs)]
     Ts = [eng.matmul(B.transpose(0, 1), B, conj_a=True) for B in Bs]
     eig = heev_top_batched(eng, Ts, [kts[i] for i in idx])
