@@ -154,12 +154,14 @@ class LowRankOptions:
     eigenvalues below eps lambda_1, M^H M maps each column of Q1 to its
     own size, and the ratio is 1.000 or less on all of those blocks.
 
-    The result is kept only where Q carries all of G to its rounding level:
-    the invariance ||M^H B - Q T||_F <= ``tol`` ||T||_F, and the trace that is
-    missing, ||M||_F^2 - ||B||_F^2 <= ``tol`` ||M||_F^2, which bounds every
-    eigenvalue left out because G is positive semidefinite.  That is the size
-    of the dense reduction's own backward error.  A block that misses either
-    goes through the dense path.
+    The range is kept only where it carries all of G to G's own rounding
+    level: the trace that is missing, ||M - B Q^H||_F^2 <= ``tol`` sqrt(n)
+    ||M||_F^2, bounds every eigenvalue left out because G is positive semidefinite.
+    It is estimated without cancellation from ``check`` Gaussian vectors w, for
+    which ||M w - B (Q^H w)||^2 has that mean and falls to a tenth of it once in 1e12
+    times.  The host reads it twice, for Q1 (which leaves up to ten times
+    more, hence 64 limits) and for Q, both before the eigenproblem, and a block that
+    misses goes to the dense path with the others of its call.
 
     r comes from a sketch of ``probe`` columns, whose R factor's diagonal
     falls like the eigenvalues: the slope of its logarithm extrapolated to
@@ -171,9 +173,9 @@ class LowRankOptions:
     rows, 128 vectors: 5.7 ms, 4.6 through 224 columns.  A probe that says no costs 0.2
     to 0.5 ms, 4 % of a block of 480 rows and 1 % of one of 2048."""
 
-    def __init__(self, min_n=480, min_ratio=2.5, oversample=32, probe=32, tol=2e-14):
+    def __init__(self, min_n=480, min_ratio=2.5, oversample=32, probe=32, tol=1e-16, check=32):
         self.min_n, self.min_ratio, self.oversample = min_n, min_ratio, oversample
-        self.probe, self.tol = probe, tol
+        self.probe, self.tol, self.check = probe, tol, check
         self.calls = 0
         self.missed = 0
 
@@ -205,8 +207,7 @@ def lowrank_top_batched(eng: Engine, Ms, kts):
     """The kts[i] largest eigenpairs of each Gram matrix G = M^H M through its
     numerical range (LowRankOptions).  Ms: (matrix, adjoint) pairs, M the
     matrix or, with adjoint, its conjugate transpose.  Returns per entry
-    (w, K, check, M K) -- w, K and check like heev_top_batched, with 1 in the
-    check's second entry where the range misses part of G -- or None where
+    (w, K, check, M K) -- w, K and check like heev_top_batched -- or None where
     the dense path is to be taken."""
     out = [None] * len(Ms)
     size = lambda i: Ms[i][0].shape[0 if Ms[i][1] else 1]
@@ -223,32 +224,49 @@ def lowrank_top_batched(eng: Engine, Ms, kts):
         X, adj = Ms[i]
         return eng.matmul(X, v) if adj else eng.matmul(X.transpose(0, 1), v, conj_a=True)
 
-    dev = Ms[0][0].device
+    dev, norm = Ms[0][0].device, torch.linalg.vector_norm
 
     def gaussian(rows, cols, seed):  # seeded by its shape alone: a block's result does not depend on the batch it is in
         gen = torch.Generator(device=dev).manual_seed(seed)
         return torch.randn((rows, cols), dtype=torch.float64, device=dev, generator=gen)
 
-    Rs = _qr_by_type(eng, [back(i, fwd(i, gaussian(size(i), lowrank_opts.probe, 0x5EED))) for i in idx])[1]
-    diag = torch.stack([torch.diagonal(R).abs() for R in Rs]).cpu().numpy()
+    def orth(mats):
+        return dict(zip(idx, _qr_by_type(eng, [mats[i] for i in idx])[0]))
+
+    def keep(bad):  # drops the blocks whose (device) flag is set
+        for i, b in zip(list(idx), torch.stack([bad[i] for i in idx]).cpu().tolist()):
+            if b:
+                idx.remove(i)
+                lowrank_opts.missed += 1
+
+    Y = [back(i, fwd(i, gaussian(size(i), lowrank_opts.probe, 0x5EED))) for i in idx]
+    diag = torch.stack([torch.diagonal(R).abs() for R in _qr_by_type(eng, Y)[1]]).cpu().numpy()
     rs = {i: _range_columns(size(i), kts[i], d) for i, d in zip(idx, diag)}
     idx = [i for i in idx if rs[i]]
+    lowrank_opts.calls += len(idx)
     if not idx:
         return out
-    lowrank_opts.calls += len(idx)
-    Qs = _qr_by_type(eng, [back(i, gaussian(long(i), rs[i], 0x5EED + 1)) for i in idx])[0]
-    Qs = _qr_by_type(eng, [back(i, fwd(i, Q)) for i, Q in zip(idx, Qs)])[0]
-    Bs = [fwd(i, Q) for i, Q in zip(idx, Qs)]
-    Ts = [eng.matmul(B.transpose(0, 1), B, conj_a=True) for B in Bs]
-    eig = heev_top_batched(eng, Ts, [kts[i] for i in idx])
-    norm = torch.linalg.vector_norm
-    for i, Q, B, T, (w, S, chk) in zip(idx, Qs, Bs, Ts, eig):
-        res = norm(back(i, B) - eng.matmul(Q, T)) / norm(T)
-        full = norm(Ms[i][0]) ** 2
-        miss = (full - norm(B) ** 2) / full
-        fail = ~((res <= lowrank_opts.tol) & (miss <= lowrank_opts.tol))
-        S = S if Q.is_complex() else S.real.contiguous()
-        out[i] = (w, eng.matmul(Q, S), torch.stack([chk[0], fail.to(torch.float64), chk[2]]), eng.matmul(B, S))
+    W = {i: gaussian(size(i), lowrank_opts.check, 0x5EED + 2) for i in idx}
+    MW = {i: fwd(i, W[i]) for i in idx}
+    limit = {i: lowrank_opts.tol * math.sqrt(size(i)) for i in idx}
+    full = {i: norm(Ms[i][0]) ** 2 for i in idx}
+
+    def missing(i):  # of the trace, relative
+        x = MW[i] - eng.matmul(B[i], eng.matmul(Q[i].transpose(0, 1), W[i], conj_a=True))
+        return norm(x) ** 2 / (lowrank_opts.check * full[i])
+
+    Q = orth({i: back(i, gaussian(long(i), rs[i], 0x5EED + 1)) for i in idx})
+    B = {i: fwd(i, Q[i]) for i in idx}
+    keep({i: ~(missing(i) <= 64 * limit[i]) for i in idx})
+    if not idx:
+        return out
+    Q = orth({i: back(i, B[i]) for i in idx})
+    B = {i: fwd(i, Q[i]) for i in idx}
+    T = {i: eng.matmul(B[i].transpose(0, 1), B[i], conj_a=True) for i in idx}
+    keep({i: ~(missing(i) <= limit[i]) for i in idx})
+    for i, (w, S, chk) in zip(idx, heev_top_batched(eng, [T[i] for i in idx], [kts[i] for i in idx])):
+        S = S if Q[i].is_complex() else S.real.contiguous()
+        out[i] = (w, eng.matmul(Q[i], S), chk, eng.matmul(B[i], S))
     return out
 
 

@@ -575,7 +575,7 @@ def _device_eig_ok(G: torch.Tensor) -> bool:
     return heev.heev_opts.enabled and G.is_cuda and heev.heev_opts.min_n <= n <= 4096
 
 
-def _kept_sides(eng: Engine, Xs, keep_left: bool, ktops, use_heev: bool = True, lowrank: bool = True) -> list:
+def _kept_sides(eng: Engine, Xs, keep_left: bool, ktops, use_heev: bool = True) -> list:
     """_full_kept_side for all QN blocks of one truncation: large blocks with
     few eigenvalues above rounding through their numerical range
     (heev.lowrank_top_batched), the others by their Gram matrix and the device
@@ -588,7 +588,7 @@ def _kept_sides(eng: Engine, Xs, keep_left: bool, ktops, use_heev: bool = True, 
         dim = min(X.shape)
         items.append(dict(X=X, kt=dim if ktop is None else min(int(ktop), dim), dim=dim, ME=None))
     dev = [it for it in items if use_heev and _device_eig_ok(it["X"])]
-    if dev and lowrank:
+    if dev:
         res = heev.lowrank_top_batched(eng, [(it["X"], _gram_is_left(it["X"], keep_left)) for it in dev],
                                        [it["kt"] for it in dev])
         for it, r in zip(dev, res):
@@ -614,13 +614,11 @@ def _kept_sides(eng: Engine, Xs, keep_left: bool, ktops, use_heev: bool = True, 
         Qs, _ = eng.qr_blocks([outs[i]["need_qr"] for i in need])
         for i, Q in zip(need, Qs):
             outs[i] = finish(items[i], Q)
-    for it, o in zip(items, outs):
-        o["lowrank"] = it["ME"] is not None
     return outs
 
 
 def _full_kept_side(eng: Engine, X: torch.Tensor, keep_left: bool, ktop: Optional[int] = None,
-                    use_heev: bool = True, lowrank: bool = True) -> dict:
+                    use_heev: bool = True) -> dict:
     """Kept-side basis K, projection P and sigma S of one block from the
     Hermitian eigendecomposition of the Gram matrix of its smaller side (all
     min(m, n) triplets).
@@ -636,7 +634,7 @@ def _full_kept_side(eng: Engine, X: torch.Tensor, keep_left: bool, ktop: Optiona
     entry sorts after every head entry of its block, and since a block
     contributes at most the cap (< ktop) entries, none is selected; they only
     fill the list the truncation rule reads."""
-    return _kept_sides(eng, [X], keep_left, [ktop], use_heev, lowrank)[0]
+    return _kept_sides(eng, [X], keep_left, [ktop], use_heev)[0]
 
 
 def svd_truncate(coef: torch.Tensor, qnbigl, qnbigr, qntot, keep_left: bool, m_trunc_fn, percent=0,
@@ -745,7 +743,7 @@ def _trunc_eig(states):
                 flop_log.append(_block_flops(m_, n_, b["ktop"] or min(m_, n_), b["X"].is_complex()))
         fulls = _kept_sides(states[0]["eng"], [b["X"] for b in group], keep_left, [b["ktop"] for b in group])
         for b, full in zip(group, fulls):
-            b.update(K=full["K"], P=full["P"], S=full["S"], lowrank=full["lowrank"])
+            b.update(K=full["K"], P=full["P"], S=full["S"])
             if full["chk"] is not None:
                 b["chk"] = full["chk"]
             else:
@@ -871,12 +869,6 @@ def _trunc_select(st, host):
     off_chk = off + 2 * len(sub)
     for i, b in enumerate(dev_eig):
         ok = heev.accepted(host[off_chk + 3 * i: off_chk + 3 * i + 3])
-        if not ok and b["lowrank"]:
-            # part of the block's Gram matrix lies outside the sketched range: the dense device path
-            heev.lowrank_opts.missed += 1
-            b.update(_full_kept_side(eng, b["X"], keep_left, b["ktop"], lowrank=False))
-            host_b = torch.cat([b["S"], b["chk"]]).cpu().numpy()
-            b["Sh"], ok = host_b[:b["dim"]], heev.accepted(host_b[b["dim"]:])
         if not ok:
             # the device eigensolver missed its checks on this block: cuSOLVER
             heev.heev_opts.fallbacks += 1

@@ -1,7 +1,7 @@
 """The range route against the dense route on the same blocks: truncated
 coefficients no further from torch's SVD, on the spectra of sweeps (a
 decade every keep / 5 to keep / 7 values), a power law, a steep head before
-a slow tail and one large value far ahead of the rest.
+a slow tail and one large value far ahead of the rest; and missed blocks of a batch in one dense call.
 
 Both routes end in an eigenproblem with rounding at eps lambda_1, whose mixing
 of kept and discarded vectors is the error; the range route adds nothing of
@@ -66,3 +66,28 @@ def test_no_further_from_64_bits_than_the_dense_route(m, n, spectrum, keep, cplx
         err.append(float(torch.linalg.vector_norm(res.left @ res.right - ref)))
     assert err[0] <= 1.05 * err[1] + 1e-15 * float(S[0])
 
+
+def test_missed_blocks_share_one_dense_call(monkeypatch):
+    """three truncations whose block passes the probe and misses the check"""
+    calls = []
+    orig = heev.heev_top_batched
+    monkeypatch.setattr(heev, "heev_top_batched", lambda eng, Gs, kts: (calls.append([G.shape[0] for G in Gs]),
+                                                                       orig(eng, Gs, kts))[1])
+    keep, args, refs = 32, [], []
+    for seed in (1, 2, 3):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        j = torch.arange(640, dtype=torch.float64, device="cuda")
+        s = torch.where(j < keep, 10.0 ** (-2.0 * j / keep), torch.full_like(j, 1e-5))
+        s[8:keep] *= 0.5
+        c = lambda a, b: torch.complex(*torch.randn((2, a, b), dtype=torch.float64, device="cuda", generator=g))
+        X = (torch.linalg.qr(c(700, 640))[0] * s) @ torch.linalg.qr(c(640, 640))[0].mH
+        args.append(dict(coef=X, qnbigl=np.zeros((700, 1), int), qnbigr=np.zeros((640, 1), int), qntot=np.array([0]),
+                         keep_left=True, m_trunc_fn=lambda s: keep, kcap=keep))
+        U, S, Vh = torch.linalg.svd(X, full_matrices=False)
+        refs.append((U[:, :keep] * S[:keep]) @ Vh[:keep])
+    c0, m0 = heev.lowrank_opts.calls, heev.lowrank_opts.missed
+    got = svd_qn.svd_truncate_batch(args)
+    assert (heev.lowrank_opts.calls - c0, heev.lowrank_opts.missed - m0) == (3, 3)
+    assert calls == [[640] * 3]
+    for res, ref in zip(got, refs):
+        assert float(torch.linalg.vector_norm(res.left @ res.right - ref)) <= 1e-9 * float(torch.linalg.vector_norm(ref))
