@@ -167,6 +167,11 @@ class LowRankOptions:
     falls like the eigenvalues: the slope of its logarithm extrapolated to
     rounding level, at least kt + oversample and at most n / min_ratio.  Where
     that upper limit is below 0.7 of the extrapolation the block is not tried.
+    Nor is it where a dense block of 0.8 its order or more belongs to the same
+    truncation and r > n^2 / 10240: the dense reduction, a chain of columns, takes
+    little longer for two blocks than for one (1.2 / 3.7 / 16 / 82 ms at n = 1024 /
+    1440 / 2048 / 3584, which grows like n^3), while the range alone costs 5.3
+    / 6.2 / 10.4 / 30.7 ms at r = n / 5 and grows like n r.
 
     Kept sides of two complex 2048^2 blocks, 320 vectors each: 48.7 ms by the
     dense path, 13.4 / 21.3 / 28.3 through 416 / 608 / 800 columns; two of 600
@@ -203,10 +208,11 @@ def _range_columns(n: int, kt: int, diag=None) -> int:
     return min(most, max(least, (int(need) + 31) // 32 * 32))
 
 
-def lowrank_top_batched(eng: Engine, Ms, kts):
+def lowrank_top_batched(eng: Engine, Ms, kts, calls):
     """The kts[i] largest eigenpairs of each Gram matrix G = M^H M through its
     numerical range (LowRankOptions).  Ms: (matrix, adjoint) pairs, M the
-    matrix or, with adjoint, its conjugate transpose.  Returns per entry
+    matrix or, with adjoint, its conjugate transpose; calls: which truncation
+    each entry belongs to.  Returns per entry
     (w, K, check, M K) -- w, K and check like heev_top_batched -- or None where
     the dense path is to be taken."""
     out = [None] * len(Ms)
@@ -242,7 +248,11 @@ def lowrank_top_batched(eng: Engine, Ms, kts):
     Y = [back(i, fwd(i, gaussian(size(i), lowrank_opts.probe, 0x5EED))) for i in idx]
     diag = torch.stack([torch.diagonal(R).abs() for R in _qr_by_type(eng, Y)[1]]).cpu().numpy()
     rs = {i: _range_columns(size(i), kts[i], d) for i, d in zip(idx, diag)}
-    idx = [i for i in idx if rs[i]]
+    beside = {}  # the largest block of each truncation that the probe sends to the dense path
+    for i, c in enumerate(calls):
+        if not rs.get(i):
+            beside[c] = max(beside.get(c, 0), size(i))
+    idx = [i for i in idx if rs[i] and (size(i) > 1.25 * beside.get(calls[i], 0) or 10240 * rs[i] <= size(i) ** 2)]
     lowrank_opts.calls += len(idx)
     if not idx:
         return out

@@ -575,22 +575,23 @@ def _device_eig_ok(G: torch.Tensor) -> bool:
     return heev.heev_opts.enabled and G.is_cuda and heev.heev_opts.min_n <= n <= 4096
 
 
-def _kept_sides(eng: Engine, Xs, keep_left: bool, ktops, use_heev: bool = True) -> list:
+def _kept_sides(eng: Engine, Xs, keep_left: bool, ktops, use_heev: bool = True, calls=None) -> list:
     """_full_kept_side for all QN blocks of one truncation: large blocks with
     few eigenvalues above rounding through their numerical range
     (heev.lowrank_top_batched), the others by their Gram matrix and the device
     eigensolver on all of them at once (heev_top_batched; blocks above its
     size limit, or with the device eigensolver switched off, take cuSOLVER),
     and one batched Householder QR where a projected basis needs
-    orthonormalising."""
+    orthonormalising.  ``calls``: which truncation each block belongs to
+    (default: all to one)."""
     items = []
-    for X, ktop in zip(Xs, ktops):
+    for X, ktop, call in zip(Xs, ktops, calls or [0] * len(Xs)):
         dim = min(X.shape)
-        items.append(dict(X=X, kt=dim if ktop is None else min(int(ktop), dim), dim=dim, ME=None))
+        items.append(dict(X=X, call=call, kt=dim if ktop is None else min(int(ktop), dim), dim=dim, ME=None))
     dev = [it for it in items if use_heev and _device_eig_ok(it["X"])]
     if dev:
         res = heev.lowrank_top_batched(eng, [(it["X"], _gram_is_left(it["X"], keep_left)) for it in dev],
-                                       [it["kt"] for it in dev])
+                                       [it["kt"] for it in dev], [it["call"] for it in dev])
         for it, r in zip(dev, res):
             if r is not None:
                 it.update(w=r[0], E=r[1], chk=r[2], ME=r[3])
@@ -734,14 +735,17 @@ def _trunc_eig(states):
     """Kept sides of the pending blocks of every state: one _kept_sides pass
     per kept side over all of them."""
     for keep_left in (True, False):
-        group = [b for st in states if st["keep_left"] == keep_left for b in st["pending"]]
+        side = [st for st in states if st["keep_left"] == keep_left]
+        group = [b for st in side for b in st["pending"]]
         if not group:
             continue
+        calls = [c for c, st in enumerate(side) for _ in st["pending"]]
         if flop_log is not None:
             for b in group:
                 m_, n_ = b["X"].shape
                 flop_log.append(_block_flops(m_, n_, b["ktop"] or min(m_, n_), b["X"].is_complex()))
-        fulls = _kept_sides(states[0]["eng"], [b["X"] for b in group], keep_left, [b["ktop"] for b in group])
+        fulls = _kept_sides(states[0]["eng"], [b["X"] for b in group], keep_left, [b["ktop"] for b in group],
+                            calls=calls)
         for b, full in zip(group, fulls):
             b.update(K=full["K"], P=full["P"], S=full["S"])
             if full["chk"] is not None:

@@ -91,3 +91,27 @@ def test_missed_blocks_share_one_dense_call(monkeypatch):
     assert calls == [[640] * 3]
     for res, ref in zip(got, refs):
         assert float(torch.linalg.vector_norm(res.left @ res.right - ref)) <= 1e-9 * float(torch.linalg.vector_norm(ref))
+
+
+@pytest.mark.parametrize("other,tried", [(640, 0), (520, 0), (500, 1)])
+def test_range_route_beside_a_dense_block(other, tried):
+    """a block beside one that the probe refuses: left to the dense reduction that runs anyway, unless that
+    one is of less than 0.8 the order; the same in a batch with another truncation whose blocks both qualify"""
+    keep, n = 32, 640
+    A = _block(n, n, "exponential", keep, True, 5)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    F = torch.complex(*torch.randn((2, other, other), dtype=torch.float64, device="cuda", generator=g)) / other
+    X = torch.zeros((n + other, n + other), dtype=A.dtype, device="cuda")
+    X[:n, :n], X[n:, n:] = A, F
+    Y = torch.zeros((2 * n, 2 * n), dtype=A.dtype, device="cuda")
+    Y[:n, :n], Y[n:, n:] = A, 0.5 * A
+    job = lambda Z, k: dict(coef=Z, qnbigl=np.repeat([0, 1], [n, k]).reshape(-1, 1),
+                            qnbigr=np.repeat([1, 0], [n, k]).reshape(-1, 1), qntot=np.array([1]), keep_left=True,
+                            m_trunc_fn=lambda s: 2 * keep, kcap=2 * keep)
+    c0 = heev.lowrank_opts.calls
+    alone = svd_qn.svd_truncate(**job(X, other))
+    assert heev.lowrank_opts.calls - c0 == tried
+    both = svd_qn.svd_truncate_batch([job(Y, n), job(X, other)])
+    assert heev.lowrank_opts.calls - c0 == 2 * tried + 2
+    ref = alone.left @ alone.right
+    assert float(torch.linalg.vector_norm(both[1].left @ both[1].right - ref)) <= 1e-12 * float(torch.linalg.vector_norm(ref))
