@@ -23,7 +23,7 @@
 //                     eigenvalue: LU of T - lambda I with partial pivoting,
 //                     three solves from a hashed start vector, in shared
 //                     memory (inviter_smem_kernel) but for the largest.  The host
-//                     orthonormalises the block (CholeskyQR2) and checks the
+//                     orthonormalises the block (Householder QR) and checks the
 //                     residuals ||T z - lambda z||.
 //   4. back-transformation K = Q Z in blocks of 64 reflectors (compact WY
 //                     form, three FP64 GEMMs per block, last block first).

@@ -9,7 +9,7 @@
 //   panel kernels    one 8-CTA thread-block cluster per matrix factorises the
 //                    panel, its rows split over the CTAs.  Up to 4096 rows
 //                    (8192 real) the panel lives in registers
-//                    (qr_panel_reg_kernel, one cluster barrier per column);
+//                    (qr_panel_reg_kernel, one CTA and one cluster barrier per column);
 //                    taller matrices keep it in shared memory
 //                    (qr_panel_kernel, two barriers per column).  The
 //                    partial sums are added in the same order by every CTA,
@@ -334,15 +334,15 @@ __global__ void __cluster_dims__(QCL, 1, 1) __launch_bounds__(QT, 1)
 // ---------------------------------------------------------------- register panels
 // The same panel with its entries in registers: warp w owns the columns
 // c = w + 8 s (s < NC), lane l the rows l + 32 i (i < R) of the CTA's chunk.
-// What bounds it is the chain per column, so that chain is one reduction and
-// one cluster barrier: with x the pivot column below the diagonal, every warp
-// has S_c = sum_r conj(x_r) A[r, c] of its columns ready, taken in the pass
-// that applied the previous reflector; S of the pivot itself is ||x||^2, so
-// beta, tau and the scale of v follow, and w_c = A[p, c] + conj(scale) S_c is
-// the row the update needs.  Columns left of the pivot hold reflectors, whose
-// S_c give the column of V^H V that T needs.  The partial S and the pivot row
-// are pushed into every CTA's shared memory before the barrier, so that all
-// reads after it are local.  A 2048 x 128 pair of complex matrices takes
+// What bounds it is the chain per column: the owner warp of the pivot column
+// puts x, its part below the diagonal, into shared memory (a CTA barrier), every
+// warp sums S_c = sum_r conj(x_r) A[r, c] over its columns and rows, the partial S and
+// the pivot row are pushed into every CTA's shared memory (a cluster
+// barrier), and each warp forms the scalars and updates its columns.  One reduction
+// serves for all of it: S of the pivot itself is ||x||^2, so beta, tau and the
+// scale of v follow, and w_c = A[p, c] + conj(scale) S_c is the row the update
+// needs.  Columns left of the pivot hold reflectors, whose S_c give the
+// column of V^H V that T needs.  A 2048 x 128 pair of complex matrices takes
 // 121 us per 32-column panel, 517 us in the shared-memory kernel (two
 // reductions, two cluster barriers and 200 KB of shared-memory traffic per
 // column).

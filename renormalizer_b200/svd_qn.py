@@ -148,9 +148,11 @@ def qn_block_svd(coef: torch.Tensor, qnbigl, qnbigr, qntot, full_matrices=True, 
 class _QrBlock:
     """One QN block of a QR ("L") or RQ ("R").  For RQ the block is gathered
     with both index lists reversed and then conjugate-transposed, so that it
-    goes to the same QR; rows / cols are the lists as gathered, place the
-    result's columns in the assembled factors, and the *_d their device
-    copies."""
+    goes to the same QR: (J A J)^H = Q1 R1 gives A = (J R1^H J)(J Q1^H J) with
+    J R1^H J upper triangular, and Householder QR takes the entries in the
+    order of LAPACK's RQ, so that R and Q agree with scipy.linalg.rq including
+    the signs.  rows / cols are the lists as gathered, place the result's
+    columns in the assembled factors, and the *_d their device copies."""
     nl: tuple
     nr: tuple
     rows: np.ndarray
@@ -163,8 +165,8 @@ class _QrBlock:
 
 
 def _qr_begin(coef: torch.Tensor, qnbigl, qnbigr, qntot, system: str):
-    """The QN blocks of one QR / RQ (qn_block_qr), gathered: (blocks, rows,
-    cols, arange), all index lists in one transfer."""
+    """The QN blocks of one QR / RQ, gathered: (blocks, rows, cols, arange), all
+    index lists in one transfer."""
     if system not in ("L", "R"):
         raise AssertionError("system must be L or R for QR")
     eng = Engine.get(coef.device)
@@ -189,28 +191,6 @@ def _qr_begin(coef: torch.Tensor, qnbigl, qnbigr, qntot, system: str):
             blk = torch.conj_physical(blk.transpose(0, 1), out=out)
         blocks.append(_QrBlock(nl, nr, *lists[3 * i:3 * i + 3], *dev[3 * i:3 * i + 3], blk))
     return blocks, rows, cols, dev[-1]
-
-
-def qn_block_qr(coef: torch.Tensor, qnbigl, qnbigr, qntot, system: str):
-    """Per-block QR (system "L") or RQ (system "R"), economic (svd_qn.py:195-204),
-    every QN block of the site in one batched Householder QR (reno_qr_blocks,
-    LAPACK's sign conventions).  RQ comes from the QR of the reversed
-    conjugate transpose: (J A J)^H = Q1 R1 gives A = (J R1^H J)(J Q1^H J), with
-    J R1^H J upper triangular.  Householder QR processes the entries in the
-    same order as LAPACK's RQ (last row first, pivot on its last entry), so R
-    and Q agree with scipy.linalg.rq including the signs, not only up to a
-    rotation."""
-    found, rows, cols, _ = _qr_begin(coef, qnbigl, qnbigr, qntot, system)
-    Qs, Rs = Engine.get(coef.device).qr_blocks([f.blk for f in found])
-    blocks = []
-    for f, Q, R in zip(found, Qs, Rs):
-        if system == "L":
-            blocks.append(QNBlock(f.nl, f.nr, f.rows, f.cols, Q, None, None, R))
-        else:
-            blocks.append(QNBlock(f.nl, f.nr, f.rows[::-1], f.cols[::-1],
-                                  R.mH.flip([0, 1]).resolve_conj().contiguous(), None, None,
-                                  Q.mH.flip([0, 1]).resolve_conj().contiguous()))
-    return blocks, rows, cols
 
 
 def _check_scatter(src, r, c, dc, dst, dst_rs, dst_cs):
@@ -489,21 +469,6 @@ def _subspace_block(eng, X, keep_left, k, opts, Q=None, iters=None):
         return _topk_kept_side(eng, X, k, opts, Q, iters)
     K, Ph, S, chk, Q = _topk_kept_side(eng, X.transpose(0, 1).conj(), k, opts, Q, iters)
     return K, Ph.transpose(0, 1).conj().resolve_conj(), S, chk, Q
-
-
-def _gram_eigh(eng: Engine, G: torch.Tensor, kt: int, use_heev: bool):
-    """Eigenpairs of the Gram matrix G, descending: (w, V, check).  With the
-    device eigensolver (``heev.heev_opts``) only the leading kt are computed
-    (w has kt entries) and check is its device-side acceptance triple;
-    otherwise cuSOLVER's full decomposition and check None."""
-    n = G.shape[0]
-    if use_heev and heev.heev_opts.enabled and kt < n and n >= heev.heev_opts.min_n and G.is_cuda:
-        w, V, chk = heev.heev_top(eng, G, kt)
-        if not G.is_complex():
-            V = V.real.contiguous()
-        return w, V, chk
-    w, V = torch.linalg.eigh(G)
-    return torch.flip(w, dims=[0]), torch.flip(V, dims=[1]), None
 
 
 def _gram_is_left(X: torch.Tensor, keep_left: bool) -> bool:
