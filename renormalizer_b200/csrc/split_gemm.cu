@@ -12,10 +12,10 @@
 // Pipeline (persistent: one CTA per SM walks 128 x 256 output tiles; 10 warps):
 //   warp 0     TMA producer: 4 tiles per stage (A_hi, A_lo, B_hi, B_lo),
 //              64-byte swizzled K-major boxes, mbarrier complete_tx.  Four
-//              48 KB stages: two of 96 KB refill one while the other computes,
-//              which at 64 bytes a clock leaves no time for the latency (M = 256
+//              48 KB stages: with two of 96 KB only one is in flight while the
+//              other computes, too little to cover the L2's latency (M = 256
 //              two-site matvec 1604 -> 1576 us, its last stage 360 -> 322; the
-//              first stays near the L2's rate, 401 us)
+//              first loads 3.8 GB through L2 in 413 us)
 //   warp 1     TMEM allocator + single-thread tcgen05.mma issuer: 3 products
 //              per stage, tcgen05.commit frees the stage
 //   warps 2-9  epilogue (two warps per TMEM lane quarter, half the columns
